@@ -482,7 +482,7 @@ class Accelerator:
 
     # -- unique (the step after a sort) --
     def ComputeUniqueTempStorageSize(self, dtype: torch.dtype, dataLength: int) -> int:
-        """UniqueExtensions.cs:114-121; here the temp holds the survivors, so it grows with n."""
+        """UniqueExtensions.cs:114-121; here the temp holds a record per tile, so it grows with n."""
         out = ctypes.c_int64(0)
         B200AlgException.ThrowIfFailed(self.L.b200alg_unique_temp_bytes(dtype_code(dtype), int(dataLength), ctypes.byref(out)))
         return _ints(out.value)

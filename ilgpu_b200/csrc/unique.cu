@@ -2,18 +2,20 @@
 // Replaces UniqueKernel / CreateUnique (UniqueExtensions.cs:59-195), whose groups run one after
 // the other (SequentialGroupExecutor) and whose first thread compacts a whole tile alone.
 // Here every tile flags the elements that differ from their left neighbour, chains its count
-// to the previous tiles with decoupled look-back, and writes its survivors to scratch; a second
-// kernel copies the survivors back.  Equality follows Comparison{T} = first.CompareTo(second)
+// to the previous tiles with decoupled look-back, and writes its survivors where they belong,
+// in place.  Equality follows Comparison{T} = first.CompareTo(second)
 // (ComparisonOperations.tt): integers compare by value; floating-point values compare equal when
 // they are numerically equal or both NaN.
 #include "common.cuh"
 #include "lookback.cuh"
 
+#include <type_traits>
+
 namespace b200alg {
 
-constexpr int kUniqueThreads = 256;
-constexpr int kUniqueItems = 16;
-constexpr int kUniqueTile = kUniqueThreads * kUniqueItems;
+constexpr int kUniqueThreads = 512;
+constexpr int kUniqueVecs = 4;                                        // 16-byte vectors per thread
+constexpr int kUniqueTileBytes = kUniqueThreads * kUniqueVecs * 16;
 
 template <typename T> struct SameValue {
     static __device__ __forceinline__ bool eq(T a, T b) { return a == b; }
@@ -31,57 +33,122 @@ template <> struct SameValue<__half> {
     }
 };
 
+// The 1- and 2-byte integers travel through the 32-bit shuffles.
+template <typename T> __device__ __forceinline__ T shfl_value_up(T v) {
+    if constexpr (sizeof(T) <= 2 && !std::is_same<T, __half>::value) return (T)__shfl_up_sync(0xffffffffu, (unsigned int)v, 1);
+    else return shfl_up(v, 1);
+}
+template <typename T> __device__ __forceinline__ T shfl_value_last(T v) {
+    if constexpr (sizeof(T) <= 2 && !std::is_same<T, __half>::value) return (T)__shfl_sync(0xffffffffu, (unsigned int)v, 31);
+    else return shfl_idx(v, 31);
+}
+
+// Bound: HBM (every element read once, every survivor written once).  A tile is 32 KB: 16-byte
+// loads, four in flight per thread, in warp-striped order (vector j of lane l holds elements
+// (warp * 4 * 32 + j * 32 + l) * VEC ... of the tile), so a warp reads whole lines; survivors meet
+// in shared memory and leave in consecutive stores.
+//
+// `kept` may be `in` itself (the in-place unique): a tile stores only once it knows its prefix,
+// hence after every earlier tile has published its count and so has read its elements, and it
+// stores at or below its own elements' places.  The one element a tile reads outside its own
+// range is the last one of the tile before; only that element itself (unmoved) is stored there
+// before this tile has published.
 template <typename T>
-__global__ void __launch_bounds__(kUniqueThreads)
-unique_select_kernel(const T *__restrict__ in, int64_t n, T *__restrict__ kept, long long *__restrict__ starts,
-                     long long *out_count, TempHeader *hdr, void *state_base, int num_tiles) {
-    __shared__ unsigned int warp_total[kUniqueThreads / 32];
-    __shared__ unsigned int warp_excl[kUniqueThreads / 32];
-    __shared__ unsigned int s_prefix;
+__global__ void __launch_bounds__(kUniqueThreads, 3)
+unique_select_kernel(const T *in, int64_t n, T *kept, long long *__restrict__ starts, long long *out_count, TempHeader *hdr,
+                     void *state_base, int num_tiles) {
+    constexpr int VEC = 16 / (int)sizeof(T);
+    constexpr int NV = kUniqueVecs;
+    constexpr int TILE = VEC * NV * kUniqueThreads;
+    constexpr int WARPS = kUniqueThreads / 32;
+    union Vec { uint4 u; T t[VEC]; __device__ Vec() {} };
+
+    __shared__ __align__(16) unsigned char survivors_raw[TILE * sizeof(T)];
+    __shared__ unsigned int warp_total[WARPS];
+    __shared__ unsigned int warp_excl[WARPS];
+    __shared__ unsigned int s_prefix, s_count;
     __shared__ int s_tile;
+    T *survivors = reinterpret_cast<T *>(survivors_raw);
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid == 0) s_tile = (int)atomicAdd(&hdr->reserved[0], 1u);  // tiles are handed out in order
     __syncthreads();
     const int tile = s_tile;
-    const int64_t first = (int64_t)tile * kUniqueTile + (int64_t)tid * kUniqueItems;
+    const int64_t base = (int64_t)tile * TILE;
+    const int64_t remaining = n - base;
+    const int warp_first = warp * (NV * 32 * VEC);  // the warp's first element inside the tile
 
-    // thread t owns kUniqueItems consecutive elements; keep[k] = element k starts a new run
-    T item[kUniqueItems];
-    T left = T();
-    const bool has_left = first > 0 && first < n;
-    if (has_left) left = in[first - 1];
-    unsigned int keep_mask = 0u, count = 0u;
+    Vec v[NV];
+    if (remaining >= TILE && ((uintptr_t)in & 15u) == 0) {
+        const uint4 *src = reinterpret_cast<const uint4 *>(in + base + warp_first) + lane;
 #pragma unroll
-    for (int k = 0; k < kUniqueItems; ++k) {
-        const int64_t idx = first + k;
-        if (idx < n) {
-            item[k] = in[idx];
-            const bool keep = (idx == 0) || !SameValue<T>::eq(item[k], k == 0 ? left : item[k - 1]);
-            keep_mask |= (unsigned int)keep << k;
-            count += keep;
+        for (int j = 0; j < NV; ++j) v[j].u = src[j * 32];
+    } else {
+#pragma unroll
+        for (int j = 0; j < NV; ++j)
+#pragma unroll
+            for (int e = 0; e < VEC; ++e) {
+                const int at = warp_first + (j * 32 + lane) * VEC + e;
+                if (at < remaining) v[j].t[e] = in[base + at];
+            }
+    }
+    // the element in front of the warp's chunk
+    const bool has_left = base + warp_first > 0 && warp_first < remaining;
+    T left = v[0].t[0];
+    if (has_left) left = in[base + warp_first - 1];
+
+    // keep bit e of vector j: element starts a new run.  The counts of two vectors share a word
+    // (16 bits each: a warp holds at most 512 elements of one j).
+    unsigned int keep[NV], packed[NV / 2];
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+        T before = shfl_value_up(v[j].t[VEC - 1]);
+        if (lane == 0) before = left;
+        left = shfl_value_last(v[j].t[VEC - 1]);
+        unsigned int m = 0u;
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) {
+            const int at = warp_first + (j * 32 + lane) * VEC + e;
+            const bool first = base == 0 && at == 0;
+            if (at < remaining && (first || !SameValue<T>::eq(v[j].t[e], e == 0 ? before : v[j].t[e == 0 ? 0 : e - 1]))) m |= 1u << e;
         }
+        keep[j] = m;
+        if (j & 1) packed[j / 2] |= (unsigned int)__popc(m) << 16;
+        else packed[j / 2] = (unsigned int)__popc(m);
     }
-
-    // block scan of the per-thread counts
-    unsigned int incl = count;
+    unsigned int incl[NV / 2];
 #pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const unsigned int up = __shfl_up_sync(0xffffffffu, incl, d);
-        if (lane >= d) incl += up;
+    for (int q = 0; q < NV / 2; ++q) incl[q] = packed[q];
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1)
+#pragma unroll
+        for (int q = 0; q < NV / 2; ++q) {
+            const unsigned int up = __shfl_up_sync(0xffffffffu, incl[q], d);
+            if (lane >= d) incl[q] += up;
+        }
+    unsigned int local[NV];  // survivors of the warp in front of this lane's vector j
+    unsigned int chunk = 0u;
+#pragma unroll
+    for (int q = 0; q < NV / 2; ++q) {
+        const unsigned int total = __shfl_sync(0xffffffffu, incl[q], 31);
+        const unsigned int excl = incl[q] - packed[q];
+        local[2 * q] = chunk + (excl & 0xffffu);
+        chunk += total & 0xffffu;
+        local[2 * q + 1] = chunk + (excl >> 16);
+        chunk += total >> 16;
     }
-    if (lane == 31) warp_total[warp] = incl;
+    if (lane == 31) warp_total[warp] = chunk;
     __syncthreads();
     if (warp == 0) {
-        unsigned int wt = lane < kUniqueThreads / 32 ? warp_total[lane] : 0u;
+        unsigned int wt = lane < WARPS ? warp_total[lane] : 0u;
         unsigned int wi = wt;
 #pragma unroll
-        for (int d = 1; d < kUniqueThreads / 32; d <<= 1) {
+        for (int d = 1; d < WARPS; d <<= 1) {
             const unsigned int up = __shfl_up_sync(0xffffffffu, wi, d);
             if (lane >= d) wi += up;
         }
-        if (lane < kUniqueThreads / 32) warp_excl[lane] = wi - wt;
-        const unsigned int aggregate = __shfl_sync(0xffffffffu, wi, kUniqueThreads / 32 - 1);
+        if (lane < WARPS) warp_excl[lane] = wi - wt;
+        const unsigned int aggregate = __shfl_sync(0xffffffffu, wi, WARPS - 1);
 
         TileState<unsigned int> state(state_base, num_tiles);
         unsigned int prefix = 0u;
@@ -117,20 +184,30 @@ unique_select_kernel(const T *__restrict__ in, int64_t n, T *__restrict__ kept, 
         }
         if (lane == 0) {
             s_prefix = prefix;
+            s_count = aggregate;
             if (tile == num_tiles - 1) *out_count = (long long)prefix + aggregate;
         }
     }
     __syncthreads();
 
-    unsigned int pos = s_prefix + warp_excl[warp] + (incl - count);
+    const unsigned int first_slot = warp_excl[warp];
 #pragma unroll
-    for (int k = 0; k < kUniqueItems; ++k) {
-        if ((keep_mask >> k) & 1u) {
-            kept[pos] = item[k];
-            if (starts) starts[pos] = first + k;  // where the run begins (run-length encoding)
-            ++pos;
+    for (int j = 0; j < NV; ++j) {
+        unsigned int slot = first_slot + local[j];
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) {
+            if ((keep[j] >> e) & 1u) {
+                survivors[slot] = v[j].t[e];
+                // where the run begins (run-length encoding)
+                if (starts) starts[(int64_t)s_prefix + slot] = base + warp_first + (j * 32 + lane) * VEC + e;
+                ++slot;
+            }
         }
     }
+    __syncthreads();
+    const unsigned int count = s_count;
+    T *to = kept + s_prefix;
+    for (unsigned int i = tid; i < count; i += kUniqueThreads) to[i] = survivors[i];
 }
 
 // lengths[r] = distance from the start of run r to the start of the next run (or to n).
@@ -142,39 +219,24 @@ run_lengths_kernel(const long long *starts, const long long *count, long long n,
         lengths[r] = (r + 1 < m ? starts[r + 1] : n) - starts[r];
 }
 
-template <typename T>
-__global__ void __launch_bounds__(256)
-unique_copy_back_kernel(T *data, const T *kept, const long long *count) {
-    const long long m = *count;
-    const long long step = (long long)gridDim.x * blockDim.x;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += step) data[i] = kept[i];
-}
-
 struct UniqueLayout {
-    int64_t tiles, off_state, off_kept, total;
+    int64_t tiles, off_state, total;
 };
 
 static UniqueLayout unique_layout(int elem_bytes, int64_t n) {
     UniqueLayout L;
-    L.tiles = ceil_div(n < 1 ? 1 : n, kUniqueTile);
+    L.tiles = ceil_div((n < 1 ? 1 : n) * elem_bytes, kUniqueTileBytes);
     L.off_state = sizeof(TempHeader);
-    L.off_kept = L.off_state + round_up(L.tiles * kDescStride, 256);
-    L.total = L.off_kept + round_up((n < 1 ? 1 : n) * elem_bytes, 256);
+    L.total = L.off_state + round_up(L.tiles * kDescStride, 256);
     return L;
 }
 
 template <typename T>
 static int run_unique(cudaStream_t s, void *data, int64_t n, void *out_count, void *temp, const UniqueLayout &L) {
     char *t = (char *)temp;
-    B200ALG_CUDA_TRY(cudaMemsetAsync(temp, 0, (size_t)L.off_kept, s));
-    unique_select_kernel<T><<<(int)L.tiles, kUniqueThreads, 0, s>>>((const T *)data, n, (T *)(t + L.off_kept), nullptr,
-                                                                  (long long *)out_count, (TempHeader *)temp, t + L.off_state,
-                                                                  (int)L.tiles);
-    B200ALG_LAUNCH_CHECK();
-    int64_t want = ceil_div(n, 256 * 8);
-    const int64_t cap = (int64_t)sm_count() * 8;
-    const int blocks = (int)(want < 1 ? 1 : (want > cap ? cap : want));
-    unique_copy_back_kernel<T><<<blocks, 256, 0, s>>>((T *)data, (const T *)(t + L.off_kept), (const long long *)out_count);
+    B200ALG_CUDA_TRY(cudaMemsetAsync(temp, 0, (size_t)L.total, s));
+    unique_select_kernel<T><<<(int)L.tiles, kUniqueThreads, 0, s>>>((const T *)data, n, (T *)data, nullptr, (long long *)out_count,
+                                                                  (TempHeader *)temp, t + L.off_state, (int)L.tiles);
     B200ALG_LAUNCH_CHECK();
     return B200ALG_OK;
 }
@@ -184,9 +246,9 @@ static int run_unique(cudaStream_t s, void *data, int64_t n, void *out_count, vo
 struct RunLengthLayout {
     int64_t tiles, off_state, off_starts, total;
 };
-static RunLengthLayout run_length_layout(int64_t n) {
+static RunLengthLayout run_length_layout(int elem_bytes, int64_t n) {
     RunLengthLayout L;
-    L.tiles = ceil_div(n < 1 ? 1 : n, kUniqueTile);
+    L.tiles = ceil_div((n < 1 ? 1 : n) * elem_bytes, kUniqueTileBytes);
     L.off_state = sizeof(TempHeader);
     L.off_starts = L.off_state + round_up(L.tiles * kDescStride, 256);
     L.total = L.off_starts + round_up((n < 1 ? 1 : n) * 8, 256);
@@ -219,7 +281,7 @@ extern "C" int b200alg_run_length_encode_temp_bytes(int dtype, int64_t n, int64_
     if (!out_bytes || n < 0) return B200ALG_INVALID_ARGUMENT;
     if (dtype_bytes(dtype) == 0) return B200ALG_UNSUPPORTED;
     if (n > kMaxElements) return B200ALG_TOO_LARGE;
-    *out_bytes = run_length_layout(n).total;
+    *out_bytes = run_length_layout(dtype_bytes(dtype), n).total;
     return B200ALG_OK;
 }
 
@@ -236,7 +298,7 @@ extern "C" int b200alg_run_length_encode(void *stream, const void *data, int64_t
     if (es == 0) return B200ALG_UNSUPPORTED;
     if (n > kMaxElements) return B200ALG_TOO_LARGE;
     if (((uintptr_t)data % es) || ((uintptr_t)values % es) || ((uintptr_t)lengths % 8) || ((uintptr_t)temp % 256)) return B200ALG_MISALIGNED;
-    const RunLengthLayout L = run_length_layout(n);
+    const RunLengthLayout L = run_length_layout(dtype_bytes(dtype), n);
     if (temp_bytes < L.total) return B200ALG_TEMP_TOO_SMALL;
     cudaStream_t s = (cudaStream_t)stream;
     switch (dtype) {

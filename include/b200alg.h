@@ -211,8 +211,8 @@ int b200alg_sequence(void *stream, void *view, int64_t n, int dtype, int64_t sta
  * ComparisonOperations.tt): removes consecutive duplicates of data[0..n) in place and stores
  * the number of elements left in out_count[0] (int64, device).  Integers compare by value;
  * floating-point values are equal when numerically equal or both NaN (CompareTo).  temp
- * holds the survivors before they are copied back, so it grows with n (the reference's
- * ComputeUniqueTempStorageSize is one int because its kernel is a serial chain of groups). */
+ * holds one record per 32 KB of data (the reference's ComputeUniqueTempStorageSize is one
+ * int because its kernel is a serial chain of groups). */
 int b200alg_unique_temp_bytes(int dtype, int64_t n, int64_t *out_bytes);
 int b200alg_unique(void *stream, void *data, int64_t n, int dtype, void *out_count, void *temp, int64_t temp_bytes);
 
