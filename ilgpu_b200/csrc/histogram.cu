@@ -6,7 +6,12 @@
 // HistogramIncrement* (HistogramOperations.tt:30-41).
 #include "common.cuh"
 
+#include <cooperative_groups.h>
+#include <type_traits>
+
 namespace b200alg {
+
+namespace cg = cooperative_groups;
 
 constexpr int kHistThreads = 512;
 constexpr int kHistWarps = kHistThreads / 32;
@@ -187,6 +192,144 @@ histogram_smem_kernel(const T *__restrict__ in, int64_t stride, int64_t n, LocPa
     if (overflow && __syncthreads_or(of) && threadIdx.x == 0) atomicOr(overflow, 1);
 }
 
+// ---- one table per SM, for more bins than the kernel above holds ------------------------
+// One 1024-thread block per SM keeps a table of all bins in most of the SM's shared memory:
+// 32-bit counters, or, when those do not fit, 16-bit counters two to a word.  The blocks of a
+// cluster add their tables up through distributed shared memory before they are flushed with one
+// atomic per non-empty bin and cluster.  Bound: HBM for long inputs, the flush for short ones.
+//
+// 16-bit counters are below 2^14 at the start of a chunk of 3 * 2^14 elements, so they cannot
+// wrap inside it; a sweep over the table after every chunk moves what a counter holds above that
+// to the global bin.  (Counting with an atomic that returns the old value finds those counters
+// without a sweep, but took twice as long per element.)
+constexpr int kTableThreads = 1024;
+constexpr int kTableBytes = 224 * 1024;
+constexpr int kTableChunk = 3 << 14;   // elements of a block between two sweeps
+constexpr int kTableMaxCluster = 4;
+
+// Which kernel: the table where bins are many and the elements enough to pay for the flush.  Below
+// 16 elements per bin one global atomic per element is as fast (65536 bins: 16.5 us both ways at
+// 2^20 elements; 47 us against 377 us at 3 * 10^7); up to 1024 bins the kernel above, whose smaller
+// blocks are cleared and flushed sooner, unless the input does not fit in L2 and its locator does
+// more than a few float operations per element (2^26 doubles, 256 bins: 85 us against 97 us; floats
+// are at the HBM rate either way).
+constexpr int64_t kTableLongInput = 1ll << 27;  // bytes
+template <typename T, int LOCATOR> bool use_table(int64_t nb, int64_t n, bool dense) {
+    if (nb * 2 > kTableBytes || n < 16 * nb) return false;
+    if (!dense) return nb * 4 > kHistSmemBytes;  // few loads in flight here
+    const bool costly = !(std::is_same<T, float>::value && LOCATOR == B200ALG_LOCATOR_EQUAL_WIDTH_CLAMP);
+    return (nb > 1024 && n >= (1 << 17)) || (costly && n * (int64_t)sizeof(T) >= kTableLongInput);
+}
+
+template <typename T, int LOCATOR, bool HALVES>
+__global__ void __launch_bounds__(kTableThreads)
+histogram_table_kernel(const T *__restrict__ in, int64_t stride, int64_t n, LocParams p, void *bins, int bin_dtype, int *overflow) {
+    extern __shared__ __align__(16) unsigned int table[];
+    const int nb = (int)p.num_bins;
+    const int quads = ((HALVES ? (nb + 1) / 2 : nb) + 3) / 4;  // 16-byte pieces of the table
+    uint4 *table4 = reinterpret_cast<uint4 *>(table);
+    for (int i = threadIdx.x; i < quads; i += kTableThreads) table4[i] = make_uint4(0u, 0u, 0u, 0u);
+    __syncthreads();
+    bool of = false;
+    auto count = [&](T x) {
+        const int b = Locate<T, LOCATOR>::run(x, p);
+        if (!Locate<T, LOCATOR>::kInRange && (unsigned int)b >= (unsigned int)nb) return;
+        if (HALVES) atomicAdd(table + (b >> 1), (b & 1) ? 0x10000u : 1u);
+        else atomicAdd(table + b, 1u);  // lanes that meet in one bin cost little: they all add one
+    };
+    auto sweep = [&]() {
+        __syncthreads();
+        for (int i = threadIdx.x; i < quads; i += kTableThreads) {
+            const uint4 q = table4[i];
+            if ((q.x | q.y | q.z | q.w) & 0xC000C000u) {
+                const unsigned int w[4] = {q.x & 0xC000C000u, q.y & 0xC000C000u, q.z & 0xC000C000u, q.w & 0xC000C000u};
+#pragma unroll 1
+                for (int k = 0; k < 8; ++k) {
+                    const unsigned int c = (w[k >> 1] >> ((k & 1) * 16)) & 0xFFFFu;
+                    if (c) of |= add_to_bin(bins, i * 8 + k, c, bin_dtype);
+                }
+                table4[i] = make_uint4(q.x & 0x3FFF3FFFu, q.y & 0x3FFF3FFFu, q.z & 0x3FFF3FFFu, q.w & 0x3FFF3FFFu);
+            }
+        }
+        __syncthreads();
+    };
+    if (stride == 1) {
+        constexpr int VEC = 16 / sizeof(T);
+        union V { uint4 u; T t[VEC]; };
+        int64_t head = (int64_t)(((16u - (unsigned)((uintptr_t)in & 15u)) & 15u) / sizeof(T));
+        if (head > n) head = n;
+        const uint4 *vin = reinterpret_cast<const uint4 *>(in + head);
+        const int64_t nvec = (n - head) / VEC;
+        const int64_t tail = head + nvec * VEC;
+        constexpr int NV = 4;  // 16-byte loads in flight per thread
+        constexpr int ROUND = kTableThreads * NV * VEC;  // elements of a block per round
+        static_assert(kTableChunk >= ROUND, "a chunk is whole rounds");
+        const int64_t step = (int64_t)gridDim.x * kTableThreads;
+        int pending = 0;
+        for (int64_t first = (int64_t)blockIdx.x * kTableThreads; first < nvec; first += NV * step) {
+            const uint4 *from = vin + first + threadIdx.x;
+            V v[NV];
+            if (first + (NV - 1) * step + kTableThreads <= nvec) {  // bounds checks cost as much as the counting
+#pragma unroll
+                for (int k = 0; k < NV; ++k) v[k].u = __ldcs(from + k * step);
+#pragma unroll
+                for (int k = 0; k < NV; ++k)
+#pragma unroll
+                    for (int e = 0; e < VEC; ++e) count(v[k].t[e]);
+            } else {
+#pragma unroll 1
+                for (int k = 0; k < NV; ++k)
+                    if (first + threadIdx.x + k * step < nvec) {
+                        v[0].u = __ldcs(from + k * step);
+#pragma unroll
+                        for (int e = 0; e < VEC; ++e) count(v[0].t[e]);
+                    }
+            }
+            if (HALVES) {
+                pending += ROUND;
+                if (pending > kTableChunk - ROUND) {
+                    sweep();
+                    pending = 0;
+                }
+            }
+        }
+        if (blockIdx.x == 0) {  // the unaligned ends: fewer than 16 bytes each
+            if (HALVES) sweep();
+            if (threadIdx.x < head) count(in[threadIdx.x]);
+            if (tail + threadIdx.x < n) count(in[tail + threadIdx.x]);
+        }
+    } else {
+        int pending = 0;
+        for (int64_t first = (int64_t)blockIdx.x * kTableThreads; first < n; first += (int64_t)gridDim.x * kTableThreads) {
+            if (first + threadIdx.x < n) count(in[(first + threadIdx.x) * stride]);
+            if (HALVES && (pending += kTableThreads) == kTableChunk) {
+                sweep();
+                pending = 0;
+            }
+        }
+    }
+    // every block of the cluster flushes its share of the bins
+    cg::cluster_group cluster = cg::this_cluster();
+    cluster.sync();
+    const int blocks = (int)cluster.num_blocks();
+    const int share = ((nb + blocks - 1) / blocks + 1) / 2 * 2;
+    const int lo = (int)cluster.block_rank() * share;
+    const int hi = lo + share < nb ? lo + share : nb;
+    const unsigned int *peer[kTableMaxCluster];
+#pragma unroll
+    for (int r = 0; r < kTableMaxCluster; ++r) peer[r] = cluster.map_shared_rank(table, r < blocks ? r : 0);
+#pragma unroll 2
+    for (int b = lo + threadIdx.x; b < hi; b += kTableThreads) {
+        unsigned long long c = 0ull;
+#pragma unroll
+        for (int r = 0; r < kTableMaxCluster; ++r)
+            if (r < blocks) c += HALVES ? (peer[r][b >> 1] >> ((b & 1) * 16)) & 0xFFFFu : peer[r][b];
+        if (c) of |= add_to_bin(bins, b, c, bin_dtype);
+    }
+    cluster.sync();  // nobody leaves while its table is being read
+    if (overflow && __syncthreads_or(of) && threadIdx.x == 0) atomicOr(overflow, 1);
+}
+
 // ---- fallback for bin counts that do not fit in shared memory ---------------------------
 template <typename T, int LOCATOR>
 __global__ void __launch_bounds__(256)
@@ -205,7 +348,8 @@ template <typename T, int LOCATOR>
 static int launch_histogram(cudaStream_t s, const void *in, int64_t stride, int64_t n, const LocParams &p, void *bins,
                             int bin_dtype, void *overflow) {
     const int64_t nb = p.num_bins;
-    if (nb * 4 <= kHistSmemBytes) {
+    const bool table = use_table<T, LOCATOR>(nb, n, stride == 1);
+    if (nb * 4 <= kHistSmemBytes && !table) {
         int replicas = 1;
         while (replicas < 32 && (int64_t)replicas * 2 * nb * 4 <= kHistSmemBytes) replicas *= 2;
         const size_t smem = (size_t)replicas * nb * 4;
@@ -218,6 +362,38 @@ static int launch_histogram(cudaStream_t s, const void *in, int64_t stride, int6
             histogram_smem_kernel<T, LOCATOR, true><<<blocks, kHistThreads, smem, s>>>((const T *)in, 1, n, p, bins, bin_dtype, (int *)overflow, replicas);
         else
             histogram_smem_kernel<T, LOCATOR, false><<<blocks, kHistThreads, smem, s>>>((const T *)in, stride, n, p, bins, bin_dtype, (int *)overflow, replicas);
+    } else if (table) {
+        const bool halves = nb * 4 > kTableBytes;
+        const size_t smem = (size_t)round_up(halves ? (nb + 1) / 2 * 4 : nb * 4, 16);
+        auto kernel = halves ? histogram_table_kernel<T, LOCATOR, true> : histogram_table_kernel<T, LOCATOR, false>;
+        // Clusters of four leave some SMs without one (their GPC holds no multiple of four) but
+        // quarter the flush; long inputs would rather have every SM.
+        const bool big = n * (int64_t)sizeof(T) >= kTableLongInput;
+        const unsigned int cluster = big ? 2 : kTableMaxCluster;
+        static ContextCache<int> resident[4];
+        int blocks = 0;
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = cluster;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.blockDim = dim3(kTableThreads);
+        cfg.stream = s;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        if (!resident[halves * 2 + big].find(&blocks)) {
+            B200ALG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTableBytes));
+            cfg.gridDim = dim3(cluster);
+            cfg.dynamicSmemBytes = kTableBytes;
+            int clusters = 0;
+            B200ALG_CUDA_TRY(cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg));
+            if (clusters < 1) return B200ALG_UNSUPPORTED;
+            blocks = clusters * (int)cluster;
+            resident[halves * 2 + big].store(blocks);
+        }
+        cfg.gridDim = dim3(blocks);
+        cfg.dynamicSmemBytes = smem;
+        B200ALG_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, (const T *)in, stride, n, p, bins, bin_dtype, (int *)overflow));
     } else {
         int64_t want = ceil_div(n, 256 * 4);
         const int64_t cap = (int64_t)sm_count() * 8;
