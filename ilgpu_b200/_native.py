@@ -75,6 +75,14 @@ MG_SIGNATURES = {
 
 _lib = None
 _mg_lib = None
+_host = None
+
+# what csrc/host_calls.cpp calls, in the order of its table
+_HOST_ENTRY_POINTS = (
+    "b200alg_radix_sort_temp_bytes", "b200alg_radix_sort_keys", "b200alg_radix_sort_pairs", "b200alg_radix_sort_pairs_sequence",
+    "b200alg_scan_temp_bytes", "b200alg_scan_carry", "b200alg_reduce", "b200alg_histogram", "b200alg_initialize",
+    "b200alg_unique_temp_bytes", "b200alg_unique",
+)
 
 
 class NativeLibraryMissing(RuntimeError):
@@ -113,6 +121,20 @@ def lib() -> ctypes.CDLL:
             fn.argtypes = args
         _lib = L
     return _lib
+
+
+def host():
+    """The native host path of the mirror's calls (csrc/host_calls.cpp), bound to lib()."""
+    global _host
+    if _host is None:
+        L = lib()
+        try:
+            from . import _host as module
+        except ImportError as e:
+            raise NativeLibraryMissing(f"ilgpu_b200/_host.so: {e}; build it with `make -C ilgpu_b200/csrc`") from e
+        module.bind(tuple(ctypes.cast(getattr(L, name), ctypes.c_void_p).value for name in _HOST_ENTRY_POINTS))
+        _host = module
+    return _host
 
 
 def status_string(status: int) -> str:

@@ -274,6 +274,9 @@ class Accelerator:
             raise InvalidOperationException("no CUDA device: this path has no CPU fallback")
         self.device = torch.device("cuda", device) if isinstance(device, int) else torch.device(device)
         self.L = N.lib()
+        # host path of the calls below: it does what the Python code after it does, for valid arguments
+        self._host = N.host()
+        self._index = -1 if self.device.index is None else self.device.index
 
     # -- memory / streams (plumbing) --
     def Allocate1D(self, length: int, dtype: torch.dtype) -> torch.Tensor:
@@ -312,7 +315,11 @@ class Accelerator:
         code = dtype_code(operation.dtype)
         order = (N.SORT_DESCENDING if operation.descending else 0) | (N.SORT_FLOAT_TOTAL_ORDER if float_total_order else 0)
 
+        fast, index = self._host.sort_keys, self._index
+
         def sort(stream, view, temp):
+            if fast(index, code, order, stream, view, temp):
+                return
             _check_view(view, "view", operation.dtype)
             n = view.numel()
             if n > 2**31 - 1:
@@ -334,7 +341,11 @@ class Accelerator:
         code = dtype_code(operation.dtype)
         order = (N.SORT_DESCENDING if operation.descending else 0) | (N.SORT_FLOAT_TOTAL_ORDER if float_total_order else 0)
 
+        fast, index = self._host.sort_pairs, self._index
+
         def sort_sequenced(stream, keys, values, seq, temp):
+            if isinstance(seq, Sequencer) and fast(index, code, order, dtype_code(seq.dtype), stream, keys, values, temp):
+                return
             if not isinstance(seq, Sequencer):
                 raise NotSupportedException("only the built-in sequencers cross the native boundary")
             _check_view(keys, "keys", operation.dtype)
@@ -356,6 +367,8 @@ class Accelerator:
             return sort_sequenced
 
         def sort(stream, keys, values, temp):
+            if fast(index, code, order, -1, stream, keys, values, temp):
+                return
             _check_view(keys, "keys", operation.dtype)
             _check_view(values, "values")
             n = keys.numel()
@@ -389,7 +402,11 @@ class Accelerator:
         code = dtype_code(operation.dtype)
         inclusive = 1 if kind == ScanKind.Inclusive else 0
 
+        fast, index, op = self._host.scan, self._index, operation.op
+
         def scan(stream, input, output, temp, carry_in=None):
+            if carry_in is None and fast(index, code, op, inclusive, stream, input, output, temp):
+                return
             # order and kinds of the checks: ScanExtensions.cs:675-689
             _check_view(input, "input", operation.dtype)
             _check_view(output, "output", operation.dtype)
@@ -416,7 +433,11 @@ class Accelerator:
         ReductionExtensions.cs:30-35)."""
         code = dtype_code(operation.dtype)
 
+        fast, index, op = self._host.reduce, self._index, operation.op
+
         def reduce(stream, input, output):
+            if fast(index, code, op, stream, input, output):
+                return
             # ReductionExtensions.cs:146-153
             if input is None:
                 raise ArgumentNullException("input")
@@ -438,6 +459,13 @@ class Accelerator:
         """With ``output``: asynchronous (ReductionExtensions.cs:180-196).  Without: allocates
         one element, reduces, copies it to the CPU - that synchronises - and returns the
         value (ReductionExtensions.cs:198-216)."""
+        if output is not None:
+            if self._host.reduce(self._index, dtype_code(operation.dtype), operation.op, stream, input, output):
+                return None
+        else:
+            value = self._host.reduce_value(self._index, dtype_code(operation.dtype), operation.op, stream, input)
+            if value is not None:
+                return value
         reduce = self.CreateReduction(operation)
         if output is not None:
             reduce(stream, input, output)
@@ -450,7 +478,11 @@ class Accelerator:
     def CreateHistogram(self, locator, checked: bool = True):
         """Returns ``histogram(stream, view, histogram, histogramOverflow)``
         (HistogramExtensions.cs:293-354); the unchecked variant (:371-427) takes no overflow view."""
+        fast, index, where, lo, hi = self._host.histogram, self._index, locator.code, float(locator.lo), float(locator.hi)
+
         def run(stream, view, histogram, histogramOverflow=None):
+            if checked == (histogramOverflow is not None) and fast(index, where, lo, hi, stream, view, histogram, histogramOverflow):
+                return
             # HistogramExtensions.cs:322-338
             _check_view(view, "view")
             _check_view(histogram, "histogram")
@@ -514,6 +546,10 @@ class Accelerator:
     def Unique(self, stream, input: torch.Tensor) -> int:
         """Allocates output and temp, runs, copies the count back - which synchronises
         (UniqueExtensions.cs:200-220)."""
+        if isinstance(input, torch.Tensor):
+            count = self._host.unique(self._index, _TORCH_TO_CODE.get(input.dtype, -1), stream, input)
+            if count is not None:
+                return count
         output = self.Allocate1D(1, torch.int64)
         temp = self.Allocate1D(self.ComputeUniqueTempStorageSize(input.dtype, input.numel()), torch.int32)
         self.CreateUnique(input.dtype)(stream, input, output, temp)
@@ -522,6 +558,8 @@ class Accelerator:
     # -- edges of the path --
     def Initialize(self, stream, view: torch.Tensor, value) -> None:
         """InitializeExtensions.cs: fills the view with one value."""
+        if self._host.initialize(self._index, stream, view, value):
+            return
         _check_view(view, "view")
         host = torch.tensor([value], dtype=view.dtype)
         with self.Bind():
