@@ -3,10 +3,11 @@
 //   1. one pass over the keys builds the histograms of ALL digit positions,
 //   2. a one-block kernel turns them into global digit offsets and finds digit positions
 //      on which every key agrees (those passes are skipped),
-//   3. one kernel per remaining digit position: a tile of keys is ranked in shared memory
-//      (the lanes of a warp meet in per-warp digit tables), the tile's digit counts are chained to the previous tiles'
-//      with decoupled look-back, and the tile is scattered to its final place for that
-//      digit - each key is read once and written once per pass.
+//   3. one kernel per remaining digit position moves every key to its final place for that digit, each
+//      key read once and written once (digit_pass.cuh).
+//
+// The partition of a multi-GPU sort is a pass of its own kind (a bucket of a splitter list instead of
+// a digit); its tiles are chained with decoupled look-back.
 //
 // Replaces RadixSortKernel1 / RadixSortKernel2 and the host loop around them
 // (RadixSortExtensions.cs:660-738, :852-912, :1276-1334: 2 bits per pass, 4 launches per
@@ -30,7 +31,8 @@ enum : int {
     kCtlFinal = 24,        // buffer the sorted data ended in (kBufOut: nothing left to do)
     kCtlFirstPass = 25,    // first pass that runs (kNoPass when every pass is skipped)
     kCtlDst = 32,          // [32..39] buffer this pass writes
-    kCtlStatusHalf = 40    // [40..47] which of the two look-back arrays this pass uses
+    kCtlStatusHalf = 40,   // [40..47] which of the two look-back arrays this pass uses
+    kCtlRole = 48          // [48..55] blocks of this pass that have started
 };
 // The three buffers a sort moves its data between.
 enum : unsigned int { kBufIn = 0, kBufOut = 1, kBufAlt = 2 };
@@ -238,7 +240,7 @@ sort_offsets_kernel(const unsigned long long *ghist, unsigned long long *gbase, 
     }
 }
 
-// ---- 3. one digit pass -------------------------------------------------------------------
+// ---- 3. the partition pass -------------------------------------------------------------------
 // Look-back words: the top two bits carry the state, the rest the count.
 template <typename SW> struct StatusWord;
 template <> struct StatusWord<unsigned int> {
@@ -252,21 +254,11 @@ template <> struct StatusWord<unsigned long long> {
     static __device__ __forceinline__ unsigned long long ld(const unsigned long long *p) { return ld_relaxed_u64(p); }
 };
 
-// What a pass partitions by.  RadixDigit: one 8-bit digit of the transformed key.
-// SplitterBucket: the number of splitters that are <= (key, global index) in the order
+// What the partition of a multi-GPU sort goes by: the number of splitters that are <= (key, global index) in the order
 // (transformed key, index) - used to split a shard into per-rank buckets before the
 // all-to-all of a multi-GPU sort; ties between equal keys are broken by position, which
 // keeps the partition balanced under heavy duplicates and stable.
-template <typename K, typename XF = KeyXform<K>> struct RadixDigit {
-    static constexpr bool kUsesIndex = false;
-    XF xf;
-    int shift;
-    __device__ __forceinline__ unsigned int operator()(K key, int64_t, const unsigned char *) const {
-        return (unsigned int)(xf(key) >> shift) & 0xFFu;
-    }
-};
 template <typename K> struct SplitterBucket {
-    static constexpr bool kUsesIndex = true;
     static constexpr int kSmall = 7;  // up to this many splitters are compared without a loop
     // The tables a block keeps in shared memory (16-byte aligned), by byte offset: splitter
     // indices, transformed splitter keys, then (partition pass only) the destination pointers.
@@ -381,17 +373,14 @@ template <> struct ValueBytes<NoValue> { static constexpr int value = 0; };
 template <typename SW> struct IndexOf { using type = unsigned int; };
 template <> struct IndexOf<unsigned long long> { using type = unsigned long long; };
 
-// Full dense tiles are staged in shared memory by one bulk asynchronous copy (TMA, no
+// Full dense tiles of the partition are staged in shared memory by one bulk asynchronous copy (TMA, no
 // multicast) that is issued a tile ahead.  (Measured against plain loads of the next tile into
-// registers during the write-out: 1.22 ms against 1.31 ms for the 2^26-key sort.)
+// registers during the write-out: 7 % slower.)
 constexpr bool kSortTma = true;
 constexpr int kLookWindow = 4;  // predecessors examined per look-back round (2 and 8 measured slower)
-// The digit passes are launched as programmatic dependents of one another: the blocks of the
-// next pass move in as those of this one leave and do their set-up before they wait for it.
-constexpr bool kSortPdl = true;
 
-template <typename K, typename V, bool KEEP_DIGITS, int THREADS, int ITEMS>
-struct OnesweepSmem {
+template <typename K, typename V, int THREADS, int ITEMS>
+struct PartitionSmem {
     static constexpr int TILE = THREADS * ITEMS;
     static constexpr int WARPS = THREADS / 32;
     static constexpr int VB = ValueBytes<V>::value;
@@ -406,7 +395,7 @@ struct OnesweepSmem {
     // when two blocks per SM would not fit otherwise, the masks live at the head of the
     // reorder buffer (and every warp clears its row again before it ranks the next tile).
     static constexpr size_t table_bytes = (size_t)WARPS * kRadix * 4;
-    static constexpr size_t fixed_bytes = kRadix * 16 + 256 + (KEEP_DIGITS ? (size_t)TILE + kRadix * 32 : 0) + 128;
+    static constexpr size_t fixed_bytes = kRadix * 16 + 256 + (size_t)TILE + kRadix * 32 + 128;
     static constexpr bool MASKS_IN_SORTED =
         (size_t)TILE * SLOT >= table_bytes &&
         (size_t)TILE * SLOT + 2 * table_bytes + fixed_bytes + (size_t)TILE * sizeof(K) > 112 * 1024;
@@ -418,9 +407,9 @@ struct OnesweepSmem {
     static constexpr size_t off_misc = off_goff + kRadix * 8;
     static constexpr size_t off_context = off_misc + 128;   // the block's PassContext
     static constexpr size_t off_digits = off_context + 128;
-    static constexpr size_t off_splitters = off_digits + (KEEP_DIGITS ? (size_t)TILE : 0);
+    static constexpr size_t off_splitters = off_digits + (size_t)TILE;
     // splitters: 256 positions (8 bytes), 256 keys (8 bytes), 2 x 256 destination pointers
-    static constexpr size_t off_stage = (off_splitters + (KEEP_DIGITS ? (size_t)kRadix * 32 : 0) + 127) / 128 * 128;
+    static constexpr size_t off_stage = (off_splitters + (size_t)kRadix * 32 + 127) / 128 * 128;
     // The staging buffer of the bulk copies is dropped (keys are then loaded directly) where
     // it would cost the second block per SM.
     static constexpr size_t kTwoBlocksPerSm = 113 * 1024;
@@ -439,7 +428,6 @@ template <typename K, typename V, typename SW> struct PassContext {
     int num_tiles;
     bool dense;   // the source is contiguous
     bool bulk;    // full tiles of the source can be staged by bulk copies (dense, 16-byte aligned)
-    int value_seq;  // not kSeqNone: this pass makes the values from the element index instead of reading them
     TempHeader *hdr;
     unsigned int *ticket;
     const unsigned long long *gbase;
@@ -459,18 +447,18 @@ __device__ __forceinline__ int take_ticket(const PassContext<K, V, SW> &c, K *st
     return next;
 }
 
-// One tile of one digit pass; returns the block's next tile.  FAST = the tile is full and both
+// One tile of the partition; returns the block's next tile.  FAST = the tile is full and both
 // buffers are dense (no bounds checks, no stride arithmetic).  Keys are held in warp-striped
 // order: item i of lane l is element warp * 32 * ITEMS + i * 32 + l of the tile.
-template <typename K, typename V, typename SW, typename Digit, int THREADS, int ITEMS, bool FAST>
-__device__ __forceinline__ int onesweep_tile(const PassContext<K, V, SW> &c, int tile, unsigned int &bulk_phase,
-                                             K (&key)[ITEMS], bool &have_keys, const Digit &dg, unsigned char *smem_raw) {
+template <typename K, typename V, typename SW, int THREADS, int ITEMS, bool FAST>
+__device__ __forceinline__ int partition_tile(const PassContext<K, V, SW> &c, int tile, unsigned int &bulk_phase,
+                                             K (&key)[ITEMS], bool &have_keys, const SplitterBucket<K> &dg, unsigned char *smem_raw) {
     constexpr int WARPS = THREADS / 32;
     constexpr int TILE = THREADS * ITEMS;
     constexpr bool HAS_VALUES = ValueBytes<V>::value != 0;
     using S = StatusWord<SW>;
     using Idx = typename IndexOf<SW>::type;
-    using L = OnesweepSmem<K, V, Digit::kUsesIndex, THREADS, ITEMS>;
+    using L = PartitionSmem<K, V, THREADS, ITEMS>;
     K *skeys = reinterpret_cast<K *>(smem_raw + L::off_sorted);
     V *svals = reinterpret_cast<V *>(smem_raw + L::off_sorted + (L::SPLIT ? (size_t)TILE * sizeof(K) : 0));
     // count_tbl[w][d]: number, later first slot, of the d-keys of warp w; mask_tbl[w][d]: lanes of
@@ -565,7 +553,7 @@ __device__ __forceinline__ int onesweep_tile(const PassContext<K, V, SW> &c, int
             take_ranks(i, d, peers, true);
         }
     };
-    if constexpr (Digit::kUsesIndex) {
+    {
         // A partition into up to eight buckets.  Buckets first, for all items, without a branch; an
         // element whose key equals a splitter's (rare) is settled by its index afterwards.  With
         // two or four buckets the tables would serialise (all lanes of a bucket hit one word), so
@@ -592,7 +580,7 @@ __device__ __forceinline__ int onesweep_tile(const PassContext<K, V, SW> &c, int
 #pragma unroll
                 for (int i = 0; i < ITEMS; ++i)
                     if ((ties >> i) & 1u)
-                        packed[i] = Digit::resolve_tie(dg.xf, dg.index_base, dg.num_splitters, key[i], tile_base + warp_base + i * 32,
+                        packed[i] = SplitterBucket<K>::resolve_tie(dg.xf, dg.index_base, dg.num_splitters, key[i], tile_base + warp_base + i * 32,
                                                        tables, packed[i]);
             }
 #pragma unroll
@@ -619,29 +607,18 @@ __device__ __forceinline__ int onesweep_tile(const PassContext<K, V, SW> &c, int
         const int ns = dg.num_splitters;  // uniform over the grid
         if (ns <= 1) rank_few(std::integral_constant<int, 1>{});
         else if (ns <= 3) rank_few(std::integral_constant<int, 3>{});
-        else if (ns <= Digit::kSmall) rank_few(std::integral_constant<int, 7>{});
+        else if (ns <= SplitterBucket<K>::kSmall) rank_few(std::integral_constant<int, 7>{});
         else rank_by_tables();
-    } else {
-        rank_by_tables();
     }
     __syncthreads();  // A: the tables are complete; every thread has its keys out of the staging buffer
 
     // The values are not held during the ranking: sixteen more live registers there spill.
     V val[HAS_VALUES ? ITEMS : 1];
     if constexpr (HAS_VALUES) {  // requested now, in flight while the digit threads work, needed for the reorder
-        bool from_index = false;
-        if constexpr (sizeof(V) <= 8) from_index = c.value_seq != kSeqNone;
-        if (from_index) {
-            if constexpr (sizeof(V) <= 8) {
 #pragma unroll
-                for (int i = 0; i < ITEMS; ++i) val[i] = sequence_value<V>(c.value_seq, tile_base + warp_base + i * 32);
-            }
-        } else {
-#pragma unroll
-            for (int i = 0; i < ITEMS; ++i) {
-                const int local = warp_base + i * 32;
-                if (FAST || local < valid) val[i] = c.vsrc[tile_base + local];
-            }
+        for (int i = 0; i < ITEMS; ++i) {
+            const int local = warp_base + i * 32;
+            if (FAST || local < valid) val[i] = c.vsrc[tile_base + local];
         }
     }
 
@@ -690,9 +667,7 @@ __device__ __forceinline__ int onesweep_tile(const PassContext<K, V, SW> &c, int
         const unsigned int d = packed[i] & 0xFFu;
         const unsigned int slot = (packed[i] >> 8) + my_count[d];
         skeys[slot] = key[i];
-        if constexpr (Digit::kUsesIndex) {
-            if (dg.num_splitters > Digit::kSmall) sdigit[slot] = (unsigned char)d;  // few buckets: found again from the slot
-        }
+        if (dg.num_splitters > SplitterBucket<K>::kSmall) sdigit[slot] = (unsigned char)d;  // few buckets: found again from the slot
         if constexpr (L::SPLIT) svals[slot] = val[i];
         if constexpr (SECOND_ROUND) pos[i] = slot;
     }
@@ -764,10 +739,9 @@ __device__ __forceinline__ int onesweep_tile(const PassContext<K, V, SW> &c, int
 
     // With few buckets (the ranks of one box) the write-out goes bucket by bucket: a bucket is a
     // run of consecutive slots with one destination, so nothing is looked up per element.
-    bool few_buckets = false;
-    if constexpr (Digit::kUsesIndex) few_buckets = dg.num_splitters <= Digit::kSmall;
+    const bool few_buckets = dg.num_splitters <= SplitterBucket<K>::kSmall;
     auto store_runs = [&](bool keys_too, bool values_too) {
-        if constexpr (Digit::kUsesIndex) {
+        {
             const bool scattered = dg.bucket_keys != nullptr;
             // A run is stored so that every warp writes whole, aligned 128-byte lines of the
             // destination (the first lanes take the elements in front of the first line start):
@@ -788,7 +762,7 @@ __device__ __forceinline__ int onesweep_tile(const PassContext<K, V, SW> &c, int
                 const int lo = (int)bin_excl[b], hi = (int)bin_excl[b + 1];  // padding keys rank last
                 const Idx g = bin_goff[b];  // modulo 2^32 or 2^64: only g + p is an index
                 if (keys_too) {
-                    K *kd = scattered ? reinterpret_cast<K *>(Digit::key_pointer(tables, b)) : c.dst;
+                    K *kd = scattered ? reinterpret_cast<K *>(SplitterBucket<K>::key_pointer(tables, b)) : c.dst;
                     if (scattered || FAST) {
                         store_run(kd, skeys, lo, hi, g);
                     } else {
@@ -797,7 +771,7 @@ __device__ __forceinline__ int onesweep_tile(const PassContext<K, V, SW> &c, int
                 }
                 if constexpr (!std::is_same<V, NoValue>::value) {
                     if (values_too) {
-                        V *vd = scattered && dg.bucket_values ? reinterpret_cast<V *>(Digit::value_pointer(tables, b)) : c.vdst;
+                        V *vd = scattered && dg.bucket_values ? reinterpret_cast<V *>(SplitterBucket<K>::value_pointer(tables, b)) : c.vdst;
                         store_run(vd, svals, lo, hi, g);
                     }
                 }
@@ -813,14 +787,13 @@ __device__ __forceinline__ int onesweep_tile(const PassContext<K, V, SW> &c, int
             const int p = tid + i * THREADS;
             if (FAST || p < valid) {
                 const K k = skeys[p];
-                unsigned int d;
-                if constexpr (Digit::kUsesIndex) d = sdigit[p]; else d = dg(k, 0, tables);
+                const unsigned int d = sdigit[p];
                 const Idx at = bin_goff[d] + (Idx)p;
                 if constexpr (SECOND_ROUND) out_idx[i] = at;
                 bool stored = false;
-                if constexpr (Digit::kUsesIndex) {
+                {
                     if (dg.bucket_keys) {  // plain stores, possibly over NVLink into a peer's receive buffer
-                        reinterpret_cast<K *>(Digit::key_pointer(tables, d))[at] = k;
+                        reinterpret_cast<K *>(SplitterBucket<K>::key_pointer(tables, d))[at] = k;
                         stored = true;
                     }
                 }
@@ -829,9 +802,9 @@ __device__ __forceinline__ int onesweep_tile(const PassContext<K, V, SW> &c, int
                 }
                 if constexpr (L::SPLIT) {  // the value travels with its key
                     bool vstored = false;
-                    if constexpr (Digit::kUsesIndex) {
+                    {
                         if (dg.bucket_values) {
-                            reinterpret_cast<V *>(Digit::value_pointer(tables, d))[at] = svals[p];
+                            reinterpret_cast<V *>(SplitterBucket<K>::value_pointer(tables, d))[at] = svals[p];
                             vstored = true;
                         }
                     }
@@ -857,9 +830,9 @@ __device__ __forceinline__ int onesweep_tile(const PassContext<K, V, SW> &c, int
                 const int p = tid + i * THREADS;
                 if (FAST || p < valid) {
                     bool stored = false;
-                    if constexpr (Digit::kUsesIndex) {
+                    {
                         if (dg.bucket_values) {
-                            reinterpret_cast<V *>(Digit::value_pointer(tables, sdigit[p]))[out_idx[i]] = svals[p];
+                            reinterpret_cast<V *>(SplitterBucket<K>::value_pointer(tables, sdigit[p]))[out_idx[i]] = svals[p];
                             stored = true;
                         }
                     }
@@ -876,22 +849,20 @@ __device__ __forceinline__ int onesweep_tile(const PassContext<K, V, SW> &c, int
 // Persistent blocks.  Tiles are handed out by an atomic ticket, in order, so a tile only ever
 // waits for tiles whose blocks already run: forward progress does not depend on how many
 // blocks of the grid are resident.
-template <typename K, typename V, typename SW, typename Digit, int THREADS, int ITEMS>
+template <typename K, typename V, typename SW, int THREADS, int ITEMS>
 __global__ void __launch_bounds__(THREADS, 1024 / THREADS)
-onesweep_kernel(SortBuffers<K, V> io, int pass, Digit dg, TempHeader *hdr, const unsigned long long *gbase_all,
-                SW *status_all, int max_tiles, int value_seq) {
+partition_kernel(SortBuffers<K, V> io, int pass, SplitterBucket<K> dg, TempHeader *hdr, const unsigned long long *gbase_all,
+                SW *status_all, int max_tiles) {
     constexpr int TILE = THREADS * ITEMS;
     static_assert(THREADS >= 2 * kRadix, "one thread per digit for the offsets and one for the look-back");
-    using L = OnesweepSmem<K, V, Digit::kUsesIndex, THREADS, ITEMS>;
+    using L = PartitionSmem<K, V, THREADS, ITEMS>;
 
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    if (kSortPdl) grid_dependency_release();  // the next kernel of the call may take the SMs this one leaves
     {   // The part of the set-up that reads nothing: the lane masks of the ranking tables start at
         // zero and are left at zero by every item.
         uint4 *zm = reinterpret_cast<uint4 *>(smem_raw + L::off_mask);
         for (int i = threadIdx.x; i < (THREADS / 32) * kRadix / 4; i += THREADS) zm[i] = make_uint4(0u, 0u, 0u, 0u);
     }
-    if (kSortPdl) grid_dependency_wait();  // everything the kernels before this one wrote is visible from here on
     if (hdr->reserved[kCtlSkip + pass]) return;
     // The pass description lives in shared memory: a dozen pointers that would otherwise sit
     // in registers for the whole kernel.
@@ -912,7 +883,6 @@ onesweep_kernel(SortBuffers<K, V> io, int pass, Digit dg, TempHeader *hdr, const
         c.num_tiles = num_tiles;
         c.dense = io.stride == 1;
         c.bulk = c.dense && ((uintptr_t)c.src % 16 == 0);
-        c.value_seq = hdr->reserved[kCtlFirstPass] == (unsigned int)pass ? value_seq : kSeqNone;
         c.hdr = hdr;
         c.ticket = &hdr->reserved[kCtlTicket + pass];
         c.gbase = gbase_all + pass * kRadix;
@@ -928,8 +898,7 @@ onesweep_kernel(SortBuffers<K, V> io, int pass, Digit dg, TempHeader *hdr, const
         }
         misc[8] = (unsigned int)take_ticket<K, V, SW, TILE, L::STAGED>(c, reinterpret_cast<K *>(smem_raw + L::off_stage), bar);
     }
-    if constexpr (Digit::kUsesIndex)
-        dg.stage(smem_raw + L::off_splitters, true);
+    dg.stage(smem_raw + L::off_splitters, true);
     __syncthreads();
     int tile = (int)misc[8];
     __syncthreads();  // misc[8] is written again during the first tile
@@ -939,9 +908,9 @@ onesweep_kernel(SortBuffers<K, V> io, int pass, Digit dg, TempHeader *hdr, const
     bool have_keys = false;
     while (tile < num_tiles) {
         if (dense && (int64_t)(tile + 1) * TILE <= n)
-            tile = onesweep_tile<K, V, SW, Digit, THREADS, ITEMS, true>(c, tile, bulk_phase, key, have_keys, dg, smem_raw);
+            tile = partition_tile<K, V, SW, THREADS, ITEMS, true>(c, tile, bulk_phase, key, have_keys, dg, smem_raw);
         else
-            tile = onesweep_tile<K, V, SW, Digit, THREADS, ITEMS, false>(c, tile, bulk_phase, key, have_keys, dg, smem_raw);
+            tile = partition_tile<K, V, SW, THREADS, ITEMS, false>(c, tile, bulk_phase, key, have_keys, dg, smem_raw);
     }
 }
 
@@ -974,16 +943,22 @@ sort_copy_back_kernel(SortBuffers<K, V> io, const TempHeader *hdr, int value_seq
     }
 }
 
+}  // namespace b200alg
+
+#include "digit_pass.cuh"
+
+namespace b200alg {
+
 // ---- host side ---------------------------------------------------------------------------
 struct SortLayout {
     int passes;
     int tile;
     int64_t tiles;
     bool wide_status;
-    int64_t off_ghist, off_gbase, off_status, control_bytes, off_keys, off_values, total;
+    int64_t off_ghist, off_gbase, off_status, half_bytes, control_bytes, off_keys, off_values, total;
 };
 
-// Block shape of the digit pass: 512 threads, two blocks per SM, 8192 keys per tile (4096 for
+// Block shape of the partition pass: 512 threads, two blocks per SM, 8192 keys per tile (4096 for
 // 8-byte keys).  256- and 1024-thread blocks, 12 and 24 items per thread all measured slower.
 constexpr int kSortThreads = 512;
 constexpr int kSortItems = 16;
@@ -992,20 +967,29 @@ template <typename K> struct SortTuning {
     static constexpr int ITEMS = sizeof(K) == 8 ? kSortItems / 2 : kSortItems;
 };
 
-static SortLayout sort_layout(int key_bytes, int value_bytes, int64_t n) {
+// half_bytes: of the words that the tiles of a pass publish (two such halves take turns).
+static SortLayout layout_for(int key_bytes, int value_bytes, int64_t n, int tile, bool partition) {
     SortLayout L;
     L.passes = key_bytes;
-    L.tile = kSortThreads * (key_bytes == 8 ? kSortItems / 2 : kSortItems);
+    L.tile = tile;
     L.tiles = ceil_div(n < 1 ? 1 : n, L.tile);
     L.wide_status = n >= (1ll << 30);
+    const int64_t word = L.wide_status ? 8 : 4;
+    L.half_bytes = partition ? L.tiles * kRadix * word : (L.tiles + 1) / 2 * kRadix * (word + 4);
     L.off_ghist = sizeof(TempHeader);
     L.off_gbase = L.off_ghist + (int64_t)kMaxPasses * kRadix * 8;
     L.off_status = L.off_gbase + (int64_t)kMaxPasses * kRadix * 8;
-    L.control_bytes = L.off_status + round_up(2 * L.tiles * kRadix * (L.wide_status ? 8 : 4), 256);
+    L.control_bytes = L.off_status + round_up(2 * L.half_bytes, 256);
     L.off_keys = L.control_bytes;
     L.off_values = L.off_keys + round_up(n * key_bytes, 256);
     L.total = L.off_values + round_up(n * value_bytes, 256);
     return L;
+}
+static SortLayout sort_layout(int key_bytes, int value_bytes, int64_t n) {
+    return layout_for(key_bytes, value_bytes, n, pass_tile(key_bytes, value_bytes), false);
+}
+static SortLayout partition_layout(int key_bytes, int64_t n) {
+    return layout_for(key_bytes, 0, n, kSortThreads * (key_bytes == 8 ? kSortItems / 2 : kSortItems), true);
 }
 
 // Opts the kernel in to its dynamic shared memory and asks how many of its blocks fit on one
@@ -1047,22 +1031,21 @@ struct SortCall {
 
 template <typename K, typename V, typename SW, typename XF>
 static int run_passes(cudaStream_t s, const SortCall &call, const KeyXform<K> &xf, void *temp, const SortLayout &L) {
-    constexpr int THREADS = SortTuning<K>::THREADS, ITEMS = SortTuning<K>::ITEMS;
-    using Smem = OnesweepSmem<K, V, false, THREADS, ITEMS>;
-    auto kernel = onesweep_kernel<K, V, SW, RadixDigit<K, XF>, THREADS, ITEMS>;
+    using Smem = PassSmem<K, V, typename IndexOf<SW>::type>;
+    auto kernel = digit_pass_kernel<K, V, SW, XF>;
     int blocks_per_sm = 0;
     {
-        const int rc = configure_persistent(kernel, THREADS, Smem::bytes, &blocks_per_sm);
+        const int rc = configure_persistent(kernel, kPassThreads, Smem::bytes, &blocks_per_sm);
         if (rc != B200ALG_OK) return rc;
     }
     const int64_t n = call.n;
     const int64_t resident = (int64_t)sm_count() * blocks_per_sm;
-    const int grid = (int)(L.tiles < resident ? L.tiles : resident);
+    const int grid = (int)(L.tiles + kScanners < resident ? L.tiles + kScanners : resident);
     char *t = (char *)temp;
     TempHeader *hdr = (TempHeader *)temp;
     unsigned long long *ghist = (unsigned long long *)(t + L.off_ghist);
     unsigned long long *gbase = (unsigned long long *)(t + L.off_gbase);
-    SW *status = (SW *)(t + L.off_status);
+    void *published = t + L.off_status;
     SortBuffers<K, V> io;
     io.in = (const K *)call.in_keys;
     io.out = (K *)call.out_keys;
@@ -1074,7 +1057,8 @@ static int run_passes(cudaStream_t s, const SortCall &call, const KeyXform<K> &x
     io.n = n;
     io.n_device = call.n_device;
 
-    B200ALG_CUDA_TRY(cudaMemsetAsync(temp, 0, (size_t)L.control_bytes, s));
+    // the published words of the first pass; every pass clears those of the next
+    B200ALG_CUDA_TRY(cudaMemsetAsync(temp, 0, (size_t)(L.off_status + L.half_bytes), s));
     {
         const int64_t per_block = (int64_t)kHistoThreads * (16 / sizeof(K)) * 2;
         int64_t want = ceil_div(n, per_block);
@@ -1102,17 +1086,11 @@ static int run_passes(cudaStream_t s, const SortCall &call, const KeyXform<K> &x
     sort_offsets_kernel<<<1, kRadix, 0, s>>>(ghist, gbase, hdr, L.passes, (long long)n, io.n_device, 1, call.out_of_place ? 1 : 0);
     B200ALG_LAUNCH_CHECK();
     for (int p = 0; p < L.passes; ++p) {
-        RadixDigit<K, XF> dg;
-        if constexpr (std::is_same<XF, KeyXform<K>>::value) dg.xf = xf;
-        dg.shift = p * 8;
+        XF pass_xf;
+        if constexpr (std::is_same<XF, KeyXform<K>>::value) pass_xf = xf;
         if (g_timed_pass == p) B200ALG_CUDA_TRY(cudaEventRecord(g_timed_pass_events[0], s));
-        if (kSortPdl) {
-            B200ALG_CUDA_TRY(launch_dependent(kernel, dim3(grid), dim3(THREADS), Smem::bytes, s, io, p, dg, hdr,
-                                              (const unsigned long long *)gbase, status, (int)L.tiles, call.value_seq));
-        } else {
-            kernel<<<grid, THREADS, Smem::bytes, s>>>(io, p, dg, hdr, gbase, status, (int)L.tiles, call.value_seq);
-            B200ALG_LAUNCH_CHECK();
-        }
+        B200ALG_CUDA_TRY(launch_dependent(kernel, dim3(grid), dim3(kPassThreads), Smem::bytes, s, io, p, pass_xf, hdr,
+                                          (const unsigned long long *)gbase, published, (int)L.tiles, call.value_seq));
         if (g_timed_pass == p) B200ALG_CUDA_TRY(cudaEventRecord(g_timed_pass_events[1], s));
     }
     {
@@ -1246,8 +1224,8 @@ template <typename K, typename V, typename SW>
 static int run_partition(cudaStream_t s, const K *keys, const V *values, int64_t n, const SplitterBucket<K> &dg,
                          K *out_keys, V *out_values, int64_t *counts, int num_buckets, void *temp, const SortLayout &L) {
     constexpr int THREADS = SortTuning<K>::THREADS, ITEMS = SortTuning<K>::ITEMS;
-    using Smem = OnesweepSmem<K, V, true, THREADS, ITEMS>;
-    auto kernel = onesweep_kernel<K, V, SW, SplitterBucket<K>, THREADS, ITEMS>;
+    using Smem = PartitionSmem<K, V, THREADS, ITEMS>;
+    auto kernel = partition_kernel<K, V, SW, THREADS, ITEMS>;
     int blocks_per_sm = 0;
     {
         const int rc = configure_persistent(kernel, THREADS, Smem::bytes, &blocks_per_sm);
@@ -1275,7 +1253,7 @@ static int run_partition(cudaStream_t s, const K *keys, const V *values, int64_t
     export_bucket_counts_kernel<<<1, kRadix, 0, s>>>(ghist, counts, num_buckets);
     B200ALG_LAUNCH_CHECK();
     SortBuffers<K, V> io{keys, out_keys, nullptr, values, out_values, nullptr, 1, n, nullptr};
-    kernel<<<grid, THREADS, Smem::bytes, s>>>(io, 0, dg, hdr, gbase, status, (int)L.tiles, (int)kSeqNone);
+    kernel<<<grid, THREADS, Smem::bytes, s>>>(io, 0, dg, hdr, gbase, status, (int)L.tiles);
     B200ALG_LAUNCH_CHECK();
     return B200ALG_OK;
 }
@@ -1301,8 +1279,8 @@ template <typename K, typename V, typename SW>
 static int run_bucket_scatter(cudaStream_t s, const K *keys, const V *values, int64_t n, const SplitterBucket<K> &dg,
                               void *temp, const SortLayout &L) {
     constexpr int THREADS = SortTuning<K>::THREADS, ITEMS = SortTuning<K>::ITEMS;
-    using Smem = OnesweepSmem<K, V, true, THREADS, ITEMS>;
-    auto kernel = onesweep_kernel<K, V, SW, SplitterBucket<K>, THREADS, ITEMS>;
+    using Smem = PartitionSmem<K, V, THREADS, ITEMS>;
+    auto kernel = partition_kernel<K, V, SW, THREADS, ITEMS>;
     int blocks_per_sm = 0;
     {
         const int rc = configure_persistent(kernel, THREADS, Smem::bytes, &blocks_per_sm);
@@ -1321,7 +1299,7 @@ static int run_bucket_scatter(cudaStream_t s, const K *keys, const V *values, in
     sort_offsets_kernel<<<1, kRadix, 0, s>>>(ghist, gbase, hdr, 1, (long long)n, nullptr, 0, 1);
     B200ALG_LAUNCH_CHECK();
     SortBuffers<K, V> io{keys, nullptr, nullptr, values, nullptr, nullptr, 1, n, nullptr};
-    kernel<<<grid, THREADS, Smem::bytes, s>>>(io, 0, dg, hdr, gbase, status, (int)L.tiles, (int)kSeqNone);
+    kernel<<<grid, THREADS, Smem::bytes, s>>>(io, 0, dg, hdr, gbase, status, (int)L.tiles);
     B200ALG_LAUNCH_CHECK();
     return B200ALG_OK;
 }
@@ -1361,7 +1339,7 @@ static int bucket_ops(void *stream, bool scatter, const void *keys, const void *
     if (((uintptr_t)keys % kb) || ((uintptr_t)temp % 256)) return B200ALG_MISALIGNED;
     uint64_t xn, xp;
     if (!key_xform_constants(key_dtype, order, xn, xp)) return B200ALG_UNSUPPORTED;
-    const SortLayout L = sort_layout(kb, 0, n);
+    const SortLayout L = partition_layout(kb, n);
     if (temp_bytes < L.control_bytes) return B200ALG_TEMP_TOO_SMALL;
     cudaStream_t s = (cudaStream_t)stream;
     if (n == 0) {
@@ -1506,7 +1484,7 @@ extern "C" int b200alg_bucket_partition_temp_bytes(int key_dtype, int64_t n, int
     const int kb = dtype_bytes(key_dtype);
     if (kb == 0) return B200ALG_UNSUPPORTED;
     if (n > kMaxElements) return B200ALG_TOO_LARGE;
-    *out_bytes = sort_layout(kb, 0, n).control_bytes;
+    *out_bytes = partition_layout(kb, n).control_bytes;
     return B200ALG_OK;
 }
 
@@ -1527,7 +1505,7 @@ extern "C" int b200alg_bucket_partition(void *stream, const void *keys, const vo
         return B200ALG_MISALIGNED;
     uint64_t xn, xp;
     if (!key_xform_constants(key_dtype, order, xn, xp)) return B200ALG_UNSUPPORTED;
-    const SortLayout L = sort_layout(kb, 0, n);
+    const SortLayout L = partition_layout(kb, n);
     if (temp_bytes < L.control_bytes) return B200ALG_TEMP_TOO_SMALL;
     cudaStream_t s = (cudaStream_t)stream;
     if (n == 0) {

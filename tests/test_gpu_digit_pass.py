@@ -1,0 +1,49 @@
+"""The digit pass of the radix sort around its tiles: one key, the last key of a tile, of two tiles
+(whose places are published together) and one more, for key and value sizes with different tiles;
+keys that meet in few digits; against a stable host sort."""
+import numpy as np
+import pytest
+import torch
+
+from ilgpu_b200 import RadixSortOperations
+from tests.helpers import NP
+
+pytestmark = pytest.mark.gpu
+
+# keys per tile: 512 threads, as many keys each as two blocks per SM leave room for
+TILES = {("UInt8", None): 10240, ("UInt32", None): 10240, ("UInt64", None): 5632, ("UInt32", np.int32): 6144,
+         ("UInt64", np.uint32): 4096, ("Int64", np.float64): 3072, ("UInt16", np.uint8): 8192}
+NAMES = {v: k for k, v in NP.items()}
+
+
+def _sorts(acc, name, keys, values):
+    op = getattr(RadixSortOperations, "Ascending" + name)
+    dev = torch.from_numpy(keys).cuda()
+    if values is None:
+        temp = acc.Allocate1D(acc.ComputeRadixSortTempStorageSize(op, keys.size), torch.int32)
+        acc.CreateRadixSort(op)(None, dev, temp)
+        acc.CheckDeviceStatus(None, temp)
+        return dev.cpu().numpy(), None
+    vals = torch.from_numpy(values).cuda()
+    temp = acc.Allocate1D(acc.ComputeRadixSortPairsTempStorageSize(op, vals.dtype, keys.size), torch.int32)
+    acc.CreateRadixSortPairs(op)(None, dev, vals, temp)
+    acc.CheckDeviceStatus(None, temp)
+    return dev.cpu().numpy(), vals.cpu().numpy()
+
+
+@pytest.mark.parametrize("name,value", list(TILES))
+@pytest.mark.parametrize("tiles,extra", [(0, 1), (1, -1), (1, 0), (1, 1), (2, 0), (2, 1), (3, 0), (131, 7)])
+def test_tile_edges(accelerator, name, value, tiles, extra):
+    n = tiles * TILES[name, value] + extra
+    rng = np.random.default_rng(n)
+    info = np.iinfo(NP[name])
+    for few in (False, True):
+        keys = rng.integers(info.min, info.max, size=n, dtype=NP[name], endpoint=True)
+        if few:   # whole warps, and in later passes whole tiles, of one digit
+            keys = rng.choice(keys[:3] if n > 3 else keys, size=n).astype(NP[name])
+        values = None if value is None else np.arange(n).astype(value)
+        got, got_values = _sorts(accelerator, name, keys, values)
+        order = np.argsort(keys, kind="stable")
+        np.testing.assert_array_equal(got, keys[order])
+        if values is not None:
+            np.testing.assert_array_equal(got_values, values[order])
