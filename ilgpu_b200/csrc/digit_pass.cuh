@@ -226,18 +226,6 @@ __device__ __forceinline__ void take_tile(PassMisc<K, V, SW> &m, unsigned char *
     }
 }
 
-// Whether of two neighbouring slots the first has to come after the second (and must not: see the top
-// of this file).
-template <typename K, bool VALUES, typename XF>
-__device__ __forceinline__ bool out_of_order(K first, K second, unsigned int first_place, unsigned int second_place, XF xf, int shift) {
-    if constexpr (!VALUES) {
-        const K sorted = (K)((K)~(K)0 >> (8 * (int)sizeof(K) - 8 - shift));  // this digit and the ones below it
-        return (K)(xf(first) & sorted) > (K)(xf(second) & sorted);
-    } else {
-        return (((xf(first) ^ xf(second)) >> shift) & 0xFFu) == 0 && first_place > second_place;
-    }
-}
-
 // Puts the slots of a tile in order: neighbours that are the wrong way round change places until none
 // are.  Reached only when the atomics of a warp were not served in lane order.
 template <typename K, typename V, typename XF, typename L>
@@ -266,13 +254,6 @@ __device__ __noinline__ void repair_order(unsigned char *smem, XF xf, int shift)
         again = block_any(again);
     }
 }
-
-// The raw key whose transform is all ones: it fills a ragged tile up and sorts behind every real key.
-template <typename K> __device__ __forceinline__ K padding_key(const KeyXform<K> &xf) {
-    const K r = (K)((K)~(K)0 ^ xf.xor_pos);
-    return (r >> (sizeof(K) * 8 - 1)) ? (K)((K)~(K)0 ^ xf.xor_neg) : r;
-}
-template <typename K> __device__ __forceinline__ K padding_key(const KeyIdentity<K> &) { return (K)~(K)0; }
 
 // Writes the tile in the slots to global memory; true when a slot is out of order.
 template <typename K, typename V, typename SW, typename XF, typename L, bool FAST>

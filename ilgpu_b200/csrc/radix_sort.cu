@@ -15,13 +15,11 @@
 // structure-of-arrays here).  Every pass is a stable partition, so the result equals the
 // reference's: a stable sort by the transformed key.
 #include "common.cuh"
+#include "sort_common.cuh"
 
 #include <type_traits>
 
 namespace b200alg {
-
-constexpr int kRadix = 256;
-constexpr int kMaxPasses = 8;
 
 // Control words that live in TempHeader::reserved.
 enum : int {
@@ -37,58 +35,7 @@ enum : int {
 // The three buffers a sort moves its data between.
 enum : unsigned int { kBufIn = 0, kBufOut = 1, kBufAlt = 2 };
 
-// Views of one sort call.  An in-place sort has in == out (possibly strided); an out-of-place
-// sort leaves `in` untouched.  The alternate buffer is dense scratch of n elements.
-template <typename K, typename V> struct SortBuffers {
-    const K *in;
-    K *out, *alt;
-    const V *vin;
-    V *vout, *valt;
-    int64_t stride;             // of the input / output view
-    int64_t n;                  // element count, or its upper bound when n_device is set
-    const long long *n_device;  // element count in device memory (NULL: n is exact)
-};
-template <typename K, typename V> __device__ __forceinline__ int64_t effective_n(const SortBuffers<K, V> &io) {
-    if (!io.n_device) return io.n;
-    const long long v = *io.n_device;
-    return v < 0 ? 0 : (v > io.n ? io.n : (int64_t)v);
-}
 constexpr unsigned int kNoPass = 0xFFu;
-
-// Values that are a function of the element's index (the reference's sequencers:
-// IndexSequencer and the integer / Half / Float / Double sequencers, Sequencer.cs:37-72,
-// Sequencers.tt:26-38): the pairs sort can produce them in its first pass instead of reading
-// a value view.
-enum : int { kSeqNone = 0, kSeqInteger = 1, kSeqFloating = 2 };
-template <typename V> __device__ __forceinline__ V sequence_value(int kind, int64_t i) {
-    if constexpr (sizeof(V) == 2) {
-        if (kind == kSeqFloating) return (V)__half_as_ushort(__float2half_rn((float)i));
-        return (V)i;
-    } else if constexpr (sizeof(V) == 4) {
-        if (kind == kSeqFloating) return (V)__float_as_uint((float)i);
-        return (V)i;
-    } else if constexpr (sizeof(V) == 8) {
-        if (kind == kSeqFloating) return (V)__double_as_longlong((double)i);
-        return (V)i;
-    } else if constexpr (sizeof(V) == 1) {
-        return (V)i;
-    } else {
-        return V{};
-    }
-}
-
-// Key transform: bits = raw ^ (sign(raw) ? xor_neg : xor_pos) covers every key type of
-// RadixSortOperations.tt:77-93 and the descending complement of :122-123.
-template <typename K> struct KeyXform {
-    K xor_neg, xor_pos;
-    __device__ __forceinline__ K operator()(K raw) const {
-        return raw ^ ((raw >> (sizeof(K) * 8 - 1)) ? xor_neg : xor_pos);
-    }
-};
-// Ascending unsigned keys need no transform at all.
-template <typename K> struct KeyIdentity {
-    __device__ __forceinline__ K operator()(K raw) const { return raw; }
-};
 
 static bool key_xform_constants(int dtype, int order, uint64_t &xn, uint64_t &xp) {
     const int bits = dtype_bytes(dtype) * 8;
@@ -364,10 +311,6 @@ template <typename K> struct SplitterBucket {
         return b;
     }
 };
-
-struct NoValue {};
-template <typename V> struct ValueBytes { static constexpr int value = sizeof(V); };
-template <> struct ValueBytes<NoValue> { static constexpr int value = 0; };
 
 // Index of an element of the whole view: 32 bits while the look-back words are, else 64.
 template <typename SW> struct IndexOf { using type = unsigned int; };
@@ -1016,19 +959,6 @@ static int configure_persistent(KernelT kernel, int threads, size_t bytes, int *
 thread_local cudaEvent_t g_timed_pass_events[2] = {nullptr, nullptr};
 thread_local int g_timed_pass = -1;
 
-// What a sort call works on, untyped (the entry points fill this in).
-struct SortCall {
-    const void *in_keys;
-    void *out_keys;
-    const void *in_values;
-    void *out_values;
-    int64_t stride;
-    int64_t n;                  // element count, or its upper bound when n_device is set
-    const long long *n_device;
-    int value_seq;
-    bool out_of_place;
-};
-
 template <typename K, typename V, typename SW, typename XF>
 static int run_passes(cudaStream_t s, const SortCall &call, const KeyXform<K> &xf, void *temp, const SortLayout &L) {
     using Smem = PassSmem<K, V, typename IndexOf<SW>::type>;
@@ -1404,6 +1334,11 @@ static int sort_common(void *stream, const SortCall &call, int key_dtype, int va
     if (temp_bytes < L.total) return B200ALG_TEMP_TOO_SMALL;
     if (call.n == 0) return B200ALG_OK;
     cudaStream_t s = (cudaStream_t)stream;
+    if (g_timed_pass < 0) {
+        bool taken = false;
+        const int rc = resident_sort(s, call, kb, value_bytes, xn, xp, temp, temp_bytes, &taken);
+        if (rc != B200ALG_OK || taken) return rc;
+    }
     switch (value_bytes) {
     case 0: return dispatch_key<NoValue>(s, kb, call, xn, xp, temp, L);
     case 1: return dispatch_key<uint8_t>(s, kb, call, xn, xp, temp, L);

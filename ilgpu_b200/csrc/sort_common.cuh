@@ -1,0 +1,105 @@
+// What the kernels of the radix sort share: key transforms, sequenced values, and the check that ranks
+// taken with atomics came out in order.
+#pragma once
+
+#include "common.cuh"
+
+namespace b200alg {
+
+constexpr int kRadix = 256;
+constexpr int kMaxPasses = 8;
+
+// Views of one sort call.  An in-place sort has in == out (possibly strided); an out-of-place
+// sort leaves `in` untouched.  The alternate buffer is dense scratch of n elements.
+template <typename K, typename V> struct SortBuffers {
+    const K *in;
+    K *out, *alt;
+    const V *vin;
+    V *vout, *valt;
+    int64_t stride;             // of the input / output view
+    int64_t n;                  // element count, or its upper bound when n_device is set
+    const long long *n_device;  // element count in device memory (NULL: n is exact)
+};
+template <typename K, typename V> __device__ __forceinline__ int64_t effective_n(const SortBuffers<K, V> &io) {
+    if (!io.n_device) return io.n;
+    const long long v = *io.n_device;
+    return v < 0 ? 0 : (v > io.n ? io.n : (int64_t)v);
+}
+
+// Values that are a function of the element's index (the reference's sequencers:
+// IndexSequencer and the integer / Half / Float / Double sequencers, Sequencer.cs:37-72,
+// Sequencers.tt:26-38): the pairs sort can produce them in its first pass instead of reading
+// a value view.
+enum : int { kSeqNone = 0, kSeqInteger = 1, kSeqFloating = 2 };
+template <typename V> __device__ __forceinline__ V sequence_value(int kind, int64_t i) {
+    if constexpr (sizeof(V) == 2) {
+        if (kind == kSeqFloating) return (V)__half_as_ushort(__float2half_rn((float)i));
+        return (V)i;
+    } else if constexpr (sizeof(V) == 4) {
+        if (kind == kSeqFloating) return (V)__float_as_uint((float)i);
+        return (V)i;
+    } else if constexpr (sizeof(V) == 8) {
+        if (kind == kSeqFloating) return (V)__double_as_longlong((double)i);
+        return (V)i;
+    } else if constexpr (sizeof(V) == 1) {
+        return (V)i;
+    } else {
+        return V{};
+    }
+}
+
+// Key transform: bits = raw ^ (sign(raw) ? xor_neg : xor_pos) covers every key type of
+// RadixSortOperations.tt:77-93 and the descending complement of :122-123.
+template <typename K> struct KeyXform {
+    K xor_neg, xor_pos;
+    __device__ __forceinline__ K operator()(K raw) const {
+        return raw ^ ((raw >> (sizeof(K) * 8 - 1)) ? xor_neg : xor_pos);
+    }
+};
+// Ascending unsigned keys need no transform at all.
+template <typename K> struct KeyIdentity {
+    __device__ __forceinline__ K operator()(K raw) const { return raw; }
+};
+
+struct NoValue {};
+template <typename V> struct ValueBytes { static constexpr int value = sizeof(V); };
+template <> struct ValueBytes<NoValue> { static constexpr int value = 0; };
+
+// Whether of two neighbouring slots the first has to come after the second (and must not: see the top
+// of digit_pass.cuh).
+template <typename K, bool VALUES, typename XF>
+__device__ __forceinline__ bool out_of_order(K first, K second, unsigned int first_place, unsigned int second_place, XF xf, int shift) {
+    if constexpr (!VALUES) {
+        const K sorted = (K)((K)~(K)0 >> (8 * (int)sizeof(K) - 8 - shift));  // this digit and the ones below it
+        return (K)(xf(first) & sorted) > (K)(xf(second) & sorted);
+    } else {
+        return (((xf(first) ^ xf(second)) >> shift) & 0xFFu) == 0 && first_place > second_place;
+    }
+}
+
+// The raw key whose transform is all ones: it fills a ragged tile up and sorts behind every real key.
+template <typename K> __device__ __forceinline__ K padding_key(const KeyXform<K> &xf) {
+    const K r = (K)((K)~(K)0 ^ xf.xor_pos);
+    return (r >> (sizeof(K) * 8 - 1)) ? (K)((K)~(K)0 ^ xf.xor_neg) : r;
+}
+template <typename K> __device__ __forceinline__ K padding_key(const KeyIdentity<K> &) { return (K)~(K)0; }
+
+// What a sort call works on, untyped (the entry points fill this in).
+struct SortCall {
+    const void *in_keys;
+    void *out_keys;
+    const void *in_values;
+    void *out_values;
+    int64_t stride;
+    int64_t n;                  // element count, or its upper bound when n_device is set
+    const long long *n_device;
+    int value_seq;
+    bool out_of_place;
+};
+
+// The sort of a view that fits on the GPU's SMs as a whole, in one launch (small_sort.cu).  *taken: false
+// when the view is too long for that.
+int resident_sort(cudaStream_t s, const SortCall &call, int key_bytes, int value_bytes, uint64_t xor_neg, uint64_t xor_pos, void *temp,
+                  int64_t temp_bytes, bool *taken);
+
+}  // namespace b200alg
