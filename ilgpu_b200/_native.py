@@ -44,6 +44,7 @@ SIGNATURES = {
     "b200alg_scan_carry": (_int, [_vp, _vp, _i64, _vp, _i64, _i64, _int, _int, _int, _vp, _vp, _i64]),
     "b200alg_scan_static": (_int, [_vp, _vp, _i64, _vp, _i64, _i64, _int, _int, _int]),
     "b200alg_reduce": (_int, [_vp, _vp, _i64, _i64, _int, _int, _vp]),
+    "b200alg_reduce_to_host": (_int, [_vp, _vp, _i64, _i64, _int, _int, _vp, _vp]),
     "b200alg_histogram": (_int, [_vp, _vp, _i64, _i64, _int, _int, _dbl, _dbl, _vp, _i64, _int, _vp]),
     "b200alg_initialize": (_int, [_vp, _vp, _i64, _i64, _int, _vp]),
     "b200alg_sequence": (_int, [_vp, _vp, _i64, _int, _i64, _i64]),
@@ -80,7 +81,7 @@ _host = None
 # what csrc/host_calls.cpp calls, in the order of its table
 _HOST_ENTRY_POINTS = (
     "b200alg_radix_sort_temp_bytes", "b200alg_radix_sort_keys", "b200alg_radix_sort_pairs", "b200alg_radix_sort_pairs_sequence",
-    "b200alg_scan_temp_bytes", "b200alg_scan_carry", "b200alg_reduce", "b200alg_histogram", "b200alg_initialize",
+    "b200alg_scan_temp_bytes", "b200alg_scan_carry", "b200alg_reduce", "b200alg_reduce_to_host", "b200alg_histogram", "b200alg_initialize",
     "b200alg_unique_temp_bytes", "b200alg_unique",
 )
 

@@ -31,6 +31,7 @@ struct Library {
     decltype(&b200alg_scan_temp_bytes) scan_temp_bytes;
     decltype(&b200alg_scan_carry) scan_carry;
     decltype(&b200alg_reduce) reduce;
+    decltype(&b200alg_reduce_to_host) reduce_to_host;
     decltype(&b200alg_histogram) histogram;
     decltype(&b200alg_initialize) initialize;
     decltype(&b200alg_unique_temp_bytes) unique_temp_bytes;
@@ -246,9 +247,8 @@ PyObject *reduce_value(PyObject *, PyObject *const *a, Py_ssize_t count) {
         const at::Tensor out = at::empty({8}, at::TensorOptions().dtype(at::kByte).device(at::kCUDA, device));
         void *result = out.data_ptr();
         const int status = released([&]() -> int {
-            const int rc = lib.reduce(stream, in.data, in.stride, in.n, code, op, result);
+            const int rc = lib.reduce_to_host(stream, in.data, in.stride, in.n, code, op, result, slot);
             if (rc != B200ALG_OK) return rc;
-            if (cudaMemcpyAsync(slot, result, in.bytes, cudaMemcpyDeviceToHost, (cudaStream_t)stream) != cudaSuccess) return B200ALG_CUDA_ERROR;
             return cudaStreamSynchronize((cudaStream_t)stream) == cudaSuccess ? B200ALG_OK : B200ALG_CUDA_ERROR;
         });
         if (status != B200ALG_OK) return false;

@@ -2,7 +2,11 @@
 // Replaces ReductionImplementation + CreateReduction (ReductionExtensions.cs:52-167).
 #include "common.cuh"
 
+#include <cooperative_groups.h>
+
 namespace b200alg {
+
+namespace cg = cooperative_groups;
 
 // AtomicApply of IScanReduceOperation<T> (ScanReduceOperations.tt:66-70).
 template <typename T, int OP> struct AtomicApply;
@@ -57,29 +61,36 @@ template <typename T> __global__ void set_scalar_kernel(T *out, T v) {
     *out = v;
 }
 
+// The fold of the whole block, in its first thread.
 template <typename T, int OP, int THREADS>
-__device__ __forceinline__ void block_fold_and_publish(T acc, T *out) {
+__device__ __forceinline__ T block_fold(T acc) {
     using O = Op<T, OP>;
     __shared__ T warp_part[THREADS / 32];
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) acc = O::apply(acc, shfl_down(acc, d));
     if (lane_id() == 0) warp_part[threadIdx.x >> 5] = acc;
     __syncthreads();
+    T v = O::identity();
     if (threadIdx.x < 32) {
-        T v = threadIdx.x < THREADS / 32 ? warp_part[threadIdx.x] : O::identity();
+        v = threadIdx.x < THREADS / 32 ? warp_part[threadIdx.x] : O::identity();
 #pragma unroll
         for (int d = 16; d > 0; d >>= 1) v = O::apply(v, shfl_down(v, d));
-        if (threadIdx.x == 0) {
-            grid_dependency_wait();  // out[0] holds Identity from here on
-            AtomicApply<T, OP>::run(out, v);
-        }
+    }
+    return v;
+}
+template <typename T, int OP, int THREADS>
+__device__ __forceinline__ void block_fold_and_publish(T acc, T *out) {
+    const T v = block_fold<T, OP, THREADS>(acc);
+    if (threadIdx.x == 0) {
+        grid_dependency_wait();  // out[0] holds Identity from here on
+        AtomicApply<T, OP>::run(out, v);
     }
 }
 
-// Dense input.  The 16-byte aligned body is read as uint4 vectors with four loads in
-// flight per thread; block 0 also folds the unaligned head and the tail.
+// What this thread folds of a dense input.  The 16-byte aligned body is read as uint4 vectors with
+// four loads in flight per thread; block 0 also folds the unaligned head and the tail.
 template <typename T, int OP, int THREADS>
-__global__ void __launch_bounds__(THREADS) reduce_dense_kernel(const T *__restrict__ in, int64_t n, T *out) {
+__device__ __forceinline__ T fold_dense(const T *__restrict__ in, int64_t n) {
     using O = Op<T, OP>;
     constexpr int VEC = 16 / sizeof(T);
     union V { uint4 u; T t[VEC]; };
@@ -119,8 +130,41 @@ __global__ void __launch_bounds__(THREADS) reduce_dense_kernel(const T *__restri
         for (int64_t j = threadIdx.x; j < head; j += THREADS) r = O::apply(r, in[j]);
         for (int64_t j = tail + threadIdx.x; j < n; j += THREADS) r = O::apply(r, in[j]);
     }
-    block_fold_and_publish<T, OP, THREADS>(r, out);
+    return r;
 }
+template <typename T, int OP, int THREADS>
+__global__ void __launch_bounds__(THREADS) reduce_dense_kernel(const T *__restrict__ in, int64_t n, T *out) {
+    block_fold_and_publish<T, OP, THREADS>(fold_dense<T, OP, THREADS>(in, n), out);
+}
+
+// Short input: one block or one cluster, whose blocks meet in distributed shared memory.  No
+// Identity to be stored first and no atomics: one launch instead of two, and the result is a plain
+// store, so that it can go to host memory.
+constexpr int kClusterThreads = 1024, kReduceCluster = 8;
+template <typename T, int OP>
+__global__ void __launch_bounds__(kClusterThreads) reduce_cluster_kernel(const T *__restrict__ in, int64_t stride, int64_t n, T *out) {
+    using O = Op<T, OP>;
+    __shared__ T total;
+    T r = O::identity();
+    if (stride == 1) {
+        r = fold_dense<T, OP, kClusterThreads>(in, n);
+    } else {
+        for (int64_t i = (int64_t)blockIdx.x * kClusterThreads + threadIdx.x; i < n; i += (int64_t)gridDim.x * kClusterThreads)
+            r = O::apply(r, in[i * stride]);
+    }
+    r = block_fold<T, OP, kClusterThreads>(r);
+    if (gridDim.x > 1) {
+        cg::cluster_group cluster = cg::this_cluster();
+        if (threadIdx.x == 0) total = r;
+        cluster.sync();
+        if (blockIdx.x == 0 && threadIdx.x == 0)
+            for (int b = 1; b < (int)gridDim.x; ++b) r = O::apply(r, *cluster.map_shared_rank(&total, b));
+        cluster.sync();  // nobody leaves while its total is being read
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) *out = r;
+}
+// One block per 64 KB until a whole cluster works; from 1 MB on more SMs are worth two launches.
+static bool fits_cluster(int64_t n, int64_t stride, int elem_bytes) { return n * elem_bytes <= (stride == 1 ? 1 << 20 : 1 << 17); }
 
 // Stride1D.General input: element i lives at in[i * stride].
 template <typename T, int OP, int THREADS>
@@ -136,6 +180,22 @@ template <typename T, int OP>
 static int launch_reduce(cudaStream_t s, const void *in, int64_t stride, int64_t n, void *out) {
     constexpr int THREADS = 256;
     constexpr int VEC = 16 / sizeof(T);
+    if (fits_cluster(n, stride, sizeof(T))) {
+        int blocks = 1;
+        while (blocks < kReduceCluster && n * (int64_t)sizeof(T) > (int64_t)blocks * (64 << 10)) blocks *= 2;
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = blocks;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.gridDim = dim3(blocks);
+        cfg.blockDim = dim3(kClusterThreads);
+        cfg.stream = s;
+        cfg.attrs = attr;
+        cfg.numAttrs = blocks > 1 ? 1 : 0;
+        B200ALG_CUDA_TRY(cudaLaunchKernelEx(&cfg, reduce_cluster_kernel<T, OP>, (const T *)in, stride, n, (T *)out));
+        return B200ALG_OK;
+    }
     set_scalar_kernel<T><<<1, 1, 0, s>>>((T *)out, Op<T, OP>::identity());
     B200ALG_LAUNCH_CHECK();
     const int max_blocks = sm_count() * 8;
@@ -183,4 +243,14 @@ extern "C" int b200alg_reduce(void *stream, const void *in, int64_t stride, int6
     case B200ALG_F64: return dispatch_op<double>(s, in, stride, n, op, out);
     }
     return B200ALG_UNSUPPORTED;
+}
+
+extern "C" int b200alg_reduce_to_host(void *stream, const void *in, int64_t stride, int64_t n, int dtype, int op, void *scratch, void *host_out) {
+    if (!scratch || !host_out) return B200ALG_INVALID_ARGUMENT;
+    const int es = dtype_bytes(dtype);
+    if (n >= 1 && n <= (1 << 20) && stride >= 1 && fits_cluster(n, stride, es)) return b200alg_reduce(stream, in, stride, n, dtype, op, host_out);
+    const int rc = b200alg_reduce(stream, in, stride, n, dtype, op, scratch);
+    if (rc != B200ALG_OK) return rc;
+    B200ALG_CUDA_TRY(cudaMemcpyAsync(host_out, scratch, es, cudaMemcpyDeviceToHost, (cudaStream_t)stream));
+    return B200ALG_OK;
 }

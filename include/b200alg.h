@@ -188,6 +188,11 @@ int b200alg_scan_static(void *stream, const void *in, int64_t in_stride, void *o
  * Replaces the lambda of CreateReduction (ReductionExtensions.cs:135-167): out[0] is set
  * to Identity and then folded with every input element.  n >= 1. */
 int b200alg_reduce(void *stream, const void *in, int64_t stride, int64_t n, int dtype, int op, void *out);
+/* The same with the result in host memory (ReductionExtensions.cs:198-216 copies it there):
+ * host_out is pinned, mapped memory of the caller and holds the result once the stream has got
+ * there.  scratch: 8 bytes of device memory, 8-byte aligned. */
+int b200alg_reduce_to_host(void *stream, const void *in, int64_t stride, int64_t n, int dtype, int op, void *scratch,
+                           void *host_out);
 
 /* ---- histogram --------------------------------------------------------------------
  * Replaces the lambdas of CreateHistogram / CreateHistogramUnchecked
