@@ -46,7 +46,9 @@ template <typename T> __device__ __forceinline__ T shfl_value_last(T v) {
 // Bound: HBM (every element read once, every survivor written once).  A tile is 32 KB: 16-byte
 // loads, four in flight per thread, in warp-striped order (vector j of lane l holds elements
 // (warp * 4 * 32 + j * 32 + l) * VEC ... of the tile), so a warp reads whole lines; survivors meet
-// in shared memory and leave in consecutive stores.
+// in shared memory and leave in consecutive stores.  (Scalar loads of 16 consecutive elements per thread, with
+// the survivors written to scratch and copied back by a second kernel, took 153 + 26 us for 5 * 10^7
+// uint32 of which a quarter is kept; this UNIQUE_NOW.)
 //
 // `kept` may be `in` itself (the in-place unique): a tile stores only once it knows its prefix,
 // hence after every earlier tile has published its count and so has read its elements, and it
@@ -65,8 +67,7 @@ unique_select_kernel(const T *in, int64_t n, T *kept, long long *__restrict__ st
 
     __shared__ __align__(16) unsigned char survivors_raw[TILE * sizeof(T)];
     __shared__ unsigned int warp_total[WARPS];
-    __shared__ unsigned int warp_excl[WARPS];
-    __shared__ unsigned int s_prefix, s_count;
+    __shared__ unsigned int s_prefix;
     __shared__ int s_tile;
     T *survivors = reinterpret_cast<T *>(survivors_raw);
 
@@ -139,23 +140,23 @@ unique_select_kernel(const T *in, int64_t n, T *kept, long long *__restrict__ st
     }
     if (lane == 31) warp_total[warp] = chunk;
     __syncthreads();
-    if (warp == 0) {
-        unsigned int wt = lane < WARPS ? warp_total[lane] : 0u;
-        unsigned int wi = wt;
+    const unsigned int wt = lane < WARPS ? warp_total[lane] : 0u;
+    const unsigned int first_slot = __reduce_add_sync(0xffffffffu, lane < warp ? wt : 0u);
+    const unsigned int aggregate = __reduce_add_sync(0xffffffffu, wt);
+    // Survivors gather while the first warp, once it has told the tiles behind this one its count,
+    // looks for its prefix.
+    TileState<unsigned int> state(state_base, num_tiles);
+    if (tid == 0) state.publish(tile, tile == 0 ? kInclusive : kAggregate, aggregate);
 #pragma unroll
-        for (int d = 1; d < WARPS; d <<= 1) {
-            const unsigned int up = __shfl_up_sync(0xffffffffu, wi, d);
-            if (lane >= d) wi += up;
-        }
-        if (lane < WARPS) warp_excl[lane] = wi - wt;
-        const unsigned int aggregate = __shfl_sync(0xffffffffu, wi, WARPS - 1);
-
-        TileState<unsigned int> state(state_base, num_tiles);
+    for (int j = 0; j < NV; ++j) {
+        unsigned int slot = first_slot + local[j];
+#pragma unroll
+        for (int e = 0; e < VEC; ++e)
+            if ((keep[j] >> e) & 1u) survivors[slot++] = v[j].t[e];
+    }
+    if (warp == 0) {
         unsigned int prefix = 0u;
-        if (tile == 0) {
-            if (lane == 0) state.publish(0, kInclusive, aggregate);
-        } else {
-            if (lane == 0) state.publish(tile, kAggregate, aggregate);
+        if (tile > 0) {
             int look = tile - 1 - lane;  // 32 predecessors per round, nearest first
             bool gave_up = false;
             while (true) {
@@ -184,30 +185,22 @@ unique_select_kernel(const T *in, int64_t n, T *kept, long long *__restrict__ st
         }
         if (lane == 0) {
             s_prefix = prefix;
-            s_count = aggregate;
             if (tile == num_tiles - 1) *out_count = (long long)prefix + aggregate;
         }
     }
     __syncthreads();
 
-    const unsigned int first_slot = warp_excl[warp];
+    if (starts) {  // where the runs begin (run-length encoding)
 #pragma unroll
-    for (int j = 0; j < NV; ++j) {
-        unsigned int slot = first_slot + local[j];
+        for (int j = 0; j < NV; ++j) {
+            unsigned int slot = first_slot + local[j];
 #pragma unroll
-        for (int e = 0; e < VEC; ++e) {
-            if ((keep[j] >> e) & 1u) {
-                survivors[slot] = v[j].t[e];
-                // where the run begins (run-length encoding)
-                if (starts) starts[(int64_t)s_prefix + slot] = base + warp_first + (j * 32 + lane) * VEC + e;
-                ++slot;
-            }
+            for (int e = 0; e < VEC; ++e)
+                if ((keep[j] >> e) & 1u) starts[(int64_t)s_prefix + slot++] = base + warp_first + (j * 32 + lane) * VEC + e;
         }
     }
-    __syncthreads();
-    const unsigned int count = s_count;
     T *to = kept + s_prefix;
-    for (unsigned int i = tid; i < count; i += kUniqueThreads) to[i] = survivors[i];
+    for (unsigned int i = tid; i < aggregate; i += kUniqueThreads) to[i] = survivors[i];
 }
 
 // lengths[r] = distance from the start of run r to the start of the next run (or to n).
