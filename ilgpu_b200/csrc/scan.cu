@@ -186,9 +186,9 @@ __global__ void __launch_bounds__(256) scan_clear_kernel(uint4 *words, int64_t c
 constexpr int kScanStages = 2;
 constexpr int kScanTileBytes = kScanThreads * kScanVecPerThread * 16;
 
-template <typename T, int OP, bool INCLUSIVE>
+template <typename T, int OP, bool INCLUSIVE, bool LEAD>
 __global__ void __launch_bounds__(kScanThreads)
-scan_pipeline_kernel(const T *in, T *out, int64_t n, int lead, const T *carry_in, TempHeader *hdr, void *state_base, int num_tiles) {
+scan_pipeline_kernel(const T *in, T *out, int64_t n, int lead_arg, const T *carry_in, TempHeader *hdr, void *state_base, int num_tiles) {
     using O = Op<T, OP>;
     constexpr int VEC = 16 / sizeof(T);
     constexpr int NV = kScanVecPerThread;
@@ -203,8 +203,10 @@ scan_pipeline_kernel(const T *in, T *out, int64_t n, int lead, const T *carry_in
     __shared__ int s_failed;               // a wait for a bulk copy ran out: later tiles are loaded directly
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    // (LEAD is a template parameter because the extra register costs aligned views 5 %)
+    const int lead = LEAD ? lead_arg : 0;
     const int full_tiles = (int)(n / TILE);          // tiles below this index are complete,
-    const int first_full = lead == 0 ? 0 : 1;        // from this one on
+    constexpr int first_full = LEAD ? 1 : 0;         // from this one on
 
     // The last thread issues the copies: warp 0 does the look-back.
     constexpr int kStager = kScanThreads - 1;
@@ -223,7 +225,12 @@ scan_pipeline_kernel(const T *in, T *out, int64_t n, int lead, const T *carry_in
             }
         }
     }
-    __syncthreads();
+    // The descriptors of this block's tiles; every block has to have cleared its own before anybody
+    // publishes (while the first tiles are on their way).
+    if (blockIdx.x == 0 && tid == 0) hdr->wait_limit_hit = 0u;
+    for (int64_t t = (int64_t)blockIdx.x + (int64_t)tid * G; t < num_tiles; t += (int64_t)kScanThreads * G)
+        *reinterpret_cast<uint4 *>((unsigned char *)state_base + (size_t)t * kDescStride) = make_uint4(0u, 0u, 0u, 0u);
+    cg::this_grid().sync();
     unsigned int bar_phase = 0;  // bit st = parity of the next completion of stage st's barrier
     bool staging = true;         // false once a wait for a copy ran out: later tiles are loaded directly
     TileState<T> state(state_base, num_tiles);
@@ -531,19 +538,12 @@ static int launch_scan(cudaStream_t s, const void *in, int64_t in_stride, void *
         return B200ALG_OK;
     }
     const int tiles = (int)ceil_div(n_arg, TILE);
-    const size_t state_bytes = (size_t)tiles * kDescStride;
-    {
-        const int64_t words = (int64_t)((sizeof(TempHeader) + state_bytes) / 16);
-        const int64_t want = ceil_div(words, 256 * 4);
-        const int64_t cap = (int64_t)sm_count() * 4;
-        scan_clear_kernel<<<(int)(want < 1 ? 1 : (want > cap ? cap : want)), 256, 0, s>>>((uint4 *)temp, words);
-        B200ALG_LAUNCH_CHECK();
-    }
     bool launched = false;
     if (alike) {
-        auto kernel = scan_pipeline_kernel<T, OP, INCLUSIVE>;
+        auto kernel = lead ? scan_pipeline_kernel<T, OP, INCLUSIVE, true> : scan_pipeline_kernel<T, OP, INCLUSIVE, false>;
         constexpr size_t ring_bytes = (size_t)kScanStages * kScanTileBytes;
-        static ContextCache<int> cache;  // per kernel instantiation and CUDA context
+        static ContextCache<int> caches[2];  // per kernel instantiation and CUDA context
+        ContextCache<int> &cache = caches[lead != 0];
         int blocks_per_sm = 0;
         if (!cache.find(&blocks_per_sm)) {
             B200ALG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ring_bytes));
@@ -565,6 +565,13 @@ static int launch_scan(cudaStream_t s, const void *in, int64_t in_stride, void *
     }
     if (!launched) {
         const int general_tiles = (int)ceil_div(n, TILE);
+        {
+            const int64_t words = (int64_t)((sizeof(TempHeader) + (size_t)general_tiles * kDescStride) / 16);
+            const int64_t want = ceil_div(words, 256 * 4);
+            const int64_t cap = (int64_t)sm_count() * 4;
+            scan_clear_kernel<<<(int)(want < 1 ? 1 : (want > cap ? cap : want)), 256, 0, s>>>((uint4 *)temp, words);
+            B200ALG_LAUNCH_CHECK();
+        }
         B200ALG_CUDA_TRY(launch_dependent(scan_kernel<T, OP, INCLUSIVE>, dim3(general_tiles), dim3(kScanThreads), 0, s, (const T *)in, in_stride,
                                           (T *)out, out_stride, n, carry_t, hdr, state, general_tiles));
     }
