@@ -1,7 +1,7 @@
 // Radix sort: onesweep-style least-significant-digit sort with 8-bit digits.
 //
 //   1. one pass over the keys builds the histograms of ALL digit positions,
-//   2. a one-block kernel turns them into global digit offsets and finds digit positions
+//   2. its last block turns them into global digit offsets and finds digit positions
 //      on which every key agrees (those passes are skipped),
 //   3. one kernel per remaining digit position moves every key to its final place for that digit, each
 //      key read once and written once (digit_pass.cuh).
@@ -30,7 +30,8 @@ enum : int {
     kCtlFirstPass = 25,    // first pass that runs (kNoPass when every pass is skipped)
     kCtlDst = 32,          // [32..39] buffer this pass writes
     kCtlStatusHalf = 40,   // [40..47] which of the two look-back arrays this pass uses
-    kCtlRole = 48          // [48..55] blocks of this pass that have started
+    kCtlRole = 48,         // [48..55] blocks of this pass that have started
+    kCtlHistogram = 56     // histogram blocks that have finished
 };
 // The three buffers a sort moves its data between.
 enum : unsigned int { kBufIn = 0, kBufOut = 1, kBufAlt = 2 };
@@ -59,7 +60,63 @@ static bool key_xform_constants(int dtype, int order, uint64_t &xn, uint64_t &xp
     return true;
 }
 
-// ---- 1. histograms of all digit positions ----------------------------------------------
+// ---- 1. global digit offsets, skipped passes, buffer schedule ---------------------------
+// skip_enabled: a pass on whose digit every key agrees does not run.  out_of_place: the input
+// view is only read; the passes then alternate between the output view and the alternate
+// buffer so that the last one writes the output view.  In place, they alternate between the
+// view and the alternate buffer, and the result is copied home if it ended in the latter.
+// Called by all threads of a block of GROUPS x 256; a group takes a digit position at a time.
+template <int GROUPS>
+__device__ __forceinline__ void digit_offsets(const unsigned long long *ghist, unsigned long long *gbase, TempHeader *hdr, int passes,
+                                              long long n, int skip_enabled, int out_of_place) {
+    __shared__ unsigned long long warp_sum[GROUPS][kRadix / 32];
+    __shared__ int skip[kMaxPasses];
+    const int group = threadIdx.x / kRadix, d = threadIdx.x % kRadix, lane = d & 31, warp = d >> 5;
+    if (threadIdx.x < kMaxPasses) skip[threadIdx.x] = 0;
+    for (int first = 0; first < passes; first += GROUPS) {
+        const int p = first + group;
+        __syncthreads();
+        const unsigned long long c = p < passes ? __ldcg(ghist + p * kRadix + d) : 0ull;
+        if (p < passes && skip_enabled && c == (unsigned long long)n) skip[p] = 1;
+        unsigned long long incl = c;
+#pragma unroll
+        for (int k = 1; k < 32; k <<= 1) {
+            unsigned long long up = __shfl_up_sync(0xffffffffu, incl, k);
+            if (lane >= k) incl += up;
+        }
+        if (lane == 31) warp_sum[group][warp] = incl;
+        __syncthreads();
+        unsigned long long before = 0;
+        for (int w = 0; w < warp; ++w) before += warp_sum[group][w];
+        if (p < passes) gbase[p * kRadix + d] = before + incl - c;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int running = 0;
+        for (int p = 0; p < passes; ++p) running += skip[p] ? 0 : 1;
+        unsigned int first = kNoPass, cur = out_of_place ? kBufIn : kBufOut;
+        int j = 0;
+        for (int p = 0; p < passes; ++p) {
+            hdr->reserved[kCtlSkip + p] = (unsigned)skip[p];
+            if (skip[p]) continue;
+            if (first == kNoPass) first = (unsigned)p;
+            unsigned int dst;
+            if (out_of_place) dst = ((running - 1 - j) & 1) ? kBufAlt : kBufOut;
+            else dst = cur == kBufOut ? kBufAlt : kBufOut;
+            hdr->reserved[kCtlSrc + p] = cur;
+            hdr->reserved[kCtlDst + p] = dst;
+            hdr->reserved[kCtlStatusHalf + p] = (unsigned)(j & 1);
+            cur = dst;
+            ++j;
+        }
+        hdr->reserved[kCtlFinal] = cur;
+        hdr->reserved[kCtlFirstPass] = first;
+    }
+}
+
+// ---- 2. histograms of all digit positions ----------------------------------------------
+// The block that finishes last turns them into offsets and the schedule of the passes (a kernel of its
+// own for that cost 5 us).
 constexpr int kHistoThreads = 1024;
 // Counters per (digit position, digit): lane l uses replica l % replicas.  With 32 replicas
 // every lane of a warp has a bank of its own and an atomic instruction is one wavefront
@@ -70,7 +127,8 @@ constexpr int kHistoMaxSmem = 128 * 1024;
 template <typename K, int RSHIFT>
 __global__ void __launch_bounds__(kHistoThreads)
 sort_histogram_kernel(const K *__restrict__ keys, int64_t stride, int64_t n, const long long *n_device, KeyXform<K> xf,
-                      unsigned long long *ghist) {
+                      unsigned long long *ghist, unsigned long long *gbase, TempHeader *hdr, int out_of_place) {
+    grid_dependency_release();  // the first pass may take the SMs this kernel leaves
     constexpr int P = sizeof(K);
     if (n_device) {
         const long long v = *n_device;
@@ -129,62 +187,20 @@ sort_histogram_kernel(const K *__restrict__ keys, int64_t stride, int64_t n, con
         for (int r = 0; r < replicas; ++r) c += sh[(i << rshift) + ((r + threadIdx.x) & (replicas - 1))];
         if (c) atomicAdd(ghist + i, (unsigned long long)c);
     }
+    __shared__ bool last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(&hdr->reserved[kCtlHistogram], 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (last) {
+        __threadfence();
+        digit_offsets<kHistoThreads / kRadix>(ghist, gbase, hdr, P, (long long)n, 1, out_of_place);
+    }
 }
 
-// ---- 2. global digit offsets, skipped passes, buffer schedule ---------------------------
-// skip_enabled: a pass on whose digit every key agrees does not run.  out_of_place: the input
-// view is only read; the passes then alternate between the output view and the alternate
-// buffer so that the last one writes the output view.  In place, they alternate between the
-// view and the alternate buffer, and the result is copied home if it ended in the latter.
 __global__ void __launch_bounds__(kRadix)
-sort_offsets_kernel(const unsigned long long *ghist, unsigned long long *gbase, TempHeader *hdr, int passes, long long n,
-                    const long long *n_device, int skip_enabled, int out_of_place) {
-    __shared__ unsigned long long warp_sum[kRadix / 32];
-    __shared__ int s_skip;
-    const int d = threadIdx.x, lane = d & 31, warp = d >> 5;
-    if (n_device) {
-        const long long v = *n_device;
-        n = v < 0 ? 0 : (v > n ? n : v);
-    }
-    for (int p = 0; p < passes; ++p) {
-        if (d == 0) s_skip = 0;
-        __syncthreads();
-        const unsigned long long c = ghist[p * kRadix + d];
-        if (skip_enabled && c == (unsigned long long)n) s_skip = 1;
-        unsigned long long incl = c;
-#pragma unroll
-        for (int k = 1; k < 32; k <<= 1) {
-            unsigned long long up = __shfl_up_sync(0xffffffffu, incl, k);
-            if (lane >= k) incl += up;
-        }
-        if (lane == 31) warp_sum[warp] = incl;
-        __syncthreads();
-        unsigned long long before = 0;
-        for (int w = 0; w < warp; ++w) before += warp_sum[w];
-        gbase[p * kRadix + d] = before + incl - c;
-        if (d == 0) hdr->reserved[kCtlSkip + p] = (unsigned)s_skip;
-        __syncthreads();
-    }
-    if (d == 0) {
-        int running = 0;
-        for (int p = 0; p < passes; ++p) running += hdr->reserved[kCtlSkip + p] ? 0 : 1;
-        unsigned int first = kNoPass, cur = out_of_place ? kBufIn : kBufOut;
-        int j = 0;
-        for (int p = 0; p < passes; ++p) {
-            if (hdr->reserved[kCtlSkip + p]) continue;
-            if (first == kNoPass) first = (unsigned)p;
-            unsigned int dst;
-            if (out_of_place) dst = ((running - 1 - j) & 1) ? kBufAlt : kBufOut;
-            else dst = cur == kBufOut ? kBufAlt : kBufOut;
-            hdr->reserved[kCtlSrc + p] = cur;
-            hdr->reserved[kCtlDst + p] = dst;
-            hdr->reserved[kCtlStatusHalf + p] = (unsigned)(j & 1);
-            cur = dst;
-            ++j;
-        }
-        hdr->reserved[kCtlFinal] = cur;
-        hdr->reserved[kCtlFirstPass] = first;
-    }
+partition_offsets_kernel(const unsigned long long *ghist, unsigned long long *gbase, TempHeader *hdr, long long n) {
+    digit_offsets<1>(ghist, gbase, hdr, 1, n, 0, 1);  // one "pass" that always runs, from the input view to the output
 }
 
 // ---- 3. the partition pass -------------------------------------------------------------------
@@ -861,6 +877,7 @@ partition_kernel(SortBuffers<K, V> io, int pass, SplitterBucket<K> dg, TempHeade
 template <typename K, typename V>
 __global__ void __launch_bounds__(256)
 sort_copy_back_kernel(SortBuffers<K, V> io, const TempHeader *hdr, int value_seq) {
+    grid_dependency_wait();
     const int64_t n = effective_n(io);
     const int64_t step = (int64_t)gridDim.x * blockDim.x;
     const int64_t first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1008,13 +1025,11 @@ static int run_passes(cudaStream_t s, const SortCall &call, const KeyXform<K> &x
             }
         }
         if (big)
-            sort_histogram_kernel<K, kBigShift><<<blocks, kHistoThreads, histo_smem, s>>>(io.in, io.stride, n, io.n_device, xf, ghist);
+            sort_histogram_kernel<K, kBigShift><<<blocks, kHistoThreads, histo_smem, s>>>(io.in, io.stride, n, io.n_device, xf, ghist, gbase, hdr, call.out_of_place ? 1 : 0);
         else
-            sort_histogram_kernel<K, 3><<<blocks, kHistoThreads, histo_smem, s>>>(io.in, io.stride, n, io.n_device, xf, ghist);
+            sort_histogram_kernel<K, 3><<<blocks, kHistoThreads, histo_smem, s>>>(io.in, io.stride, n, io.n_device, xf, ghist, gbase, hdr, call.out_of_place ? 1 : 0);
         B200ALG_LAUNCH_CHECK();
     }
-    sort_offsets_kernel<<<1, kRadix, 0, s>>>(ghist, gbase, hdr, L.passes, (long long)n, io.n_device, 1, call.out_of_place ? 1 : 0);
-    B200ALG_LAUNCH_CHECK();
     for (int p = 0; p < L.passes; ++p) {
         XF pass_xf;
         if constexpr (std::is_same<XF, KeyXform<K>>::value) pass_xf = xf;
@@ -1027,8 +1042,7 @@ static int run_passes(cudaStream_t s, const SortCall &call, const KeyXform<K> &x
         int64_t want = ceil_div(n, 256 * 8);
         const int64_t cap = (int64_t)sm_count() * 8;
         const int blocks = (int)(want < 1 ? 1 : (want > cap ? cap : want));
-        sort_copy_back_kernel<K, V><<<blocks, 256, 0, s>>>(io, hdr, call.value_seq);
-        B200ALG_LAUNCH_CHECK();
+        B200ALG_CUDA_TRY(launch_dependent(sort_copy_back_kernel<K, V>, dim3(blocks), dim3(256), 0, s, io, (const TempHeader *)hdr, call.value_seq));
     }
     return B200ALG_OK;
 }
@@ -1178,7 +1192,7 @@ static int run_partition(cudaStream_t s, const K *keys, const V *values, int64_t
     }
     // One "pass": offsets of the buckets; the skip rule is off (n + 1 never matches a count),
     // so the pass always moves the keys from buffer 0 (input) to buffer 1 (output).
-    sort_offsets_kernel<<<1, kRadix, 0, s>>>(ghist, gbase, hdr, 1, (long long)n, nullptr, 0, 1);
+    partition_offsets_kernel<<<1, kRadix, 0, s>>>(ghist, gbase, hdr, (long long)n);
     B200ALG_LAUNCH_CHECK();
     export_bucket_counts_kernel<<<1, kRadix, 0, s>>>(ghist, counts, num_buckets);
     B200ALG_LAUNCH_CHECK();
@@ -1226,7 +1240,7 @@ static int run_bucket_scatter(cudaStream_t s, const K *keys, const V *values, in
     B200ALG_CUDA_TRY(cudaMemsetAsync(temp, 0, (size_t)L.control_bytes, s));
     // all-zero histogram: the bucket offsets come out zero (every bucket has its own base
     // pointer) and the pass is scheduled from buffer 0
-    sort_offsets_kernel<<<1, kRadix, 0, s>>>(ghist, gbase, hdr, 1, (long long)n, nullptr, 0, 1);
+    partition_offsets_kernel<<<1, kRadix, 0, s>>>(ghist, gbase, hdr, (long long)n);
     B200ALG_LAUNCH_CHECK();
     SortBuffers<K, V> io{keys, nullptr, nullptr, values, nullptr, nullptr, 1, n, nullptr};
     kernel<<<grid, THREADS, Smem::bytes, s>>>(io, 0, dg, hdr, gbase, status, (int)L.tiles);
