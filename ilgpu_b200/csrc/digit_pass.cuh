@@ -440,9 +440,7 @@ digit_pass_kernel(SortBuffers<K, V> io, int pass, XF xf, TempHeader *hdr, const 
             }
             if (lane == 31) m.warp_sum[warp] = incl;
             __syncthreads();
-            unsigned int excl = incl - total;
-#pragma unroll
-            for (int w = 0; w < kPassWarps; ++w) excl += w < warp ? m.warp_sum[w] : 0u;
+            const unsigned int excl = incl - total + __reduce_add_sync(0xffffffffu, lane < warp ? m.warp_sum[lane] : 0u);
             if (part == 0) reinterpret_cast<unsigned int *>(smem + L::off_excl)[turn * kRadix + d] = excl;
 #pragma unroll
             for (int w = 0; w < kDigitRows; w += 2) {

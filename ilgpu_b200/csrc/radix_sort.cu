@@ -128,7 +128,6 @@ template <typename K, int RSHIFT>
 __global__ void __launch_bounds__(kHistoThreads)
 sort_histogram_kernel(const K *__restrict__ keys, int64_t stride, int64_t n, const long long *n_device, KeyXform<K> xf,
                       unsigned long long *ghist, unsigned long long *gbase, TempHeader *hdr, int out_of_place) {
-    grid_dependency_release();  // the first pass may take the SMs this kernel leaves
     constexpr int P = sizeof(K);
     if (n_device) {
         const long long v = *n_device;
@@ -1011,7 +1010,7 @@ static int run_passes(cudaStream_t s, const SortCall &call, const KeyXform<K> &x
         int64_t want = ceil_div(n, per_block);
         // 32 counter replicas for long inputs (16 for 8-byte keys: 128 KB either way), else 8
         constexpr int kBigShift = sizeof(K) == 8 ? 4 : 5;
-        const bool big = n >= (1ll << 22);
+        const bool big = n >= (1ll << 19);
         const size_t histo_smem = (size_t)sizeof(K) * kRadix * sizeof(unsigned int) << (big ? kBigShift : 3);
         const int64_t cap = (int64_t)sm_count() * (histo_smem > 100 * 1024 ? 1 : 2);
         const int blocks = (int)(want < 1 ? 1 : (want > cap ? cap : want));
