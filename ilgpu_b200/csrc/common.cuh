@@ -192,6 +192,9 @@ __device__ __forceinline__ void mbar_init(unsigned long long *bar, unsigned int 
 __device__ __forceinline__ void mbar_expect_tx(unsigned long long *bar, unsigned int bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes) : "memory");
 }
+__device__ __forceinline__ void mbar_arrive(unsigned long long *bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
+}
 __device__ __forceinline__ bool mbar_try_wait(unsigned long long *bar, unsigned int parity) {
     unsigned int ok;
     asm volatile(
@@ -211,8 +214,8 @@ __device__ __forceinline__ void bulk_load(void *smem_dst, const void *gsrc, unsi
                  : "memory");
 }
 // Bounded wait; false when the limit ran out.
-__device__ __forceinline__ bool mbar_wait(unsigned long long *bar, unsigned int parity) {
-    for (unsigned int polls = 0; polls < kMaxBarrierPolls; ++polls)
+__device__ __forceinline__ bool mbar_wait(unsigned long long *bar, unsigned int parity, unsigned int max_polls = kMaxBarrierPolls) {
+    for (unsigned int polls = 0; polls < max_polls; ++polls)
         if (mbar_try_wait(bar, parity)) return true;
     return false;
 }

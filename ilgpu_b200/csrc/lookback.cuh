@@ -19,9 +19,10 @@ template <typename T, int BYTES = sizeof(T)> struct TileState;
 
 template <typename T> struct TileState<T, 4> {
     unsigned char *base;
-    __host__ __device__ TileState(void *b, int) : base((unsigned char *)b) {}
+    int stride;
+    __host__ __device__ TileState(void *b, int, int stride_ = kDescStride) : base((unsigned char *)b), stride(stride_) {}
     __device__ __forceinline__ unsigned long long *word(int tile) const {
-        return (unsigned long long *)(base + (size_t)tile * kDescStride);
+        return (unsigned long long *)(base + (size_t)tile * stride);
     }
     __device__ __forceinline__ void publish(int tile, unsigned int flag, T v) {
         unsigned int bits;
@@ -38,17 +39,18 @@ template <typename T> struct TileState<T, 4> {
 
 template <typename T> struct TileState<T, 8> {
     unsigned char *base;
-    __host__ __device__ TileState(void *b, int) : base((unsigned char *)b) {}
+    int stride;
+    __host__ __device__ TileState(void *b, int, int stride_ = kDescStride) : base((unsigned char *)b), stride(stride_) {}
     __device__ __forceinline__ void publish(int tile, unsigned int flag, T v) {
         unsigned long long bits;
         memcpy(&bits, &v, 8);
         asm volatile("{\n\t.reg .b128 w;\n\tmov.b128 w, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], w;\n\t}"
-                     ::"l"(base + (size_t)tile * kDescStride), "l"(bits), "l"((unsigned long long)flag) : "memory");
+                     ::"l"(base + (size_t)tile * stride), "l"(bits), "l"((unsigned long long)flag) : "memory");
     }
     __device__ __forceinline__ unsigned int poll(int tile, T &v) {
         unsigned long long bits, flag;
         asm volatile("{\n\t.reg .b128 w;\n\tld.relaxed.gpu.global.b128 w, [%2];\n\tmov.b128 {%0, %1}, w;\n\t}"
-                     : "=l"(bits), "=l"(flag) : "l"(base + (size_t)tile * kDescStride) : "memory");
+                     : "=l"(bits), "=l"(flag) : "l"(base + (size_t)tile * stride) : "memory");
         memcpy(&v, &bits, 8);
         return (unsigned int)flag;
     }

@@ -1,4 +1,5 @@
-// Scan: single-pass chained scan with decoupled look-back.
+// Scan: every tile is read once and written once; the tiles' prefixes come from a scanner warp that
+// follows their totals (dense views) or from decoupled look-back (all others).
 // Replaces SinglePassScanKernel + its tile helpers (ScanExtensions.cs:284-388, :530-706),
 // whose groups hand one running value down a strictly serial chain
 // (SequentialGroupExecutor.cs:58-77) and read the input twice.  Here every tile is read
@@ -168,246 +169,325 @@ __global__ void __launch_bounds__(256) scan_clear_kernel(uint4 *words, int64_t c
 }
 
 // ---- pipelined variant for dense views that are aligned alike ---------------------------
-// Persistent blocks take tiles round-robin (tile = blockIdx.x + k * gridDim.x).  A tile waits
-// for the tiles before it, so every block of the grid has to be resident at the same time:
-// the kernel is launched cooperatively, which makes the driver guarantee exactly that (or
-// refuse the launch, in which case the ticketed kernel above runs instead).  Handing the
-// tiles out by an atomic ticket, as the general kernel does, needs no such guarantee but
-// measured 2.5 to 3 times slower on long inputs, whatever the prefetch distance.
-// The input of the next tiles is staged into a shared-memory ring by bulk asynchronous
-// copies (TMA, one elected thread, completion on an mbarrier), which keeps loads in flight
-// while a block is busy with the scan and the look-back of its current tile.
-// (A look-back warp of its own, with the finished tile waiting in registers for its prefix while the
-// others scan the next, measured slower: 1626 us against 1512 us for 2^30 floats, the registers cost
-// a block per SM.)
+// Persistent blocks take tiles round-robin (tile = blockIdx.x + k * (gridDim.x - 1)); the last block is
+// the scanner, one warp that reads the tiles' totals as they appear and publishes the tiles' prefixes.
+// Blocks wait for one another, so every block of the grid has to be resident at the same time: the
+// kernel is launched cooperatively, which makes the driver guarantee exactly that (or refuse the
+// launch, in which case the ticketed kernel above runs instead).  Handing the tiles out by an atomic
+// ticket, as the general kernel does, needs no such guarantee but measured 2.5 to 3 times slower on
+// long inputs, whatever the prefetch distance.
+//
+// A prefix takes several trips through an L2 that is busy with the tiles themselves, some 5000 cycles.
+// They pass while the block works on the tile before and the tile after: a tile is looked at twice,
+// first for its total, which is handed to the scanner, and one tile later, when its prefix has come,
+// to be scanned and stored.  In between it stays in a ring of kPipeStages tiles in shared memory, into
+// which bulk copies (TMA) bring the tiles ahead.  Eight warps do that; one more hands out the totals
+// and issues the copies, one fetches the prefixes; they meet only in mbarriers.
+//
+// Bound by DRAM: 2^30 floats take 1304 us (6590 GB/s) where look-back in every block, with the tile held
+// in registers meanwhile, took 1490; 2^28 int64 672 instead of 900 us, 2^24 int32 29.7 instead of
+// 33.4 us.  Tiles of 32 KB and two blocks per SM: the scanner manages a tile every 18 cycles or so,
+// which tiles of 24 KB (1357 us) and 16 KB (1791 us) outrun; one block of 512 threads with 64 KB tiles
+// 1330 us, a fourth stage of 24 KB 1399 us.
 //
 // in and out start on 16 bytes; a view that does not begins with `lead` elements that belong to
 // whatever is in front of it, read as Identity and not stored.
-constexpr int kScanStages = 2;
-constexpr int kScanTileBytes = kScanThreads * kScanVecPerThread * 16;
+constexpr int kPipeStages = 3;
+constexpr int kPipeVecs = 8;
+constexpr int kPipeTileBytes = kScanThreads * kPipeVecs * 16;
+constexpr int kPipeThreads = kScanThreads + 64;
+constexpr int kPrefixRows = 4;  // rows of 32 tiles a scanner round looks at (2 and 8: 6 and 10 % slower)
+
+// The words the tiles of the pipelined scan and its scanner exchange: two dense arrays, the tiles' totals
+// and the tiles' prefixes.
+template <typename T> struct TileWords {
+    static constexpr int kBytes = 2 * sizeof(T);
+    static_assert(2 * kBytes <= kDescStride, "fits where the general kernel has its records");
+    TileState<T> totals, prefixes;
+    __device__ TileWords(void *base, int tiles)
+        : totals(base, tiles, kBytes), prefixes((unsigned char *)base + (size_t)(tiles + 1) / 2 * 2 * kBytes, tiles, kBytes) {}
+    static __host__ __device__ int64_t vectors(int tiles) { return (int64_t)((tiles + 1) / 2) * 2 * 2 * kBytes / 16; }
+};
+
+// One warp turns the tiles' totals into their prefixes, kPrefixRows * 32 tiles at a time.
+template <typename T, int OP>
+__device__ __forceinline__ void scan_totals(TileWords<T> words, const T *carry_in, int num_tiles, TempHeader *hdr) {
+    using O = Op<T, OP>;
+    const int lane = threadIdx.x & 31;
+    T carry = carry_in ? *carry_in : O::identity();
+    unsigned int spins = 0;
+    for (int pos = 0; pos < num_tiles;) {
+        T own[kPrefixRows];
+        unsigned int flag[kPrefixRows];
+#pragma unroll
+        for (int m = 0; m < kPrefixRows; ++m) {
+            const int t = pos + m * 32 + lane;
+            flag[m] = kInvalid;
+            own[m] = O::identity();
+            if (t < num_tiles) flag[m] = words.totals.poll(t, own[m]);
+        }
+        int ready = 0;  // totals that are there, from the first one on
+#pragma unroll
+        for (int m = 0; m < kPrefixRows; ++m) {
+            const unsigned int missing = __ballot_sync(0xffffffffu, flag[m] == kInvalid);
+            if (ready == m * 32) ready += missing ? __ffs((int)missing) - 1 : 32;
+        }
+        if (ready == 0) {
+            if (++spins > kMaxSpin) {
+                if (lane == 0) atomicExch(&hdr->wait_limit_hit, 1u);
+                return;
+            }
+            continue;
+        }
+        spins = 0;
+        T incl[kPrefixRows];
+#pragma unroll
+        for (int m = 0; m < kPrefixRows; ++m) incl[m] = m * 32 + lane < ready ? own[m] : O::identity();
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+#pragma unroll
+            for (int m = 0; m < kPrefixRows; ++m) {
+                const T up = shfl_up(incl[m], d);
+                if (lane >= d) incl[m] = O::apply(up, incl[m]);
+            }
+        }
+#pragma unroll
+        for (int m = 0; m < kPrefixRows; ++m) {
+            T ex = shfl_up(incl[m], 1);
+            if (lane == 0) ex = O::identity();
+            if (m * 32 + lane < ready) words.prefixes.publish(pos + m * 32 + lane, kInclusive, O::apply(carry, ex));
+            carry = O::apply(carry, shfl_idx(incl[m], 31));
+        }
+        pos += ready;
+    }
+}
 
 template <typename T, int OP, bool INCLUSIVE, bool LEAD>
-__global__ void __launch_bounds__(kScanThreads)
+__global__ void __launch_bounds__(kPipeThreads, 2)
 scan_pipeline_kernel(const T *in, T *out, int64_t n, int lead_arg, const T *carry_in, TempHeader *hdr, void *state_base, int num_tiles) {
     using O = Op<T, OP>;
     constexpr int VEC = 16 / sizeof(T);
-    constexpr int NV = kScanVecPerThread;
+    constexpr int NV = kPipeVecs;
     constexpr int TILE = VEC * NV * kScanThreads;
     union Vec { uint4 u; T t[VEC]; };
 
-    extern __shared__ __align__(128) unsigned char ring[];  // kScanStages x kScanTileBytes
-    __shared__ __align__(8) unsigned long long full_bar[kScanStages];
-    __shared__ T warp_total[kScanWarps];
-    __shared__ T warp_excl[kScanWarps];
-    __shared__ T s_prefix;
-    __shared__ int s_failed;               // a wait for a bulk copy ran out: later tiles are loaded directly
+    extern __shared__ __align__(128) unsigned char ring[];  // kPipeStages x kPipeTileBytes
+    __shared__ __align__(8) unsigned long long full_bar[kPipeStages];  // the copy of a tile has arrived
+    __shared__ __align__(8) unsigned long long free_bar[kPipeStages];  // every warp has taken its part of a tile
+    __shared__ __align__(8) unsigned long long totals_bar[2];          // every warp has its total of a tile
+    __shared__ __align__(8) unsigned long long base_bar[2];            // what precedes each warp's part is known
+    __shared__ T totals[2][kScanWarps];
+    __shared__ T bases[2][kScanWarps];
+    __shared__ int s_failed;  // a wait ran out
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // (LEAD is a template parameter because the extra register costs aligned views 5 %)
     const int lead = LEAD ? lead_arg : 0;
     const int full_tiles = (int)(n / TILE);          // tiles below this index are complete,
     constexpr int first_full = LEAD ? 1 : 0;         // from this one on
-
-    // The last thread issues the copies: warp 0 does the look-back.
-    constexpr int kStager = kScanThreads - 1;
-    const int G = (int)gridDim.x;
-    unsigned int in_flight = 0;  // stager: bit st set = a copy into stage st has not been waited for
-    if (tid == kStager) {
+    const int G = (int)gridDim.x - 1;                // the last block is the scanner
+    const bool scanner = (int)blockIdx.x == G;
+    const int my_tiles = scanner ? 0 : (num_tiles - (int)blockIdx.x + G - 1) / G;
+    auto tile_of = [&](int k) { return (int)blockIdx.x + k * G; };
+    auto is_full = [&](int tile) { return tile >= first_full && tile < full_tiles; };
+    auto stage_in = [&](int k) {
+        const int st = k % kPipeStages;
+        mbar_expect_tx(&full_bar[st], kPipeTileBytes);
+        bulk_load(ring + st * kPipeTileBytes, in + (int64_t)tile_of(k) * TILE, kPipeTileBytes, &full_bar[st]);
+    };
+    if (tid == kScanThreads) {
         s_failed = 0;
-        for (int st = 0; st < kScanStages; ++st) mbar_init(&full_bar[st], 1u);
+        for (int st = 0; st < kPipeStages; ++st) {
+            mbar_init(&full_bar[st], 1u);
+            mbar_init(&free_bar[st], kScanWarps);
+        }
+        for (int h = 0; h < 2; ++h) {
+            mbar_init(&totals_bar[h], kScanWarps);
+            mbar_init(&base_bar[h], 1u);
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        for (int st = 0; st < kScanStages; ++st) {
-            const int t = (int)blockIdx.x + st * G;
-            if (t >= first_full && t < full_tiles) {
-                mbar_expect_tx(&full_bar[st], kScanTileBytes);
-                bulk_load(ring + st * kScanTileBytes, in + (int64_t)t * TILE, kScanTileBytes, &full_bar[st]);
-                in_flight |= 1u << st;
-            }
-        }
+        for (int k = 0; k < kPipeStages && k < my_tiles; ++k)
+            if (is_full(tile_of(k))) stage_in(k);
     }
-    // The descriptors of this block's tiles; every block has to have cleared its own before anybody
-    // publishes (while the first tiles are on their way).
+    // The words have to be cleared before anybody publishes (while the first tiles are on their way).
     if (blockIdx.x == 0 && tid == 0) hdr->wait_limit_hit = 0u;
-    for (int64_t t = (int64_t)blockIdx.x + (int64_t)tid * G; t < num_tiles; t += (int64_t)kScanThreads * G)
-        *reinterpret_cast<uint4 *>((unsigned char *)state_base + (size_t)t * kDescStride) = make_uint4(0u, 0u, 0u, 0u);
+    for (int64_t i = (int64_t)blockIdx.x * kPipeThreads + tid; i < TileWords<T>::vectors(num_tiles); i += (int64_t)gridDim.x * kPipeThreads)
+        reinterpret_cast<uint4 *>(state_base)[i] = make_uint4(0u, 0u, 0u, 0u);
     cg::this_grid().sync();
-    unsigned int bar_phase = 0;  // bit st = parity of the next completion of stage st's barrier
-    bool staging = true;         // false once a wait for a copy ran out: later tiles are loaded directly
-    TileState<T> state(state_base, num_tiles);
+    TileWords<T> words(state_base, num_tiles);
+    if (scanner) {
+        if (warp == 0) scan_totals<T, OP>(words, carry_in, num_tiles, hdr);
+        return;
+    }
+    unsigned int max_polls = kMaxBarrierPolls;  // a thread whose wait ran out does not wait as long again
+    auto wait = [&](unsigned long long *bar, unsigned int parity) {
+        if (mbar_wait(bar, parity, max_polls)) return true;
+        max_polls = 1u;
+        s_failed = 1;
+        return false;
+    };
 
-    int k = 0;
-    for (int tile = (int)blockIdx.x; tile < num_tiles; tile += G, ++k) {
-        const int st = k % kScanStages;
-        const int64_t base = (int64_t)tile * TILE;
-        const bool full = tile >= first_full && tile < full_tiles;
-        const bool staged = full && staging;
-
-        // Vector j of lane l covers elements (warp*32*NV + j*32 + l) * VEC ... + VEC of the tile.
-        Vec v[NV];
-        if (staged) {
-            if (!mbar_wait(&full_bar[st], (bar_phase >> st) & 1u)) s_failed = 1;
-            bar_phase ^= 1u << st;
-            const uint4 *src = reinterpret_cast<const uint4 *>(ring + st * kScanTileBytes) + warp * (32 * NV);
+    if (warp == kScanWarps) {  // hands the tiles' totals to the scanner and keeps copies coming
+        for (int k = 0; k < my_tiles; ++k) {
+            wait(&totals_bar[k & 1], (unsigned int)(k >> 1) & 1u);
+            T total = lane < kScanWarps ? totals[k & 1][lane] : O::identity();
 #pragma unroll
-            for (int j = 0; j < NV; ++j) v[j].u = src[j * 32 + lane];
-            if (tid == kStager) in_flight &= ~(1u << st);
-        } else {
-#pragma unroll
-            for (int j = 0; j < NV; ++j)
-#pragma unroll
-                for (int e = 0; e < VEC; ++e) {
-                    const int64_t idx = base + (int64_t)(warp * (32 * NV) + j * 32 + lane) * VEC + e;
-                    v[j].t[e] = idx >= lead && idx < n ? in[idx] : O::identity();
+            for (int d = kScanWarps / 2; d > 0; d >>= 1) total = O::apply(total, shfl_down(total, d));
+            if (lane == 0) {
+                words.totals.publish(tile_of(k), kAggregate, total);
+                const int next = k + kPipeStages - 1;
+                if (k >= 1 && next < my_tiles && is_full(tile_of(next))) {
+                    wait(&free_bar[(k - 1) % kPipeStages], (unsigned int)((k - 1) / kPipeStages) & 1u);
+                    stage_in(next);
                 }
-        }
-
-        // inclusive scan inside each vector, then NV interleaved warp scans of the vector totals
-        T w[NV];
-#pragma unroll
-        for (int j = 0; j < NV; ++j) {
-#pragma unroll
-            for (int e = 1; e < VEC; ++e) v[j].t[e] = O::apply(v[j].t[e - 1], v[j].t[e]);
-            w[j] = v[j].t[VEC - 1];
-        }
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-#pragma unroll
-            for (int j = 0; j < NV; ++j) {
-                const T up = shfl_up(w[j], d);
-                if (lane >= d) w[j] = O::apply(up, w[j]);
             }
+            __syncwarp();
         }
-        T before[NV];  // fold of everything in the warp's chunk that precedes vector j of this lane
-        T chunk = O::identity();
-#pragma unroll
-        for (int j = 0; j < NV; ++j) {
-            T ex = shfl_up(w[j], 1);
-            if (lane == 0) ex = O::identity();
-            before[j] = O::apply(chunk, ex);
-            chunk = O::apply(chunk, shfl_idx(w[j], 31));
-        }
-        if (lane == 31) warp_total[warp] = chunk;
-        __syncthreads();  // warp totals are visible; every thread has taken its data out of the ring
-
-        if (s_failed) staging = false;  // (read by every thread between the two barriers: uniform)
-        if (tid == kStager && staging) {
-            const int t2 = tile + kScanStages * G;
-            if (t2 < full_tiles) {
-                mbar_expect_tx(&full_bar[st], kScanTileBytes);
-                bulk_load(ring + st * kScanTileBytes, in + (int64_t)t2 * TILE, kScanTileBytes, &full_bar[st]);
-                in_flight |= 1u << st;
-            }
-        }
-
-        if (warp == 0) {
-            T wt = lane < kScanWarps ? warp_total[lane] : O::identity();
-            T wi = wt;
+    } else if (warp > kScanWarps) {  // fetches the tiles' prefixes
+        unsigned int max_spins = kMaxSpin;
+        for (int k = 0; k < my_tiles; ++k) {
+            wait(&totals_bar[k & 1], (unsigned int)(k >> 1) & 1u);
+            T sum = lane < kScanWarps ? totals[k & 1][lane] : O::identity();
 #pragma unroll
             for (int d = 1; d < kScanWarps; d <<= 1) {
-                T up = shfl_up(wi, d);
-                if (lane >= d) wi = O::apply(up, wi);
+                const T up = shfl_up(sum, d);
+                if (lane >= d) sum = O::apply(up, sum);
             }
-            T we = shfl_up(wi, 1);
-            if (lane == 0) we = O::identity();
-            if (lane < kScanWarps) warp_excl[lane] = we;
-            const T aggregate = shfl_idx(wi, kScanWarps - 1);
-
-            T prefix;
-            if (tile == 0) {
-                prefix = carry_in ? *carry_in : O::identity();
-                if (lane == 0) state.publish(0, kInclusive, O::apply(prefix, aggregate));
-            } else {
-                if (lane == 0) state.publish(tile, kAggregate, aggregate);
-                // Decoupled look-back over kLookWays * 32 predecessors per round: lane l polls
-                // the tiles at distances l+1, l+33, ... so that several loads are in flight per
-                // lane; the operations are commutative, so the round's values are simply folded.
-                constexpr int kLookWays = 1;
-                constexpr int kLookLanes = 32;
-                prefix = O::identity();
-                int look = tile - 1 - lane;
-                bool gave_up = false;
-                while (true) {
-                    T pv[kLookWays];
-                    unsigned int flag[kLookWays];
-#pragma unroll
-                    for (int m = 0; m < kLookWays; ++m) {
-                        pv[m] = O::identity();
-                        flag[m] = kInclusive;  // tiles before tile 0 act as "inclusive identity"
-                        if (lane >= kLookLanes) flag[m] = kAggregate;  // outside the window: contributes nothing
-                        else if (look - 32 * m >= 0) flag[m] = state.poll(look - 32 * m, pv[m]);
+            T ahead = shfl_up(sum, 1);
+            if (lane == 0) ahead = O::identity();
+            T prefix = O::identity();
+            if (lane == 0) {
+                unsigned int spins = 0;
+                while (words.prefixes.poll(tile_of(k), prefix) == kInvalid) {
+                    if (++spins > max_spins) {
+                        atomicExch(&hdr->wait_limit_hit, 1u);
+                        max_spins = 1u;
+                        prefix = O::identity();
+                        break;
                     }
+                }
+            }
+            prefix = shfl_idx(prefix, 0);
+            if (lane < kScanWarps) bases[k & 1][lane] = O::apply(prefix, ahead);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&base_bar[k & 1]);
+        }
+    } else {
+        // Vector j of lane l covers elements (warp*32*NV + j*32 + l) * VEC ... + VEC of the tile.
+        unsigned int phase = 0u;  // bit st = parity of the next completion of stage st's copy
+        for (int k = 0; k <= my_tiles; ++k) {
+            if (k < my_tiles) {  // this warp's total of tile k
+                const int st = k % kPipeStages;
+                const int64_t base = (int64_t)tile_of(k) * TILE;
+                uint4 *slot = reinterpret_cast<uint4 *>(ring + st * kPipeTileBytes) + warp * (32 * NV) + lane;
+                bool staged = is_full(tile_of(k));
+                if (staged) {
+                    staged = wait(&full_bar[st], (phase >> st) & 1u);
+                    phase ^= 1u << st;
+                }
+                T total = O::identity();
+                if (staged) {
+                    Vec v[NV];
 #pragma unroll
-                    for (int m = 0; m < kLookWays; ++m) {
-                        unsigned int spins = 0;
-                        while (flag[m] == kInvalid) {
-                            if (++spins > kMaxSpin) { gave_up = true; flag[m] = kInclusive; pv[m] = O::identity(); break; }
-                            __nanosleep(20);
-                            flag[m] = state.poll(look - 32 * m, pv[m]);
+                    for (int j = 0; j < NV; ++j) v[j].u = slot[j * 32];
+#pragma unroll
+                    for (int j = 0; j < NV; ++j)
+#pragma unroll
+                        for (int e = 0; e < VEC; ++e) total = O::apply(total, v[j].t[e]);
+                } else {
+                    for (int j = 0; j < NV; ++j) {
+                        Vec v;
+#pragma unroll
+                        for (int e = 0; e < VEC; ++e) {
+                            const int64_t idx = base + (int64_t)(warp * (32 * NV) + j * 32 + lane) * VEC + e;
+                            v.t[e] = idx >= lead && idx < n ? in[idx] : O::identity();
+                            total = O::apply(total, v.t[e]);
                         }
+                        slot[j * 32] = v.u;
                     }
-                    // nearest predecessor with an inclusive prefix: smallest distance m*32 + lane
-                    int nearest = kLookWays * 32;
-#pragma unroll
-                    for (int m = kLookWays - 1; m >= 0; --m) {
-                        const unsigned int mask = __ballot_sync(0xffffffffu, flag[m] == kInclusive);
-                        if (mask) nearest = m * 32 + (__ffs(mask) - 1);
-                    }
-                    T contrib = O::identity();
-#pragma unroll
-                    for (int m = 0; m < kLookWays; ++m)
-                        if (m * 32 + lane <= nearest) contrib = O::apply(pv[m], contrib);
-#pragma unroll
-                    for (int d = 16; d > 0; d >>= 1) contrib = O::apply(shfl_down(contrib, d), contrib);
-                    prefix = O::apply(shfl_idx(contrib, 0), prefix);
-                    if (nearest < kLookWays * 32) break;
-                    look -= kLookWays > 1 ? kLookWays * 32 : kLookLanes;
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // (a copy may come into these slots next)
                 }
-                if (__any_sync(0xffffffffu, gave_up) && lane == 0) atomicExch(&hdr->wait_limit_hit, 1u);
-                if (lane == 0) state.publish(tile, kInclusive, O::apply(prefix, aggregate));
+#pragma unroll
+                for (int d = 16; d > 0; d >>= 1) total = O::apply(total, shfl_down(total, d));
+                if (lane == 0) {
+                    totals[k & 1][warp] = total;
+                    mbar_arrive(&totals_bar[k & 1]);
+                }
             }
-            if (lane == 0) s_prefix = prefix;
-        }
-        __syncthreads();
+            if (k == 0) continue;
 
-        const T warp_base = O::apply(s_prefix, warp_excl[warp]);
+            // tile k - 1: scan and store
+            const int q = k - 1, st = q % kPipeStages;
+            const int64_t base = (int64_t)tile_of(q) * TILE;
+            const uint4 *slot = reinterpret_cast<const uint4 *>(ring + st * kPipeTileBytes) + warp * (32 * NV) + lane;
+            Vec v[NV];
 #pragma unroll
-        for (int j = 0; j < NV; ++j) {
-            const T p = O::apply(warp_base, before[j]);
-            if (INCLUSIVE) {
+            for (int j = 0; j < NV; ++j) v[j].u = slot[j * 32];
+            // inclusive scan inside each vector, then NV interleaved warp scans of the vector totals
+            T w[NV];
 #pragma unroll
-                for (int e = 0; e < VEC; ++e) v[j].t[e] = O::apply(p, v[j].t[e]);
+            for (int j = 0; j < NV; ++j) {
+#pragma unroll
+                for (int e = 1; e < VEC; ++e) v[j].t[e] = O::apply(v[j].t[e - 1], v[j].t[e]);
+                w[j] = v[j].t[VEC - 1];
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&free_bar[st]);
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+#pragma unroll
+                for (int j = 0; j < NV; ++j) {
+                    const T up = shfl_up(w[j], d);
+                    if (lane >= d) w[j] = O::apply(up, w[j]);
+                }
+            }
+            T before[NV];  // fold of everything in the warp's part that precedes vector j of this lane
+            T chunk = O::identity();
+#pragma unroll
+            for (int j = 0; j < NV; ++j) {
+                T ex = shfl_up(w[j], 1);
+                if (lane == 0) ex = O::identity();
+                before[j] = O::apply(chunk, ex);
+                chunk = O::apply(chunk, shfl_idx(w[j], 31));
+            }
+            wait(&base_bar[q & 1], (unsigned int)(q >> 1) & 1u);
+            const T warp_base = bases[q & 1][warp];
+#pragma unroll
+            for (int j = 0; j < NV; ++j) {
+                const T p = O::apply(warp_base, before[j]);
+                if (INCLUSIVE) {
+#pragma unroll
+                    for (int e = 0; e < VEC; ++e) v[j].t[e] = O::apply(p, v[j].t[e]);
+                } else {
+#pragma unroll
+                    for (int e = VEC - 1; e > 0; --e) v[j].t[e] = O::apply(p, v[j].t[e - 1]);
+                    v[j].t[0] = p;
+                }
+            }
+            if (is_full(tile_of(q))) {
+                uint4 *dst = reinterpret_cast<uint4 *>(out + base) + warp * (32 * NV) + lane;
+#pragma unroll
+                for (int j = 0; j < NV; ++j) __stcs(dst + j * 32, v[j].u);
             } else {
 #pragma unroll
-                for (int e = VEC - 1; e > 0; --e) v[j].t[e] = O::apply(p, v[j].t[e - 1]);
-                v[j].t[0] = p;
+                for (int j = 0; j < NV; ++j)
+#pragma unroll
+                    for (int e = 0; e < VEC; ++e) {
+                        const int64_t idx = base + (int64_t)(warp * (32 * NV) + j * 32 + lane) * VEC + e;
+                        if (idx >= lead && idx < n) out[idx] = v[j].t[e];
+                    }
             }
-        }
-        if (full) {
-            uint4 *dst = reinterpret_cast<uint4 *>(out + base) + warp * (32 * NV);
-#pragma unroll
-            for (int j = 0; j < NV; ++j) __stcs(dst + j * 32 + lane, v[j].u);
-        } else {
-#pragma unroll
-            for (int j = 0; j < NV; ++j)
-#pragma unroll
-                for (int e = 0; e < VEC; ++e) {
-                    const int64_t idx = base + (int64_t)(warp * (32 * NV) + j * 32 + lane) * VEC + e;
-                    if (idx >= lead && idx < n) out[idx] = v[j].t[e];
-                }
         }
     }
 
-    // A barrier wait that ran out is reported; copies that may still be in flight are given
-    // one more bounded wait so that the block does not retire underneath them.
+    // A wait that ran out is reported; copies that may still be in flight are given one more bounded
+    // wait so that the block does not retire underneath them.
     __syncthreads();
-    if (s_failed) {
-        if (tid == kStager) {
-            atomicExch(&hdr->wait_limit_hit, 1u);
-            for (int st = 0; st < kScanStages; ++st)
-                if (in_flight & (1u << st)) {
-                    mbar_wait(&full_bar[st], 0u);
-                    mbar_wait(&full_bar[st], 1u);
-                }
+    if (s_failed && tid == kScanThreads) {
+        atomicExch(&hdr->wait_limit_hit, 1u);
+        for (int st = 0; st < kPipeStages; ++st) {
+            mbar_wait(&full_bar[st], 0u);
+            mbar_wait(&full_bar[st], 1u);
         }
     }
 }
@@ -537,28 +617,28 @@ static int launch_scan(cudaStream_t s, const void *in, int64_t in_stride, void *
                                             carry_t, hdr));
         return B200ALG_OK;
     }
-    const int tiles = (int)ceil_div(n_arg, TILE);
     bool launched = false;
     if (alike) {
+        const int tiles = (int)ceil_div(n_arg, kPipeTileBytes / (int)sizeof(T));
         auto kernel = lead ? scan_pipeline_kernel<T, OP, INCLUSIVE, true> : scan_pipeline_kernel<T, OP, INCLUSIVE, false>;
-        constexpr size_t ring_bytes = (size_t)kScanStages * kScanTileBytes;
+        constexpr size_t ring_bytes = (size_t)kPipeStages * kPipeTileBytes;
         static ContextCache<int> caches[2];  // per kernel instantiation and CUDA context
         ContextCache<int> &cache = caches[lead != 0];
         int blocks_per_sm = 0;
         if (!cache.find(&blocks_per_sm)) {
             B200ALG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ring_bytes));
-            B200ALG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm, kernel, kScanThreads, ring_bytes));
+            B200ALG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm, kernel, kPipeThreads, ring_bytes));
             if (blocks_per_sm < 1) return B200ALG_UNSUPPORTED;
             cache.store(blocks_per_sm);
         }
         // One wave of persistent blocks, launched cooperatively: the driver either makes all of
         // them resident at once (tiles are taken round-robin and wait for one another) or
         // refuses the launch.
-        const int resident = sm_count() * blocks_per_sm;
-        const int blocks = tiles < resident ? tiles : resident;
+        const int resident = sm_count() * blocks_per_sm;  // (two at least, as there are two SMs at least)
+        const int blocks = tiles < resident ? tiles + 1 : resident;  // one of them the scanner
         int lead_arg = lead, tiles_arg = tiles;
         void *args[] = {&in_t, &out_t, &n_arg, &lead_arg, &carry_t, &hdr, &state, &tiles_arg};
-        const cudaError_t e = cudaLaunchCooperativeKernel((const void *)kernel, dim3(blocks), dim3(kScanThreads), args, ring_bytes, s);
+        const cudaError_t e = cudaLaunchCooperativeKernel((const void *)kernel, dim3(blocks), dim3(kPipeThreads), args, ring_bytes, s);
         if (e == cudaSuccess) launched = true;
         else if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported) (void)cudaGetLastError();
         else return cuda_fail(e);
