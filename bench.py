@@ -32,7 +32,7 @@ SEED = 2
 # DRAM traffic of the sort's kernels comes from the ncu summary under profiles/ (written when a
 # capture is taken); it is only quoted while the kernel source is the one that was profiled.
 TRAFFIC_FILE = os.path.join(ROOT, "profiles", "sort_kernel.md")
-KERNEL_SOURCES = [os.path.join(ROOT, "ilgpu_b200", "csrc", f) for f in ("radix_sort.cu", "common.cuh")]
+KERNEL_SOURCES = [os.path.join(ROOT, "ilgpu_b200", "csrc", f) for f in ("radix_sort.cu", "digit_pass.cuh", "sort_common.cuh", "common.cuh")]
 
 
 def kernel_source_digest() -> str:
@@ -540,7 +540,7 @@ def run_native(args) -> None:
 
         def step_fn(i):
             sort(None, bufs[i], temp)
-        launches_per_step = 7   # digit histograms, offsets, 4 digit passes, copy-back (exits at once)
+        launches_per_step = 6   # digit histograms (and offsets), 4 digit passes, copy-back (exits at once)
         result_of = lambda i: bufs[i]
     else:
         from ilgpu_b200.multi_gpu import ShardedAlgorithms
@@ -795,9 +795,9 @@ def run_native(args) -> None:
             "bound": "hbm", "achieved": achieved, "peak": peak_gbs, "unit": "GB/s", "frac": achieved / peak_gbs,
             "traffic": call_traffic if world == 1 else None, "traffic_unit": "bytes per sort call (ncu summary under profiles/, quoted only for the kernel source it was captured from)",
             "peak_kind": peak_kind,
-            "kernel": "whole sort call (digit histograms + 4 onesweep passes); 36 B/key algorithmic",
+            "kernel": "whole sort call (digit histograms + 4 digit passes); 36 B/key algorithmic",
             "dominant_kernel": (None if world != 1 else {
-                "name": "onesweep_kernel (one 8-bit digit pass), 8 B/key algorithmic",
+                "name": "digit_pass_kernel (one 8-bit digit pass), 8 B/key algorithmic",
                 "ms": pass_ms,
                 "achieved": 8 * n / (pass_ms * 1e-3) / 1e9,
                 "frac": 8 * n / (pass_ms * 1e-3) / 1e9 / peak_gbs,
