@@ -1,5 +1,5 @@
-"""The pipelined scan where its blocks have one, two, three and more tiles to go round the ring, and one
-tile more or less than that, for aligned views and views that start off 16 bytes, against numpy."""
+"""The pipelined scan where its blocks have one, three and seven tiles to go round the ring, and one
+element more or less than that, for aligned views and views that start off 16 bytes, against numpy."""
 import numpy as np
 import pytest
 import torch
@@ -11,8 +11,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("name", ["Int32", "Int64", "Float"])
-@pytest.mark.parametrize("turns", [1, 2, 3, 4, 7])
-@pytest.mark.parametrize("extra", [-8192, -1, 0, 1, 8193])
+@pytest.mark.parametrize("turns", [1, 3, 7])
+@pytest.mark.parametrize("extra", [-1, 0, 1])
 @pytest.mark.parametrize("offset", [0, 1])
 def test_turns(accelerator, name, turns, extra, offset):
     blocks = 2 * torch.cuda.get_device_properties(0).multi_processor_count - 1
