@@ -37,9 +37,9 @@ template <typename T> __device__ __forceinline__ T shfl_value_up(T v) {
     if constexpr (sizeof(T) <= 2 && !std::is_same<T, __half>::value) return (T)__shfl_up_sync(0xffffffffu, (unsigned int)v, 1);
     else return shfl_up(v, 1);
 }
-template <typename T> __device__ __forceinline__ T shfl_value_last(T v) {
-    if constexpr (sizeof(T) <= 2 && !std::is_same<T, __half>::value) return (T)__shfl_sync(0xffffffffu, (unsigned int)v, 31);
-    else return shfl_idx(v, 31);
+template <typename T> __device__ __forceinline__ T shfl_value(T v, int from) {
+    if constexpr (sizeof(T) <= 2 && !std::is_same<T, __half>::value) return (T)__shfl_sync(0xffffffffu, (unsigned int)v, from);
+    else return shfl_idx(v, from);
 }
 
 // ---- run-length encoding ------------------------------------------------------------------
@@ -98,7 +98,7 @@ unique_select_kernel(const T *in, int64_t n, T *kept, long long *__restrict__ st
     for (int j = 0; j < NV; ++j) {
         T before = shfl_value_up(v[j].t[VEC - 1]);
         if (lane == 0) before = left;
-        left = shfl_value_last(v[j].t[VEC - 1]);
+        left = shfl_value(v[j].t[VEC - 1], 31);
         unsigned int m = 0u;
 #pragma unroll
         for (int e = 0; e < VEC; ++e) {
@@ -309,6 +309,8 @@ unique_in_place_kernel(T *data, int64_t n, long long *out_count, TempHeader *hdr
     constexpr int NV = kRingVecs;
     constexpr int TILE = VEC * NV * kRingWorkers;
     constexpr int WARPS = kRingWorkers / 32;
+    constexpr int PER = VEC <= 4 ? 4 : 2, BITS = 32 / PER;
+    static_assert(32 * VEC < 1 << BITS && NV % PER == 0, "a warp's count of one vector fits its bits");
     union Vec { uint4 u; T t[VEC]; __device__ Vec() {} };
 
     extern __shared__ __align__(128) unsigned char ring[];  // kRingStages x kRingStageBytes
@@ -423,14 +425,14 @@ unique_in_place_kernel(T *data, int64_t n, long long *out_count, TempHeader *hdr
                         }
                     left = base + warp_first > 0 && warp_first < valid ? data[base + warp_first - 1] : v[0].t[0];
                 }
-                // keep bit e of vector j: element starts a new run.  The counts of two vectors share a word
-                // (16 bits each: a warp holds at most 512 elements of one j).
-                unsigned int packed[NV / 2], incl[NV / 2];
+                // keep bit e of vector j: element starts a new run.  The counts of several vectors share a
+                // word: a warp holds 32 * VEC elements of one j.
+                unsigned int packed[NV / PER], incl[NV / PER];
 #pragma unroll
                 for (int j = 0; j < NV; ++j) {
-                    T in_front = shfl_value_up(v[j].t[VEC - 1]);
-                    if (lane == 0) in_front = left;
-                    left = shfl_value_last(v[j].t[VEC - 1]);
+                    const T around = shfl_value(v[j].t[VEC - 1], (lane + 31) & 31);  // (lane 0: what precedes it in j + 1)
+                    const T in_front = lane == 0 ? left : around;
+                    left = around;
                     unsigned int m = 0u;
 #pragma unroll
                     for (int e = 0; e < VEC; ++e)
@@ -441,27 +443,28 @@ unique_in_place_kernel(T *data, int64_t n, long long *out_count, TempHeader *hdr
                         m &= there <= 0 ? 0u : there < VEC ? (1u << there) - 1u : ~0u;
                     }
                     keep[j] = m;
-                    if (j & 1) packed[j / 2] |= (unsigned int)__popc(m) << 16;
-                    else packed[j / 2] = (unsigned int)__popc(m);
+                    if (j % PER) packed[j / PER] |= (unsigned int)__popc(m) << BITS * (j % PER);
+                    else packed[j / PER] = (unsigned int)__popc(m);
                 }
 #pragma unroll
-                for (int q = 0; q < NV / 2; ++q) incl[q] = packed[q];
+                for (int q = 0; q < NV / PER; ++q) incl[q] = packed[q];
 #pragma unroll
                 for (int d = 1; d < 32; d <<= 1)
 #pragma unroll
-                    for (int q = 0; q < NV / 2; ++q) {
+                    for (int q = 0; q < NV / PER; ++q) {
                         const unsigned int up = __shfl_up_sync(0xffffffffu, incl[q], d);
                         if (lane >= d) incl[q] += up;
                     }
                 unsigned int chunk = 0u;
 #pragma unroll
-                for (int q = 0; q < NV / 2; ++q) {
+                for (int q = 0; q < NV / PER; ++q) {
                     const unsigned int total = __shfl_sync(0xffffffffu, incl[q], 31);
                     const unsigned int excl = incl[q] - packed[q];
-                    local[2 * q] = chunk + (excl & 0xffffu);
-                    chunk += total & 0xffffu;
-                    local[2 * q + 1] = chunk + (excl >> 16);
-                    chunk += total >> 16;
+#pragma unroll
+                    for (int r = 0; r < PER; ++r) {
+                        local[q * PER + r] = chunk + (excl >> BITS * r & ((1u << BITS) - 1u));
+                        chunk += total >> BITS * r & ((1u << BITS) - 1u);
+                    }
                 }
                 if (lane == 31) warp_total[k & 1][warp] = chunk;
             }
