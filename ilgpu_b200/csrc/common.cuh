@@ -9,6 +9,7 @@
 #include <mutex>
 
 #include "../../include/b200alg.h"
+#include "poll_limit.cuh"
 
 namespace b200alg {
 
@@ -97,10 +98,6 @@ struct TempHeader {
     unsigned int reserved[63];
 };
 static_assert(sizeof(TempHeader) == 256, "control block is 256 bytes");
-
-// Upper bound on polls of one look-back slot before a kernel gives up (each poll is an
-// L2 round trip of ~1 us under load, so this is seconds, far beyond any healthy run).
-constexpr unsigned int kMaxSpin = 1u << 22;
 
 // ---- device side ----------------------------------------------------------------------
 #ifdef __CUDACC__

@@ -133,7 +133,7 @@ __device__ __noinline__ void scan_counts(unsigned char *smem, const Pass<K, V, S
     const int row = warp * WARP_ROWS + lane / LANES, octet = lane % LANES, d0 = scanner * kScanDigits + octet * 8;
     const int pairs = (c.num_tiles + 1) / 2;
     Idx carry = tid < kScanDigits ? (Idx)c.gbase[scanner * kScanDigits + tid] : 0;
-    unsigned int spins = 0;
+    ScannerPolls limit;
     for (int pos = 0, turn = 0; pos < pairs; turn ^= 1) {
         const int t = pos + row;
         Words4<unsigned int> a, b;
@@ -158,13 +158,13 @@ __device__ __noinline__ void scan_counts(unsigned char *smem, const Pass<K, V, S
         const int whole = __ffs((int)~__ballot_sync(0xffffffffu, rows == 15u)) - 1;  // warps (of sixteen)
         const int ready = whole * WARP_ROWS + __ffs((int)~__shfl_sync(0xffffffffu, rows, whole)) - 1;
         if (ready == 0) {
-            if (++spins > kMaxSpin) {
+            if (!limit.again(pos > 0, [](unsigned int ns) { __nanosleep(ns); })) {
                 if (tid == 0) atomicExch(&c.hdr->wait_limit_hit, 1u);
                 return;
             }
             continue;
         }
-        spins = 0;
+        limit.progress();
         const bool mine = row < ready, last = lane >= 32 - LANES;
         unsigned int own[4], incl[4];
 #pragma unroll

@@ -206,7 +206,7 @@ static int64_t unique_word_bytes(int64_t tiles) { return padded_tiles(tiles) * (
 __device__ __forceinline__ void scan_tile_counts(const unsigned int *counts, unsigned long long *prefixes, int num_tiles, TempHeader *hdr) {
     const int lane = threadIdx.x & 31;
     unsigned long long carry = 0ull;  // of the tiles before pos
-    unsigned int spins = 0;
+    ScannerPolls limit;
     int pos = 0, done = 0;            // tiles before done have their prefixes
     while (done < num_tiles) {
         const int t = pos + 4 * lane;
@@ -224,13 +224,13 @@ __device__ __forceinline__ void scan_tile_counts(const unsigned int *counts, uns
         const int first = partial ? __ffs((int)partial) - 1 : 32;  // the first lane that misses one
         const int upto = pos + 4 * first + (partial ? __shfl_sync(0xffffffffu, known, first) : 0);
         if (upto <= done) {
-            if (++spins > kMaxSpin) {
+            if (!limit.again(done > 0, [](unsigned int ns) { __nanosleep(ns); })) {
                 if (lane == 0) atomicExch(&hdr->wait_limit_hit, 1u);
                 return;
             }
             continue;
         }
-        spins = 0;
+        limit.progress();
 #pragma unroll
         for (int q = 0; q < 4; ++q) c[q] &= kCounted - 1u;
         const unsigned int own = lane < first ? c[0] + c[1] + c[2] + c[3] : 0u;
