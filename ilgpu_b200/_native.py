@@ -50,6 +50,7 @@ SIGNATURES = {
     "b200alg_sequence": (_int, [_vp, _vp, _i64, _int, _i64, _i64]),
     "b200alg_unique_temp_bytes": (_int, [_int, _i64, ctypes.POINTER(_i64)]),
     "b200alg_unique": (_int, [_vp, _vp, _i64, _int, _vp, _vp, _i64]),
+    "b200alg_unique_to_host": (_int, [_vp, _vp, _i64, _int, _vp, _vp, _i64]),
     "b200alg_run_length_encode_temp_bytes": (_int, [_int, _i64, ctypes.POINTER(_i64)]),
     "b200alg_run_length_encode": (_int, [_vp, _vp, _i64, _int, _vp, _vp, _vp, _vp, _i64]),
     "b200alg_device_status": (_int, [_vp, _vp]),
@@ -82,7 +83,7 @@ _host = None
 _HOST_ENTRY_POINTS = (
     "b200alg_radix_sort_temp_bytes", "b200alg_radix_sort_keys", "b200alg_radix_sort_pairs", "b200alg_radix_sort_pairs_sequence",
     "b200alg_scan_temp_bytes", "b200alg_scan_carry", "b200alg_reduce", "b200alg_reduce_to_host", "b200alg_histogram", "b200alg_initialize",
-    "b200alg_unique_temp_bytes", "b200alg_unique",
+    "b200alg_unique_temp_bytes", "b200alg_unique_to_host",
 )
 
 

@@ -549,10 +549,14 @@ class Accelerator:
         if isinstance(input, torch.Tensor):
             count = self._host.unique(self._index, _TORCH_TO_CODE.get(input.dtype, -1), stream, input)
             if count is not None:
+                if count < 0:
+                    B200AlgException.ThrowIfFailed(-count)
                 return count
         output = self.Allocate1D(1, torch.int64)
         temp = self.Allocate1D(self.ComputeUniqueTempStorageSize(input.dtype, input.numel()), torch.int32)
         self.CreateUnique(input.dtype)(stream, input, output, temp)
+        if input.numel() > 0:  # (an empty view leaves temp as it is)
+            self.CheckDeviceStatus(stream, temp)
         return int(output.cpu()[0])
 
     # -- edges of the path --

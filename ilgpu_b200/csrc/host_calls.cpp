@@ -35,7 +35,7 @@ struct Library {
     decltype(&b200alg_histogram) histogram;
     decltype(&b200alg_initialize) initialize;
     decltype(&b200alg_unique_temp_bytes) unique_temp_bytes;
-    decltype(&b200alg_unique) unique;
+    decltype(&b200alg_unique_to_host) unique_to_host;
 } lib;
 
 constexpr int64_t kMaxLength = (1ll << 31) - 1;  // the reference's int.MaxValue
@@ -282,7 +282,9 @@ PyObject *histogram(PyObject *, PyObject *const *a, Py_ssize_t count) {
     });
 }
 
-// unique(device, code, stream, data): the new length, once the GPU has it; None: not covered
+// unique(device, code, stream, data): the new length, once the GPU has it; a status other than success
+// that the GPU reports, as a negative number (the data has changed, the call cannot be made again);
+// None: not covered
 PyObject *unique(PyObject *, PyObject *const *a, Py_ssize_t count) {
     PyObject *value = nullptr;
     PyObject *ok = guarded([&] {
@@ -293,18 +295,19 @@ PyObject *unique(PyObject *, PyObject *const *a, Py_ssize_t count) {
         int64_t need = 0;
         if (device < 0 || !view_of(a[3], device, code, data) || data.stride != 1 || !stream_of(a[2], device, stream)) return false;
         if (lib.unique_temp_bytes(code, data.n, &need) != B200ALG_OK) return false;
-        void *slot = host_slot.get();
+        int64_t *slot = (int64_t *)host_slot.get();
         if (!slot || data.n < 1) return false;
+        slot[1] = B200ALG_OK;
         const at::Tensor temp = at::empty({need}, at::TensorOptions().dtype(at::kByte).device(at::kCUDA, device));
         void *t = temp.data_ptr();
-        // the kernel stores the count straight into the host slot
+        // the kernel stores the count, and a wait that ran out, straight into the host slot
         const int status = released([&]() -> int {
-            const int rc = lib.unique(stream, data.data, data.n, code, slot, t, need);
+            const int rc = lib.unique_to_host(stream, data.data, data.n, code, slot, t, need);
             if (rc != B200ALG_OK) return rc;
             return cudaStreamSynchronize((cudaStream_t)stream) == cudaSuccess ? B200ALG_OK : B200ALG_CUDA_ERROR;
         });
         if (status != B200ALG_OK) return false;
-        value = number_of(slot, B200ALG_I64);
+        value = PyLong_FromLongLong(slot[1] == B200ALG_OK ? slot[0] : -slot[1]);
         return value != nullptr;
     });
     if (ok != Py_True) {

@@ -201,9 +201,17 @@ constexpr unsigned int kCounted = 0x80000000u;  // beside a tile's count of surv
 static __host__ __device__ int64_t padded_tiles(int64_t tiles) { return (tiles + 3) / 4 * 4; }
 static int64_t unique_word_bytes(int64_t tiles) { return padded_tiles(tiles) * (4 + 8); }
 
+// A wait ran out: noted in the control block and, for a caller that reads the result from host memory,
+// beside it.
+__device__ __forceinline__ void report_wait_limit(TempHeader *hdr, long long *host_status) {
+    atomicExch(&hdr->wait_limit_hit, 1u);
+    if (host_status) *host_status = B200ALG_WAIT_LIMIT;
+}
+
 // One warp turns the tiles' counts into their prefixes (published as 2 * prefix + 1), four neighbouring
 // tiles per lane.
-__device__ __forceinline__ void scan_tile_counts(const unsigned int *counts, unsigned long long *prefixes, int num_tiles, TempHeader *hdr) {
+__device__ __forceinline__ void scan_tile_counts(const unsigned int *counts, unsigned long long *prefixes, int num_tiles, TempHeader *hdr,
+                                                 long long *host_status) {
     const int lane = threadIdx.x & 31;
     unsigned long long carry = 0ull;  // of the tiles before pos
     ScannerPolls limit;
@@ -225,7 +233,7 @@ __device__ __forceinline__ void scan_tile_counts(const unsigned int *counts, uns
         const int upto = pos + 4 * first + (partial ? __shfl_sync(0xffffffffu, known, first) : 0);
         if (upto <= done) {
             if (!limit.again(done > 0, [](unsigned int ns) { __nanosleep(ns); })) {
-                if (lane == 0) atomicExch(&hdr->wait_limit_hit, 1u);
+                if (lane == 0) report_wait_limit(hdr, host_status);
                 return;
             }
             continue;
@@ -304,7 +312,7 @@ template <typename T> __device__ __forceinline__ void put_if(unsigned int keep, 
 
 template <typename T>
 __global__ void __launch_bounds__(kRingThreads, kRingBlocks)
-unique_in_place_kernel(T *data, int64_t n, long long *out_count, TempHeader *hdr, unsigned int *counts, int num_tiles) {
+unique_in_place_kernel(T *data, int64_t n, long long *out_count, long long *host_status, TempHeader *hdr, unsigned int *counts, int num_tiles) {
     constexpr int VEC = 16 / (int)sizeof(T);
     constexpr int NV = kRingVecs;
     constexpr int TILE = VEC * NV * kRingWorkers;
@@ -355,7 +363,7 @@ unique_in_place_kernel(T *data, int64_t n, long long *out_count, TempHeader *hdr
     }
     __syncthreads();
     if (s_role == 0) {
-        if (warp == 0) scan_tile_counts(counts, prefixes, num_tiles, hdr);
+        if (warp == 0) scan_tile_counts(counts, prefixes, num_tiles, hdr, host_status);
         return;
     }
     unsigned int max_polls = kMaxBarrierPolls;  // a thread whose wait ran out does not wait as long again
@@ -507,7 +515,7 @@ unique_in_place_kernel(T *data, int64_t n, long long *out_count, TempHeader *hdr
     // wait so that the block does not retire underneath them.
     __syncthreads();
     if (s_failed && tid == kRingWorkers) {
-        atomicExch(&hdr->wait_limit_hit, 1u);
+        report_wait_limit(hdr, host_status);
         for (int st = 0; st < kRingStages; ++st) {
             mbar_wait(&full_bar[st], 0u);
             mbar_wait(&full_bar[st], 1u);
@@ -537,7 +545,7 @@ static UniqueLayout unique_layout(int elem_bytes, int64_t n) {
 }
 
 template <typename T>
-static int run_unique(cudaStream_t s, void *data, int64_t n, void *out_count, void *temp, const UniqueLayout &L) {
+static int run_unique(cudaStream_t s, void *data, int64_t n, void *out_count, long long *host_status, void *temp, const UniqueLayout &L) {
     char *t = (char *)temp;
     auto kernel = unique_in_place_kernel<T>;
     constexpr int ring_bytes = kRingStages * kRingStageBytes;
@@ -550,7 +558,8 @@ static int run_unique(cudaStream_t s, void *data, int64_t n, void *out_count, vo
     const int64_t most = (int64_t)kRingBlocks * sm_count();
     const int blocks = (int)(L.tiles < most ? L.tiles + 1 : most);  // one of them the scanner
     B200ALG_CUDA_TRY(cudaMemsetAsync(temp, 0, (size_t)(L.off_state + unique_word_bytes(L.tiles)), s));
-    kernel<<<blocks, kRingThreads, ring_bytes, s>>>((T *)data, n, (long long *)out_count, (TempHeader *)temp, (unsigned int *)(t + L.off_state), (int)L.tiles);
+    kernel<<<blocks, kRingThreads, ring_bytes, s>>>((T *)data, n, (long long *)out_count, host_status, (TempHeader *)temp, (unsigned int *)(t + L.off_state),
+                                                (int)L.tiles);
     B200ALG_LAUNCH_CHECK();
     return B200ALG_OK;
 }
@@ -636,7 +645,7 @@ extern "C" int b200alg_unique_temp_bytes(int dtype, int64_t n, int64_t *out_byte
     return B200ALG_OK;
 }
 
-extern "C" int b200alg_unique(void *stream, void *data, int64_t n, int dtype, void *out_count, void *temp, int64_t temp_bytes) {
+static int unique(void *stream, void *data, int64_t n, int dtype, void *out_count, long long *host_status, void *temp, int64_t temp_bytes) {
     // Argument checks mirror CreateUnique's (UniqueExtensions.cs:150-172).
     if (!out_count || n < 0) return B200ALG_INVALID_ARGUMENT;
     if ((uintptr_t)out_count % 8) return B200ALG_MISALIGNED;
@@ -653,13 +662,21 @@ extern "C" int b200alg_unique(void *stream, void *data, int64_t n, int dtype, vo
     if (temp_bytes < L.total) return B200ALG_TEMP_TOO_SMALL;
     cudaStream_t s = (cudaStream_t)stream;
     switch (dtype) {
-    case B200ALG_I8: case B200ALG_U8: return run_unique<uint8_t>(s, data, n, out_count, temp, L);
-    case B200ALG_I16: case B200ALG_U16: return run_unique<uint16_t>(s, data, n, out_count, temp, L);
-    case B200ALG_I32: case B200ALG_U32: return run_unique<uint32_t>(s, data, n, out_count, temp, L);
-    case B200ALG_I64: case B200ALG_U64: return run_unique<uint64_t>(s, data, n, out_count, temp, L);
-    case B200ALG_F16: return run_unique<__half>(s, data, n, out_count, temp, L);
-    case B200ALG_F32: return run_unique<float>(s, data, n, out_count, temp, L);
-    case B200ALG_F64: return run_unique<double>(s, data, n, out_count, temp, L);
+    case B200ALG_I8: case B200ALG_U8: return run_unique<uint8_t>(s, data, n, out_count, host_status, temp, L);
+    case B200ALG_I16: case B200ALG_U16: return run_unique<uint16_t>(s, data, n, out_count, host_status, temp, L);
+    case B200ALG_I32: case B200ALG_U32: return run_unique<uint32_t>(s, data, n, out_count, host_status, temp, L);
+    case B200ALG_I64: case B200ALG_U64: return run_unique<uint64_t>(s, data, n, out_count, host_status, temp, L);
+    case B200ALG_F16: return run_unique<__half>(s, data, n, out_count, host_status, temp, L);
+    case B200ALG_F32: return run_unique<float>(s, data, n, out_count, host_status, temp, L);
+    case B200ALG_F64: return run_unique<double>(s, data, n, out_count, host_status, temp, L);
     }
     return B200ALG_UNSUPPORTED;
+}
+
+extern "C" int b200alg_unique(void *stream, void *data, int64_t n, int dtype, void *out_count, void *temp, int64_t temp_bytes) {
+    return unique(stream, data, n, dtype, out_count, nullptr, temp, temp_bytes);
+}
+
+extern "C" int b200alg_unique_to_host(void *stream, void *data, int64_t n, int dtype, int64_t *host_out, void *temp, int64_t temp_bytes) {
+    return unique(stream, data, n, dtype, host_out, host_out ? (long long *)host_out + 1 : nullptr, temp, temp_bytes);
 }

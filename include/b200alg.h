@@ -220,6 +220,12 @@ int b200alg_sequence(void *stream, void *view, int64_t n, int dtype, int64_t sta
  * int because its kernel is a serial chain of groups). */
 int b200alg_unique_temp_bytes(int dtype, int64_t n, int64_t *out_bytes);
 int b200alg_unique(void *stream, void *data, int64_t n, int dtype, void *out_count, void *temp, int64_t temp_bytes);
+/* The same with the new length in host memory (UniqueExtensions.cs:200-220 copies it there), and
+ * beside it what b200alg_device_status would say of temp: host_out is 16 bytes of pinned, mapped
+ * memory of the caller.  Once the stream has got there, host_out[0] holds the length, and
+ * host_out[1], which the caller has set to 0, is B200ALG_WAIT_LIMIT if a bounded wait ran out (the
+ * data and the length are then not valid). */
+int b200alg_unique_to_host(void *stream, void *data, int64_t n, int dtype, int64_t *host_out, void *temp, int64_t temp_bytes);
 
 /* Run-length encoding: the step after a sort when the counts per key are wanted (sort ->
  * unique -> counts).  values[r] = the element that starts run r of data[0..n), lengths[r]
