@@ -198,6 +198,7 @@ unique_select_kernel(const T *in, int64_t n, T *kept, long long *__restrict__ st
 // ---- in place -------------------------------------------------------------------------------
 // The words the tiles and the scanner exchange.
 constexpr unsigned int kCounted = 0x80000000u;  // beside a tile's count of survivors
+constexpr unsigned int kRead = 0x40000000u;     // likewise, set with release: the tile may be overwritten
 static __host__ __device__ int64_t padded_tiles(int64_t tiles) { return (tiles + 3) / 4 * 4; }
 static int64_t unique_word_bytes(int64_t tiles) { return padded_tiles(tiles) * (4 + 8); }
 
@@ -240,7 +241,7 @@ __device__ __forceinline__ void scan_tile_counts(const unsigned int *counts, uns
         }
         limit.progress();
 #pragma unroll
-        for (int q = 0; q < 4; ++q) c[q] &= kCounted - 1u;
+        for (int q = 0; q < 4; ++q) c[q] &= kRead - 1u;
         const unsigned int own = lane < first ? c[0] + c[1] + c[2] + c[3] : 0u;
         unsigned int incl = own;
 #pragma unroll
@@ -264,14 +265,22 @@ __device__ __forceinline__ void scan_tile_counts(const unsigned int *counts, uns
 // hand their tiles' counts to a scanner warp (the first block to start) and do the next tile until
 // the prefix has come; a tile waits in a ring in shared memory, where its survivors gather in the
 // place its elements came to.  Tiles of 32 KB, three to a block, two blocks per SM: 5 * 10^7 uint32 of
-// which a quarter is kept take 62 us (look-back in every block, one tile per block: 74 us); 2^27 of
-// which one in fifty is kept 132 (157) us.
+// which a quarter is kept take 65 us (look-back in every block, one tile per block: 74 us); 2^27 of
+// which one in fifty is kept 136 (157) us.
 //
-// The result goes over the input: a tile stores only once its prefix is known, hence after it and
-// every earlier tile have been read (a copy that is ahead reads only elements that tiles at or behind it
-// may overwrite), and it stores at or below its own elements' places.  The one element a tile reads
-// outside its own range is the last one of the tile before; only that element itself (unmoved) is stored
-// there before this tile has published.
+// The result goes over the input: a tile's survivors are stored at or below its own elements' places,
+// over elements of at most two earlier tiles.  Those have been counted, hence read, long before the
+// prefix is known, but that chain of relaxed words orders nothing.  So a block says of each of its
+// tiles that it has been read (kRead beside the count, with release, after the barrier behind the
+// reads), and two lanes of the warp that fetches a prefix look for that word of the two tiles (with
+// acquire) before the block stores.  That is a trip to L2 more per tile; without it the two sizes above
+// take 62.5 and 130 us.  (Release by the counting thread and fences in the scanner: 85 and 194 us;
+// release by the counting thread and acquire by the fetching lanes: 77 and 167 us; looking for the words
+// while the prefix is on its way, in 128 tiles at a time: 66 and 139 us.)
+//
+// The one element a tile reads outside its own range is the last one of the tile before.  A tile of
+// which nothing moves is not stored at all, so that element is written only by tiles that have waited
+// for its second reader, too: the second of the two tiles above.
 constexpr int kRingStages = 3;
 constexpr int kRingWorkers = 256, kRingVecs = 8;  // 512 threads of four vectors: 71 us
 static_assert(kRingWorkers * kRingVecs * 16 == kUniqueTileBytes, "one size of tile");
@@ -323,6 +332,7 @@ unique_in_place_kernel(T *data, int64_t n, long long *out_count, long long *host
 
     extern __shared__ __align__(128) unsigned char ring[];  // kRingStages x kRingStageBytes
     __shared__ __align__(8) unsigned long long full_bar[kRingStages];  // the tile's number is known, its elements have arrived
+    __shared__ __align__(8) unsigned long long read_bar[kRingStages];  // the tile is in registers, its count is on its way
     __shared__ __align__(8) unsigned long long free_bar[kRingStages];  // every warp has stored its part of the survivors
     __shared__ __align__(8) unsigned long long base_bar[2];            // the tile's prefix is known
     __shared__ unsigned long long s_prefix[2];
@@ -354,6 +364,7 @@ unique_in_place_kernel(T *data, int64_t n, long long *out_count, long long *host
         s_role = (int)atomicAdd(&hdr->reserved[1], 1u);
         for (int st = 0; st < kRingStages; ++st) {
             mbar_init(&full_bar[st], 1u);
+            mbar_init(&read_bar[st], 1u);
             mbar_init(&free_bar[st], WARPS);
         }
         for (int h = 0; h < 2; ++h) mbar_init(&base_bar[h], 1u);
@@ -374,31 +385,46 @@ unique_in_place_kernel(T *data, int64_t n, long long *out_count, long long *host
         return false;
     };
 
-    if (warp == WARPS) {  // keeps tiles coming
-        if (lane == 0)
-            for (int k = at_once; more; ++k) {
-                if (!(k < kRingStages ? wait(&full_bar[0], 0u) : wait(&free_bar[k % kRingStages], (unsigned int)(k / kRingStages - 1) & 1u))) break;
-                more = take_tile(k);
+    if (warp == WARPS) {  // keeps tiles coming, and tells the other blocks when they have been read
+        if (lane == 0) {
+            bool well = true;
+            for (int k = at_once; k < kRingStages && more && well; ++k)
+                if ((well = wait(&full_bar[0], 0u))) more = take_tile(k);
+            for (int k = 0; well && tile_of[k % kRingStages] < num_tiles; ++k) {
+                if (!wait(&read_bar[k % kRingStages], (unsigned int)(k / kRingStages) & 1u)) break;
+                asm volatile("red.release.gpu.global.or.b32 [%0], %1;" ::"l"(counts + tile_of[k % kRingStages]), "r"(kRead) : "memory");
+                if (k > 0 && more) {  // the tile before is stored next
+                    if (!wait(&free_bar[(k - 1) % kRingStages], (unsigned int)((k - 1) / kRingStages) & 1u)) break;
+                    more = take_tile(k - 1 + kRingStages);
+                }
             }
+        }
         __syncwarp();
     } else if (warp > WARPS) {  // fetches their prefixes
-        if (lane == 0) {
+        if (lane < 2) {
             unsigned int max_spins = kMaxSpin;
             for (int k = 0;; ++k) {
-                if (!wait(&full_bar[k % kRingStages], (unsigned int)(k / kRingStages) & 1u)) break;
+                const bool arrived = wait(&full_bar[k % kRingStages], (unsigned int)(k / kRingStages) & 1u);
+                if (__any_sync(3u, !arrived)) break;
                 const int tile = tile_of[k % kRingStages];
                 if (tile >= num_tiles) break;
                 unsigned long long word = 1ull;
                 unsigned int spins = 0;
-                while (tile > 0 && ((word = ld_relaxed_u64(prefixes + tile)) & 1ull) == 0) {
-                    if (++spins > max_spins) {
-                        s_failed = 1;
-                        max_spins = 1u;
-                        break;
-                    }
+                auto again = [&]() {
+                    if (++spins <= max_spins) return true;
+                    s_failed = 1;
+                    max_spins = 1u;
+                    return false;
+                };
+                while (tile > 0 && ((word = ld_relaxed_u64(prefixes + tile)) & 1ull) == 0 && again()) {}
+                // the first of the tiles that the survivors go over, and the one behind it, have been read
+                const int64_t over = (int64_t)(word >> 1) / TILE + lane;
+                while (over < tile && (ld_acquire_u32(counts + over) & kRead) == 0 && again()) {}
+                __syncwarp(3u);
+                if (lane == 0) {
+                    s_prefix[k & 1] = word >> 1;
+                    mbar_arrive(&base_bar[k & 1]);
                 }
-                s_prefix[k & 1] = word >> 1;
-                mbar_arrive(&base_bar[k & 1]);
             }
         }
         __syncwarp();
@@ -483,7 +509,10 @@ unique_in_place_kernel(T *data, int64_t n, long long *out_count, long long *host
                 const unsigned int wt = lane < WARPS ? warp_total[k & 1][lane] : 0u;
                 const unsigned int first_slot = __reduce_add_sync(0xffffffffu, lane < warp ? wt : 0u);
                 count = __reduce_add_sync(0xffffffffu, wt);
-                if (tid == 0) st_relaxed_u32(counts + tile, count | kCounted);
+                if (tid == 0) {
+                    st_relaxed_u32(counts + tile, count | kCounted);
+                    mbar_arrive(&read_bar[st]);
+                }
 #pragma unroll
                 for (int j = 0; j < NV; ++j) {
                     unsigned int at = smem_addr(stage) + (first_slot + local[j]) * (unsigned int)sizeof(T);
@@ -498,8 +527,9 @@ unique_in_place_kernel(T *data, int64_t n, long long *out_count, long long *host
                     if (before == num_tiles - 1 && tid == 0) *out_count = prefix + before_count;
                     const T *survivors = reinterpret_cast<const T *>(stage_of(q));
                     T *to = data + prefix;
+                    const unsigned int stored = prefix + before_count == (int64_t)(before + 1) * TILE ? 0u : before_count;  // 0: nothing has moved
 #pragma unroll 4
-                    for (unsigned int i = tid; i < before_count; i += kRingWorkers) to[i] = survivors[i];
+                    for (unsigned int i = tid; i < stored; i += kRingWorkers) to[i] = survivors[i];
                 }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // a copy may come into these places next
                 __syncwarp();
