@@ -432,15 +432,24 @@ resident_sort_kernel(SortBuffers<K, V> io, KeyXform<K> xf, TempHeader *hdr, unsi
 }
 
 // ---- host side ---------------------------------------------------------------------------
-// Which blocks (times for uint32 keys and uint32 pairs, on the GPU, with the launch):
-//   one       up to 8 keys per thread (5000 keys: 19 us against 21 us with a cluster, 8000 pairs: 33 us
-//             against 23 us);
-//   cluster   up to 40960 elements (40000: 26 / 32 us against 29 / 32 us with a grid; 60000: 34 / 44 us
-//             against 30 / 32 us);
-//   grid      about 64 blocks until they have 4 keys per thread, then more, up to the length from which
-//             the passes over tiles are as fast (2^20 keys: 60 us; 800000 pairs or 8-byte keys: 65 /
-//             107 us).
-constexpr int64_t kAloneMost = kResidentThreads * 8;
+// Which blocks (times on the GPU, with the launch):
+//   one       up to 8 elements per thread, 12 of keys alone with 4 or 8 bytes.  One block against a
+//             cluster, us, by key bytes / value bytes:
+//                          4500          5000          6144          6700          8192
+//                1 / 0   10.3   8.3   10.2  10.1   10.2   8.3   10.4   8.4   12.3  10.2
+//                2 / 0   12.3  12.3   12.3  12.4   14.3  12.3   14.4  12.4   16.4  12.3
+//                4 / 0   16.4  20.5   18.3  20.5   18.4  20.5   20.5  20.5   22.6  18.5
+//                8 / 0   30.7  34.8   30.9  34.8   34.8  36.8   38.9  35.0   43.1  32.9
+//                4 / 4   20.5  22.5   22.5  22.6   24.6  22.5   26.7  22.5   28.7  22.6
+//                8 / 4   36.9  39.0   39.0  41.0   45.1  41.0   51.2  41.0   55.3  38.9
+//                8 / 8   39.0  39.1   43.0  41.0   49.1  41.0   53.2  41.0   59.4  39.1
+//   cluster   up to 40960 elements (uint32 keys / pairs: 40000: 27 / 33 us against 29 / 32 us with a
+//             grid; 60000: 35 / 43 us against 29 / 33 us);
+//   grid      about 64 blocks until they have 4 keys per thread, then more, up to about the length from
+//             which the passes over tiles are as fast (against those: 700000 uint32 keys / pairs / 8-byte
+//             keys 51 / 61 / 104 us against 59 / 64 / 99; 2^20 uint32 keys 59 against 61 us; 800000 pairs
+//             62 against 59 us).
+constexpr int64_t alone_most(int key_bytes, int value_bytes) { return kResidentThreads * (value_bytes == 0 && key_bytes >= 4 ? 12 : 8); }
 constexpr int64_t kClusterMost = 5 * kMaxCluster * kResidentThreads;
 constexpr int64_t kGridMostNarrow = 1 << 20, kGridMost = 3 << 18;
 
@@ -485,7 +494,7 @@ static int run_resident(cudaStream_t s, const SortCall &call, uint64_t xn, uint6
     *taken = false;
     const int64_t n = call.n;
     int meeting, blocks;
-    if (n <= kAloneMost && n <= kResidentThreads * ITEMS) {
+    if (n <= alone_most(sizeof(K), VB) && n <= kResidentThreads * ITEMS) {
         meeting = kAlone;
         blocks = 1;
     } else if (n <= kClusterMost && n <= (int64_t)lim.cluster * kResidentThreads * CLUSTER_ITEMS) {

@@ -13,7 +13,7 @@ from tests.helpers import NP
 
 pytestmark = pytest.mark.gpu
 
-LENGTHS = [1, 2, 511, 513, 4095, 4096, 4097, 8193, 16_385, 40_960, 40_961, 65_537, 131_073, 300_001]
+LENGTHS = [1, 2, 511, 513, 4095, 4096, 4097, 6143, 6144, 6145, 8193, 16_385, 40_960, 40_961, 65_537, 131_073, 300_001]
 
 
 def _keys(rng, dtype, n, kind):
