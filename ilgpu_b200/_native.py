@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import warnings
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 # B200ALG_LIBRARY overrides the path of the shared library (e.g. a differently tuned build).
@@ -79,13 +80,6 @@ _lib = None
 _mg_lib = None
 _host = None
 
-# what csrc/host_calls.cpp calls, in the order of its table
-_HOST_ENTRY_POINTS = (
-    "b200alg_radix_sort_temp_bytes", "b200alg_radix_sort_keys", "b200alg_radix_sort_pairs", "b200alg_radix_sort_pairs_sequence",
-    "b200alg_scan_temp_bytes", "b200alg_scan_carry", "b200alg_reduce", "b200alg_reduce_to_host", "b200alg_histogram", "b200alg_initialize",
-    "b200alg_unique_temp_bytes", "b200alg_unique_to_host",
-)
-
 
 class NativeLibraryMissing(RuntimeError):
     pass
@@ -125,16 +119,27 @@ def lib() -> ctypes.CDLL:
     return _lib
 
 
+class _NoHostPath:
+    """Covers no call: every one goes through the Python code of algorithms.py."""
+
+    def __getattr__(self, name):
+        return lambda *arguments: None
+
+
 def host():
-    """The native host path of the mirror's calls (csrc/host_calls.cpp), bound to lib()."""
+    """The native host path of the mirror's calls (csrc/host_calls.cpp), bound to lib().  It saves host time
+    only: without it (not built, or built against another torch or another state of the library) the
+    calls take their way through algorithms.py into the same kernels, and one warning says so."""
     global _host
     if _host is None:
         L = lib()
         try:
             from . import _host as module
-        except ImportError as e:
-            raise NativeLibraryMissing(f"ilgpu_b200/_host.so: {e}; build it with `make -C ilgpu_b200/csrc`") from e
-        module.bind(tuple(ctypes.cast(getattr(L, name), ctypes.c_void_p).value for name in _HOST_ENTRY_POINTS))
+            module.bind(tuple(ctypes.cast(getattr(L, name), ctypes.c_void_p).value for name in module.ENTRY_POINTS))
+        except (ImportError, AttributeError, ValueError) as e:
+            warnings.warn(f"ilgpu_b200/_host.so: {e}; small calls cost more host time without it "
+                          "(build it with `make -C ilgpu_b200/csrc host`)", RuntimeWarning)
+            module = _NoHostPath()
         _host = module
     return _host
 

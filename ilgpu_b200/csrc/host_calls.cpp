@@ -22,21 +22,27 @@
 
 namespace {
 
-// Entry points of the library that the package has loaded (addresses handed over by bind()).
+// Entry points of the library that the package has loaded (addresses handed over by bind(), in the
+// order of ENTRY_POINTS).
+#define B200ALG_ENTRY_POINTS(X) \
+    X(radix_sort_temp_bytes) \
+    X(radix_sort_keys) \
+    X(radix_sort_pairs) \
+    X(radix_sort_pairs_sequence) \
+    X(scan_temp_bytes) \
+    X(scan_carry) \
+    X(reduce) \
+    X(reduce_to_host) \
+    X(histogram) \
+    X(initialize) \
+    X(unique_temp_bytes) \
+    X(unique_to_host)
 struct Library {
-    decltype(&b200alg_radix_sort_temp_bytes) radix_sort_temp_bytes;
-    decltype(&b200alg_radix_sort_keys) radix_sort_keys;
-    decltype(&b200alg_radix_sort_pairs) radix_sort_pairs;
-    decltype(&b200alg_radix_sort_pairs_sequence) radix_sort_pairs_sequence;
-    decltype(&b200alg_scan_temp_bytes) scan_temp_bytes;
-    decltype(&b200alg_scan_carry) scan_carry;
-    decltype(&b200alg_reduce) reduce;
-    decltype(&b200alg_reduce_to_host) reduce_to_host;
-    decltype(&b200alg_histogram) histogram;
-    decltype(&b200alg_initialize) initialize;
-    decltype(&b200alg_unique_temp_bytes) unique_temp_bytes;
-    decltype(&b200alg_unique_to_host) unique_to_host;
+#define B200ALG_MEMBER(name) decltype(&b200alg_##name) name;
+    B200ALG_ENTRY_POINTS(B200ALG_MEMBER)
 } lib;
+#define B200ALG_NAME(name) "b200alg_" #name,
+constexpr const char *kEntryPoints[] = {B200ALG_ENTRY_POINTS(B200ALG_NAME)};
 
 constexpr int64_t kMaxLength = (1ll << 31) - 1;  // the reference's int.MaxValue
 
@@ -347,7 +353,7 @@ PyObject *initialize(PyObject *, PyObject *const *a, Py_ssize_t count) {
     });
 }
 
-// bind(addresses): one address per member of Library, in its order
+// bind(addresses): one address per name in ENTRY_POINTS
 PyObject *bind(PyObject *, PyObject *addresses) {
     constexpr Py_ssize_t kCount = sizeof(Library) / sizeof(void *);
     void *p[kCount];
@@ -368,4 +374,19 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", "Host path of the algorith
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__host(void) { return PyModule_Create(&module); }
+PyMODINIT_FUNC PyInit__host(void) {
+    PyObject *m = PyModule_Create(&module);
+    constexpr Py_ssize_t kCount = sizeof(kEntryPoints) / sizeof(kEntryPoints[0]);
+    PyObject *names = m ? PyTuple_New(kCount) : nullptr;
+    for (Py_ssize_t i = 0; names && i < kCount; ++i) {
+        PyObject *name = PyUnicode_FromString(kEntryPoints[i]);
+        if (!name) Py_CLEAR(names);
+        else PyTuple_SET_ITEM(names, i, name);
+    }
+    if (!names || PyModule_AddObject(m, "ENTRY_POINTS", names) < 0) {
+        Py_XDECREF(names);
+        Py_XDECREF(m);
+        return nullptr;
+    }
+    return m;
+}

@@ -40,6 +40,30 @@ def test_multi_gpu_library_exports_what_its_header_declares():
     assert lib.b200alg_comm_status(None, None) == _native.INVALID_ARGUMENT
 
 
+def test_host_path_is_optional(monkeypatch):
+    """Bound when it fits the library; left out, with a warning, when it is missing or of another state."""
+    import sys
+    import types
+    import warnings
+
+    import pytest
+    names = _native.host().ENTRY_POINTS
+    assert set(names) <= set(_declared())
+    stale = types.ModuleType("ilgpu_b200._host")           # no list of what it calls
+    other = types.ModuleType("ilgpu_b200._host")
+    other.ENTRY_POINTS, other.bind = ("b200alg_not_there",), None
+    for module in (None, stale, other):                    # None: the import fails
+        monkeypatch.setattr(_native, "_host", None)
+        monkeypatch.delattr(sys.modules["ilgpu_b200"], "_host", raising=False)
+        monkeypatch.setitem(sys.modules, "ilgpu_b200._host", module)
+        with pytest.warns(RuntimeWarning, match="_host.so"):
+            path = _native.host()
+        assert all(not getattr(path, call)(1, 2, 3) for call in ("sort_keys", "reduce_value", "unique"))
+        with warnings.catch_warnings():                    # said once
+            warnings.simplefilter("error")
+            assert _native.host() is path
+
+
 def test_host_only_entry_points():
     L = _native.lib()
     assert L.b200alg_version() == 100

@@ -15,9 +15,10 @@ UNIQUE_TO_HOST = ctypes.CFUNCTYPE(ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p
 
 
 def _bind(replaced=None):
-    addresses = [ctypes.cast(getattr(N.lib(), name), ctypes.c_void_p).value for name in N._HOST_ENTRY_POINTS]
+    names = N.host().ENTRY_POINTS
+    addresses = [ctypes.cast(getattr(N.lib(), name), ctypes.c_void_p).value for name in names]
     if replaced is not None:
-        addresses[N._HOST_ENTRY_POINTS.index("b200alg_unique_to_host")] = ctypes.cast(replaced, ctypes.c_void_p).value
+        addresses[names.index("b200alg_unique_to_host")] = ctypes.cast(replaced, ctypes.c_void_p).value
     N.host().bind(tuple(addresses))
 
 
