@@ -285,6 +285,10 @@ class Accelerator:
     def Synchronize(self) -> None:
         torch.cuda.synchronize(self.device)
 
+    def _wait(self, stream) -> None:
+        """Until the stream of a call is through: the copy of its result need not run there."""
+        (torch.cuda.current_stream(self.device) if stream is None else stream).synchronize()
+
     def Bind(self):
         """Makes this accelerator's device current (CudaAccelerator.cs:422-424)."""
         return torch.cuda.device(self.device)
@@ -472,6 +476,7 @@ class Accelerator:
             return None
         out = self.Allocate1D(1, operation.dtype)
         reduce(stream, input, out)
+        self._wait(stream)
         return out.cpu()[0].item()
 
     # -- histogram --
@@ -557,6 +562,8 @@ class Accelerator:
         self.CreateUnique(input.dtype)(stream, input, output, temp)
         if input.numel() > 0:  # (an empty view leaves temp as it is)
             self.CheckDeviceStatus(stream, temp)
+        else:
+            self._wait(stream)
         return int(output.cpu()[0])
 
     # -- edges of the path --

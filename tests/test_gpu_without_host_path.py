@@ -57,3 +57,22 @@ def test_every_call(plain, n):
     ordered = torch.from_numpy(host[order]).cuda()
     count = plain.Unique(None, ordered)
     np.testing.assert_array_equal(ordered[:count].cpu().numpy(), np.unique(host))
+
+
+def test_values_that_come_back_wait_for_their_stream(plain):
+    data = torch.arange(100_001, dtype=torch.int64, device="cuda")
+    add, side = ib.ScanReduceOperations.AddInt64, torch.cuda.Stream()
+    torch.cuda.synchronize()
+    for _ in range(3):
+        marker = torch.full((1,), -1, dtype=torch.int64, device="cuda")   # what the result's memory holds before
+        del marker
+        torch.cuda.synchronize()
+        with torch.cuda.stream(side):
+            torch.cuda._sleep(20_000_000)   # some 10 ms in front of the call
+        assert plain.Reduce(side, data, add) == 100_000 * 100_001 // 2
+        with torch.cuda.stream(side):
+            torch.cuda._sleep(20_000_000)
+        assert plain.Unique(side, data) == 100_001
+        with torch.cuda.stream(side):
+            torch.cuda._sleep(20_000_000)
+        assert plain.Unique(side, data[:0]) == 0
