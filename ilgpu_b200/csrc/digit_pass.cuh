@@ -226,33 +226,12 @@ __device__ __forceinline__ void take_tile(PassMisc<K, V, SW> &m, unsigned char *
     }
 }
 
-// Puts the slots of a tile in order: neighbours that are the wrong way round change places until none
-// are.  Reached only when the atomics of a warp were not served in lane order.
+// Puts the slots of a tile in order.  Reached only when the atomics of a warp were not served in lane
+// order.
 template <typename K, typename V, typename XF, typename L>
 __device__ __noinline__ void repair_order(unsigned char *smem, XF xf, int shift) {
-    K *keys = reinterpret_cast<K *>(smem + L::off_keys);
-    unsigned short *place = reinterpret_cast<unsigned short *>(smem + L::off_place);
-    bool again = true;
-    for (int round = 0; again && round < L::TILE; ++round) {
-        again = false;
-        for (int odd = 0; odd < 2; ++odd) {
-            for (int p = 2 * (int)threadIdx.x + odd; p + 1 < L::TILE; p += 2 * kPassThreads) {
-                if (out_of_order<K, L::VB != 0>(keys[p], keys[p + 1], L::VB ? place[p] : 0u, L::VB ? place[p + 1] : 0u, xf, shift)) {
-                    const K k = keys[p];
-                    keys[p] = keys[p + 1];
-                    keys[p + 1] = k;
-                    if (L::VB != 0) {
-                        const unsigned short s = place[p];
-                        place[p] = place[p + 1];
-                        place[p + 1] = s;
-                    }
-                    again = true;
-                }
-            }
-            __syncthreads();
-        }
-        again = block_any(again);
-    }
+    put_in_order<K, L::VB != 0>(reinterpret_cast<K *>(smem + L::off_keys), reinterpret_cast<unsigned short *>(smem + L::off_place), L::TILE,
+                                (int)threadIdx.x, kPassThreads, xf, shift, [](bool moved) { return block_any(moved); });
 }
 
 // Writes the tile in the slots to global memory; true when a slot is out of order.

@@ -273,26 +273,8 @@ resident_sort_kernel(SortBuffers<K, V> io, KeyXform<K> xf, TempHeader *hdr, unsi
             const unsigned int p = tid + i * kResidentThreads;
             if (p + 1 < tile) bad |= wrong(p);
         }
-        // Neighbours that are the wrong way round change places until none are (the atomics of a warp
-        // were not served in lane order: not observed).
-        for (unsigned int round = 0; __syncthreads_or(bad) && round < tile; ++round) {
-            bad = false;
-            for (int odd = 0; odd < 2; ++odd) {
-                for (unsigned int p = 2 * tid + odd; p + 1 < tile; p += 2 * kResidentThreads)
-                    if (wrong(p)) {
-                        const K k = slots[p];
-                        slots[p] = slots[p + 1];
-                        slots[p + 1] = k;
-                        if (VALUES) {
-                            const unsigned short s = place[p];
-                            place[p] = place[p + 1];
-                            place[p + 1] = s;
-                        }
-                        bad = true;
-                    }
-                __syncthreads();
-            }
-        }
+        if (__syncthreads_or(bad))  // (the atomics of a warp were not served in lane order: not observed)
+            put_in_order<K, VALUES>(slots, place, (int)tile, tid, kResidentThreads, xf, shift, [](bool moved) { return __syncthreads_or(moved) != 0; });
         if (meeting == kAlone) {
             clear_mine();
             first = false;

@@ -1,8 +1,9 @@
-// What the kernels of the radix sort share: key transforms, sequenced values, and the check that ranks
-// taken with atomics came out in order.
+// What the kernels of the radix sort share: key transforms, sequenced values, and (slot_order.cuh) the
+// check that ranks taken with atomics came out in order.
 #pragma once
 
 #include "common.cuh"
+#include "slot_order.cuh"
 
 namespace b200alg {
 
@@ -52,30 +53,18 @@ template <typename V> __device__ __forceinline__ V sequence_value(int kind, int6
 // RadixSortOperations.tt:77-93 and the descending complement of :122-123.
 template <typename K> struct KeyXform {
     K xor_neg, xor_pos;
-    __device__ __forceinline__ K operator()(K raw) const {
+    __host__ __device__ __forceinline__ K operator()(K raw) const {
         return raw ^ ((raw >> (sizeof(K) * 8 - 1)) ? xor_neg : xor_pos);
     }
 };
 // Ascending unsigned keys need no transform at all.
 template <typename K> struct KeyIdentity {
-    __device__ __forceinline__ K operator()(K raw) const { return raw; }
+    __host__ __device__ __forceinline__ K operator()(K raw) const { return raw; }
 };
 
 struct NoValue {};
 template <typename V> struct ValueBytes { static constexpr int value = sizeof(V); };
 template <> struct ValueBytes<NoValue> { static constexpr int value = 0; };
-
-// Whether of two neighbouring slots the first has to come after the second (and must not: see the top
-// of digit_pass.cuh).
-template <typename K, bool VALUES, typename XF>
-__device__ __forceinline__ bool out_of_order(K first, K second, unsigned int first_place, unsigned int second_place, XF xf, int shift) {
-    if constexpr (!VALUES) {
-        const K sorted = (K)((K)~(K)0 >> (8 * (int)sizeof(K) - 8 - shift));  // this digit and the ones below it
-        return (K)(xf(first) & sorted) > (K)(xf(second) & sorted);
-    } else {
-        return (((xf(first) ^ xf(second)) >> shift) & 0xFFu) == 0 && first_place > second_place;
-    }
-}
 
 // The raw key whose transform is all ones: it fills a ragged tile up and sorts behind every real key.
 template <typename K> __device__ __forceinline__ K padding_key(const KeyXform<K> &xf) {
