@@ -169,8 +169,9 @@ __device__ __forceinline__ unsigned int ld_relaxed_u32(const unsigned int *p) {
     asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
-__device__ __forceinline__ void st_release_u32(unsigned int *p, unsigned int v) {
-    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+// *p |= bits, behind everything this thread has done or been told of.
+__device__ __forceinline__ void or_release_u32(unsigned int *p, unsigned int bits) {
+    asm volatile("red.release.gpu.global.or.b32 [%0], %1;" ::"l"(p), "r"(bits) : "memory");
 }
 __device__ __forceinline__ unsigned int ld_acquire_u32(const unsigned int *p) {
     unsigned int v;

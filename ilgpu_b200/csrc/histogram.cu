@@ -14,7 +14,6 @@ namespace b200alg {
 namespace cg = cooperative_groups;
 
 constexpr int kHistThreads = 512;
-constexpr int kHistWarps = kHistThreads / 32;
 constexpr int64_t kHistSmemBytes = 48 * 1024;  // static limit, no opt-in needed
 
 struct LocParams {

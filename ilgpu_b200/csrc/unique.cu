@@ -392,7 +392,7 @@ unique_in_place_kernel(T *data, int64_t n, long long *out_count, long long *host
                 if ((well = wait(&full_bar[0], 0u))) more = take_tile(k);
             for (int k = 0; well && tile_of[k % kRingStages] < num_tiles; ++k) {
                 if (!wait(&read_bar[k % kRingStages], (unsigned int)(k / kRingStages) & 1u)) break;
-                asm volatile("red.release.gpu.global.or.b32 [%0], %1;" ::"l"(counts + tile_of[k % kRingStages]), "r"(kRead) : "memory");
+                or_release_u32(counts + tile_of[k % kRingStages], kRead);
                 if (k > 0 && more) {  // the tile before is stored next
                     if (!wait(&free_bar[(k - 1) % kRingStages], (unsigned int)((k - 1) / kRingStages) & 1u)) break;
                     more = take_tile(k - 1 + kRingStages);
