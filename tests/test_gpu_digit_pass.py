@@ -1,6 +1,7 @@
 """The digit pass of the radix sort around its tiles: one key, the last key of a tile, of two tiles
 (whose places are published together) and one more, for key and value sizes with different tiles;
-keys that meet in few digits; against a stable host sort."""
+keys that meet in few digits; against a stable host sort.  (The library sorts all but the longest of
+these in one launch; test_gpu_long_sorts.py has the same edges in the digit pass itself.)"""
 import numpy as np
 import pytest
 import torch
