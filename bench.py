@@ -32,7 +32,8 @@ SEED = 2
 # DRAM traffic of the sort's kernels comes from the ncu summary under profiles/ (written when a
 # capture is taken); it is only quoted while the kernel source is the one that was profiled.
 TRAFFIC_FILE = os.path.join(ROOT, "profiles", "sort_kernel.md")
-KERNEL_SOURCES = [os.path.join(ROOT, "ilgpu_b200", "csrc", f) for f in ("radix_sort.cu", "digit_pass.cuh", "sort_common.cuh", "common.cuh")]
+KERNEL_SOURCES = [os.path.join(ROOT, "ilgpu_b200", "csrc", f)
+                  for f in ("radix_sort.cu", "digit_pass.cuh", "sort_common.cuh", "slot_order.cuh", "poll_limit.cuh", "common.cuh")]
 
 
 def kernel_source_digest() -> str:
@@ -466,6 +467,19 @@ def run_profile_case(case: str) -> None:
         for r in range(3):
             keys = synthetic.zipf_uint64_device(n, 4 + r, "cuda")
             sort(None, keys, vals.clone(), temp)
+    elif case == "sort_small":   # one launch of a few us: what lies in L2 is what such a sort finds
+        n = 5000
+        temp = acc.Allocate1D(acc.ComputeRadixSortTempStorageSize(Sorts.AscendingUInt32, n), torch.int32)
+        sort = acc.CreateRadixSort(Sorts.AscendingUInt32)
+        for r in range(3):
+            keys = synthetic.uniform_uint32_device(n, SEED + r, "cuda")
+            sort(None, keys, temp)
+    elif case == "unique":       # runs of four on average
+        n = 50_000_017
+        starts = synthetic.uniform_float32_device(n, 6, "cuda").lt_(0.25)
+        data = torch.cumsum(starts, 0, dtype=torch.int32)
+        for r in range(3):
+            acc.Unique(None, data.clone())
     elif case == "partition":
         # the partition + exchange step of the multi-GPU sort on one GPU: eight buckets (equal
         # slices of the key range, as on an 8-GPU box), each stored into a buffer of its own
@@ -496,6 +510,13 @@ def run_profile_case(case: str) -> None:
         cell = acc.Allocate1D(1, torch.float32)
         for _ in range(3):
             acc.CreateReduction(Ops.AddFloat)(None, x, cell)
+    elif case == "histogram_bins":  # 16-bit samples, a bin for each value
+        n = 60_000_001
+        x = synthetic.normal_float32_device(n, 3, "cuda").mul_(8000.0).add_(32768.0).clamp_(0.0, 65535.0).to(torch.int32)
+        bins = torch.zeros(65_536, dtype=torch.int32, device="cuda")
+        ovf = torch.zeros(1, dtype=torch.int32, device="cuda")
+        for _ in range(3):
+            acc.Histogram(None, x, bins, ovf, ib.ModuloLocator())
     else:
         n = 1 << 28
         f = synthetic.normal_float32_device(n, 3, "cuda")
@@ -871,7 +892,7 @@ def main() -> None:
     ap.add_argument("--warmup", type=int, default=5)
     ap.add_argument("--impl", default="b200", choices=["b200", "reference"])
     ap.add_argument("--no-secondary", action="store_true", help="skip the scan / reduce / histogram figures")
-    ap.add_argument("--profile-case", choices=["sort", "sort_pairs", "partition", "scan", "reduce", "histogram"],
+    ap.add_argument("--profile-case", choices=["sort", "sort_pairs", "sort_small", "partition", "scan", "reduce", "histogram", "histogram_bins", "unique"],
                     help="run a few launches of one primitive on a small case and exit (the target of ncu captures)")
     args = ap.parse_args()
     if args.warmup < 3:

@@ -207,11 +207,11 @@ constexpr int kTableChunk = 3 << 14;   // elements of a block between two sweeps
 constexpr int kTableMaxCluster = 4;
 
 // Which kernel: the table where bins are many and the elements enough to pay for the flush.  Below
-// 16 elements per bin one global atomic per element is as fast (65536 bins: 16.5 us both ways at
-// 2^20 elements; 47 us against 377 us at 3 * 10^7); up to 1024 bins the kernel above, whose smaller
-// blocks are cleared and flushed sooner, unless the input does not fit in L2 and its locator does
-// more than a few float operations per element (2^26 doubles, 256 bins: 85 us against 97 us; floats
-// are at the HBM rate either way).
+// 16 elements per bin one global atomic per element is as fast (int32 modulo 65536 bins, this kernel
+// and the others: 19 against 9 us at 2^18 elements, 20.5 both at 2^20, 22 against 59 at 2^22, 49 against
+// 391 at 3 * 10^7); up to 1024 bins the kernel above, whose smaller blocks are cleared and flushed
+// sooner, unless the input does not fit in L2 and its locator does more than a few float operations
+// per element (2^26 doubles, 256 bins: 84 us against 96 us; floats are at the HBM rate either way).
 constexpr int64_t kTableLongInput = 1ll << 27;  // bytes
 template <typename T, int LOCATOR> bool use_table(int64_t nb, int64_t n, bool dense) {
     if (nb * 2 > kTableBytes || n < 16 * nb) return false;

@@ -342,6 +342,8 @@ unique_in_place_kernel(T *data, int64_t n, long long *out_count, long long *host
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     unsigned long long *prefixes = reinterpret_cast<unsigned long long *>(counts + padded_tiles(num_tiles));
+    // Views off 16 bytes are loaded element by element when their turn comes: 81 instead of 65 us (5 * 10^7
+    // uint32, a quarter kept), 165 instead of 85 for 10^8 bytes.
     auto bulk = [&](int tile) { return (int64_t)(tile + 1) * TILE <= n && ((uintptr_t)data & 15u) == 0; };
     auto stage_of = [&](int k) { return ring + k % kRingStages * kRingStageBytes + 128; };
     auto take_tile = [&](int k) {  // tiles are handed out in order
