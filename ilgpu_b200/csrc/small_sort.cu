@@ -1,9 +1,11 @@
-// Radix sort of views that fit on the SMs as a whole: one launch, every block keeps its share of the
-// keys in registers and shared memory while a pass works out where they go.
+// Radix sort of views that fit on the SMs as a whole: one launch.
 //
 // What a short sort costs is not moving keys but the chain of steps: with one kernel per step (clear,
 // histogram, offsets, one per digit, copy home) 5000 keys took 50 us, 25 of them inside kernels that
-// wait for memory or for one another.  Here a pass is
+// wait for memory or for one another.
+//
+// What one block can hold it sorts alone (block_sort_kernel, local_sort.cuh).  Several blocks keep their
+// shares of the keys in registers and shared memory (resident_sort_kernel); a pass is
 //
 //   rank      one shared-memory atomic per key on the warp's count of its digit
 //   count     the warps' counts become slots of the block's tile
@@ -11,12 +13,11 @@
 //   exchange  blocks publish their counts, meet, add up the counts of all blocks, move their slots to
 //             where they go, and meet again
 //
-// One block alone needs no exchange.  The up to sixteen blocks of a cluster read one another's counts
-// and move keys through distributed shared memory; only the first and the last step touch global
-// memory.  More blocks than that exchange through global memory, in place (everybody has read its share
-// when they meet), and meet in the grid barrier of a cooperative launch.  Digits that all keys share
-// are skipped.
-#include "sort_common.cuh"
+// The up to sixteen blocks of a cluster read one another's counts and move keys through distributed
+// shared memory; only the first and the last step touch global memory.  More blocks than that exchange
+// through global memory, in place (everybody has read its share when they meet), and meet in the grid
+// barrier of a cooperative launch.  Digits that all keys share are skipped.
+#include "local_sort.cuh"
 
 #include <cooperative_groups.h>
 
@@ -31,7 +32,7 @@ constexpr int kResidentFixed = kResidentWarps * kRadix * 4 + 2 * kRadix * 4 + kR
 constexpr int kColumnThreads = kResidentThreads / kRadix;     // threads that share a digit when counts become slots
 constexpr int kColumnRows = kResidentWarps / kColumnThreads;  // and warps each of them adds up
 constexpr int kMaxCluster = 16;
-enum : int { kAlone = 0, kInCluster = 1, kInGrid = 2 };
+enum : int { kInCluster = 0, kInGrid = 1 };
 
 // Shared memory of a key and its value: slots and the value's place; in a cluster, where the next pass
 // comes in as well.
@@ -159,7 +160,6 @@ resident_sort_kernel(SortBuffers<K, V> io, KeyXform<K> xf, TempHeader *hdr, unsi
                 }
             }
         }
-        if (meeting == kAlone) __syncthreads();
     }
     auto next_pass = [&](int p) {  // the first digit from p on in which keys differ
         const unsigned long long differ = m.differ;
@@ -167,47 +167,18 @@ resident_sort_kernel(SortBuffers<K, V> io, KeyXform<K> xf, TempHeader *hdr, unsi
         return p;
     };
     bool first = true;
-    // (a cluster or grid learns what differs only when it meets, so it always runs the first pass)
-    int pass = meeting == kAlone ? next_pass(0) : 0;
-    if (pass >= PASSES) {  // all keys are equal
-#pragma unroll
-        for (int i = 0; i < ITEMS; ++i) {
-            if (i >= items) break;
-            slots[own + i * 32] = key[i];
-            if (VALUES) place[own + i * 32] = (unsigned short)(own + i * 32);
-        }
-        __syncthreads();
-    }
+    // (what differs is known only when the blocks have met, so the first pass always runs)
+    int pass = 0;
     while (pass < PASSES) {
         const int shift = pass * 8;
         if (!first) {
             if (meeting == kInGrid) {
                 load(io.out, io.vout, false);
-            } else if (meeting == kInCluster) {
-#pragma unroll
-                for (int i = 0; i < ITEMS; ++i) {
-                    if (i >= items) break;
-                    key[i] = next_keys[own + i * 32];
-                }
-            } else if constexpr (VALUES) {
-                V v[ITEMS];
-#pragma unroll
-                for (int i = 0; i < ITEMS; ++i) {
-                    if (i >= items) break;
-                    key[i] = slots[own + i * 32];
-                    v[i] = values[place[own + i * 32]];
-                }
-                __syncthreads();
-#pragma unroll
-                for (int i = 0; i < ITEMS; ++i) {
-                    if (i >= items) break;
-                    values[own + i * 32] = v[i];
-                }
             } else {
 #pragma unroll
                 for (int i = 0; i < ITEMS; ++i) {
                     if (i >= items) break;
-                    key[i] = slots[own + i * 32];
+                    key[i] = next_keys[own + i * 32];
                 }
             }
         }
@@ -236,7 +207,7 @@ resident_sort_kernel(SortBuffers<K, V> io, KeyXform<K> xf, TempHeader *hdr, unsi
             }
             const unsigned int parts_ahead = total - part_total;
             total = __shfl_sync(0xffffffffu, total, lane | (kColumnThreads - 1));
-            if (part == 0 && meeting != kAlone) {
+            if (part == 0) {
                 if (meeting == kInCluster) counts[d] = (unsigned short)total;
                 else all_counts[(size_t)blockIdx.x * kRadix + d] = (unsigned short)total;
             }
@@ -275,12 +246,6 @@ resident_sort_kernel(SortBuffers<K, V> io, KeyXform<K> xf, TempHeader *hdr, unsi
         }
         if (__syncthreads_or(bad))  // (the atomics of a warp were not served in lane order: not observed)
             put_in_order<K, VALUES>(slots, place, (int)tile, tid, kResidentThreads, xf, shift, [](bool moved) { return __syncthreads_or(moved) != 0; });
-        if (meeting == kAlone) {
-            clear_mine();
-            first = false;
-            pass = next_pass(pass + 1);
-            continue;
-        }
 
         meet();  // counts (and, the first time, masks) of all blocks are there; every block holds its share
         // the counts of all blocks, one row per warp and turn, summed in the ranking tables' place
@@ -400,40 +365,129 @@ resident_sort_kernel(SortBuffers<K, V> io, KeyXform<K> xf, TempHeader *hdr, unsi
             next_values = v;
         }
     }
-    if (meeting == kAlone) {
+}
+
+// Values of a thread's elements of a block (element own + i * 32) to shared memory, eight under way at a time.
+template <typename V>
+__device__ __forceinline__ void load_values(V *values, const V *from, int value_seq, int64_t base, int own, int count, int items) {
+    constexpr int AHEAD = sizeof(V) <= 8 ? 8 : 4;
+#pragma unroll 1
+    for (int first = 0; first < items; first += AHEAD) {
+        V v[AHEAD];
 #pragma unroll
-        for (int i = 0; i < ITEMS; ++i) {
-            if (i >= items) break;
-            const int p = tid + i * kResidentThreads;
-            if (p < valid) {
-                io.out[(int64_t)p * io.stride] = slots[p];
-                if constexpr (VALUES) io.vout[p] = values[place[p]];
+        for (int i = 0; i < AHEAD; ++i) {
+            const int at = own + (first + i) * 32;
+            if (first + i < items && at < count) {
+                if constexpr (sizeof(V) <= 8) v[i] = value_seq != kSeqNone ? sequence_value<V>(value_seq, base + at) : from[base + at];
+                else v[i] = from[base + at];
             }
+        }
+#pragma unroll
+        for (int i = 0; i < AHEAD; ++i) {
+            const int at = own + (first + i) * 32;
+            if (first + i < items && at < count) values[at] = v[i];
         }
     }
 }
 
+// ---- one block ---------------------------------------------------------------------------
+template <typename K, typename V>
+__global__ void __launch_bounds__(kLocalThreads, 1)
+block_sort_kernel(SortBuffers<K, V> io, KeyXform<K> xf, TempHeader *hdr, int items, int value_seq) {
+    constexpr int VB = ValueBytes<V>::value;
+    constexpr bool PLACE = by_place<K>(VB != 0);
+    extern __shared__ __align__(128) unsigned char smem[];
+    const int tid = threadIdx.x, threads = (int)blockDim.x, most = threads * items;
+    unsigned int *words = reinterpret_cast<unsigned int *>(smem + local_fixed_bytes(threads));
+    V *values = reinterpret_cast<V *>(words + most);
+    K *keys = reinterpret_cast<K *>(reinterpret_cast<unsigned char *>(values) + (size_t)most * VB);
+    const int own = (tid >> 5) * 32 * items + (tid & 31);
+    const LocalShared shared = local_shared(smem);
+    local_clear(shared);
+    grid_dependency_wait();
+    const int count = (int)effective_n(io);
+    if (tid == 0) hdr->wait_limit_hit = 0u;
+
+    K key[kLocalItems];
+    K low = (K)~(K)0, high = 0;
+#pragma unroll
+    for (int i = 0; i < kLocalItems; ++i) {
+        if (i >= items) break;
+        const int at = own + i * 32;
+        if (at < count) key[i] = io.in[(int64_t)at * io.stride];
+    }
+    if constexpr (VB != 0) load_values<V>(values, io.vin, value_seq, 0, own, count, items);
+#pragma unroll
+    for (int i = 0; i < kLocalItems; ++i) {
+        if (i >= items) break;
+        const int at = own + i * 32;
+        if (at < count) {
+            const K b = xf(key[i]);
+            key[i] = b;
+            low = b < low ? b : low;
+            high = b > high ? b : high;
+            if constexpr (PLACE) keys[at] = b;
+        }
+    }
+    local_range(shared, low, high);
+    const LocalSort<K, PLACE> sort{shared, words, keys, count, items, low, high};
+    K *const out = io.out;
+    V *const vout = io.vout;
+    const int64_t stride = io.stride;
+    sort.run(key, [=](int p, K k, unsigned int word) {
+        out[p * stride] = xf.raw(k);
+        if constexpr (VB != 0) vout[p] = values[LocalSort<K, PLACE>::place_of(word)];
+    });
+}
+
 // ---- host side ---------------------------------------------------------------------------
-// Which blocks (times on the GPU, with the launch):
-//   one       up to 8 elements per thread, 12 of keys alone with 4 or 8 bytes.  One block against a
-//             cluster, us, by key bytes / value bytes:
-//                          4500          5000          6144          6700          8192
-//                1 / 0   10.3   8.3   10.2  10.1   10.2   8.3   10.4   8.4   12.3  10.2
-//                2 / 0   12.3  12.3   12.3  12.4   14.3  12.3   14.4  12.4   16.4  12.3
-//                4 / 0   16.4  20.5   18.3  20.5   18.4  20.5   20.5  20.5   22.6  18.5
-//                8 / 0   30.7  34.8   30.9  34.8   34.8  36.8   38.9  35.0   43.1  32.9
-//                4 / 4   20.5  22.5   22.5  22.6   24.6  22.5   26.7  22.5   28.7  22.6
-//                8 / 4   36.9  39.0   39.0  41.0   45.1  41.0   51.2  41.0   55.3  38.9
-//                8 / 8   39.0  39.1   43.0  41.0   49.1  41.0   53.2  41.0   59.4  39.1
+// Which blocks (times on the GPU, us, with the launch and the copy that brings the data):
+//   one       block_sort_kernel, against a cluster, by key bytes / value bytes:
+//                          4500          6000          7500          9000         12000
+//                1 / 0    8.4   8.3    8.2   8.4   10.2   8.6   10.3   8.2   12.3   8.8
+//                2 / 0   10.2  12.3   10.3  12.3   12.3  12.3   14.3  12.5   16.4  13.1
+//                1 / 4   12.5  13.2   12.3  13.2   14.4  13.2   16.7  13.3   21.3  24.7
+//                2 / 8   14.7  17.3   15.9  17.6   16.9  17.4   19.1  17.6   22.6  17.4
+//                4 / 0   11.3  16.6   12.3  18.4   14.3  18.5   16.4  20.8   19.1  20.8
+//                4 / 4   15.1  23.6   16.6  24.8   19.5  24.3   21.9  25.5   25.7  27.8
+//                8 / 0   12.3  29.0   14.4  35.2   16.4  34.7   18.4  37.5   22.5  39.9
+//                8 / 4   17.0  42.2   19.1  42.5   21.3  42.3   23.5  46.7   27.7  46.8
+//                8 / 8   18.7  41.9   21.2  43.3   25.3  42.4   28.3  46.9    does not fit
 //   cluster   up to 40960 elements (uint32 keys / pairs: 40000: 27 / 33 us against 29 / 32 us with a
 //             grid; 60000: 35 / 43 us against 29 / 33 us);
 //   grid      about 64 blocks until they have 4 keys per thread, then more, up to about the length from
 //             which the passes over tiles are as fast (against those: 700000 uint32 keys / pairs / 8-byte
 //             keys 51 / 61 / 104 us against 59 / 64 / 99; 2^20 uint32 keys 59 against 61 us; 800000 pairs
 //             62 against 59 us).
-constexpr int64_t alone_most(int key_bytes, int value_bytes) { return kResidentThreads * (value_bytes == 0 && key_bytes >= 4 ? 12 : 8); }
+constexpr int64_t alone_most(int key_bytes) { return key_bytes == 1 ? 6144 : key_bytes == 2 ? 7680 : kLocalMost; }
 constexpr int64_t kClusterMost = 5 * kMaxCluster * kResidentThreads;
 constexpr int64_t kGridMostNarrow = 1 << 20, kGridMost = 3 << 18;
+
+// Bytes of shared memory of an element.
+static int local_bytes(int key_bytes, int value_bytes) { return 4 + value_bytes + (value_bytes || key_bytes == 8 ? key_bytes : 0); }
+
+template <typename K, typename V>
+static int run_block_sort(cudaStream_t s, const SortCall &call, uint64_t xn, uint64_t xp, void *temp, bool *taken) {
+    constexpr int VB = ValueBytes<V>::value;
+    const int64_t n = call.n;
+    if (n > alone_most(sizeof(K))) return B200ALG_OK;
+    const int threads = n <= kLocalThreads * 2 ? kLocalThreads / 2 : kLocalThreads;  // (1000 keys: 7.2 against 8.1 us)
+    const int items = (int)ceil_div(n, threads);
+    const size_t smem = local_fixed_bytes(threads) + (size_t)threads * items * local_bytes(sizeof(K), VB);
+    if (items > kLocalItems || smem > kResidentSmem) return B200ALG_OK;
+    auto kernel = block_sort_kernel<K, V>;
+    static ContextCache<int> opted_in;
+    int done = 0;
+    if (!opted_in.find(&done)) {
+        B200ALG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kResidentSmem));
+        opted_in.store(1);
+    }
+    SortBuffers<K, V> io{(const K *)call.in_keys, (K *)call.out_keys, nullptr, (const V *)call.in_values, (V *)call.out_values, nullptr,
+                         call.stride, n, call.n_device};
+    B200ALG_CUDA_TRY(launch_dependent(kernel, dim3(1), dim3(threads), smem, s, io, KeyXform<K>{(K)xn, (K)xp}, (TempHeader *)temp, items, call.value_seq));
+    *taken = true;
+    return B200ALG_OK;
+}
 
 struct ResidentLimits {
     int cluster;  // most blocks of one cluster
@@ -443,6 +497,9 @@ struct ResidentLimits {
 template <typename K, typename V>
 static int run_resident(cudaStream_t s, const SortCall &call, uint64_t xn, uint64_t xp, void *temp, int64_t temp_bytes, bool *taken) {
     constexpr int VB = ValueBytes<V>::value, ITEMS = resident_items(sizeof(K), VB, false), CLUSTER_ITEMS = resident_items(sizeof(K), VB, true);
+    *taken = false;
+    const int rc = run_block_sort<K, V>(s, call, xn, xp, temp, taken);
+    if (rc != B200ALG_OK || *taken) return rc;
     auto kernel = resident_sort_kernel<K, V>;
     static ContextCache<ResidentLimits> cache;
     ResidentLimits lim;
@@ -473,13 +530,9 @@ static int run_resident(cudaStream_t s, const SortCall &call, uint64_t xn, uint6
         lim.grid = per_sm * sm_count();
         cache.store(lim);
     }
-    *taken = false;
     const int64_t n = call.n;
     int meeting, blocks;
-    if (n <= alone_most(sizeof(K), VB) && n <= kResidentThreads * ITEMS) {
-        meeting = kAlone;
-        blocks = 1;
-    } else if (n <= kClusterMost && n <= (int64_t)lim.cluster * kResidentThreads * CLUSTER_ITEMS) {
+    if (n <= kClusterMost && n <= (int64_t)lim.cluster * kResidentThreads * CLUSTER_ITEMS) {
         meeting = kInCluster;
         blocks = 2;
         while (blocks < lim.cluster && blocks * kResidentThreads * 2 < n) blocks *= 2;
@@ -507,7 +560,7 @@ static int run_resident(cudaStream_t s, const SortCall &call, uint64_t xn, uint6
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cfg.attrs = attr;
-    cfg.numAttrs = meeting == kAlone ? 0 : 1;
+    cfg.numAttrs = 1;
     if (meeting == kInCluster) {
         attr[0].id = cudaLaunchAttributeClusterDimension;
         attr[0].val.clusterDim.x = blocks;

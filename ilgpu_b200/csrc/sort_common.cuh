@@ -56,6 +56,12 @@ template <typename K> struct KeyXform {
     __host__ __device__ __forceinline__ K operator()(K raw) const {
         return raw ^ ((raw >> (sizeof(K) * 8 - 1)) ? xor_neg : xor_pos);
     }
+    // The key of the transformed bits.  (No transform has constants that differ in their sign bit, so the sign
+    // of bits ^ xor_pos is the key's.)
+    __host__ __device__ __forceinline__ K raw(K bits) const {
+        const K r = (K)(bits ^ xor_pos);
+        return (r >> (sizeof(K) * 8 - 1)) ? (K)(bits ^ xor_neg) : r;
+    }
 };
 // Ascending unsigned keys need no transform at all.
 template <typename K> struct KeyIdentity {
@@ -68,8 +74,7 @@ template <> struct ValueBytes<NoValue> { static constexpr int value = 0; };
 
 // The raw key whose transform is all ones: it fills a ragged tile up and sorts behind every real key.
 template <typename K> __device__ __forceinline__ K padding_key(const KeyXform<K> &xf) {
-    const K r = (K)((K)~(K)0 ^ xf.xor_pos);
-    return (r >> (sizeof(K) * 8 - 1)) ? (K)((K)~(K)0 ^ xf.xor_neg) : r;
+    return xf.raw((K)~(K)0);
 }
 template <typename K> __device__ __forceinline__ K padding_key(const KeyIdentity<K> &) { return (K)~(K)0; }
 
