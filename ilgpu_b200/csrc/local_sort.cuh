@@ -23,9 +23,7 @@
 
 namespace b200alg {
 
-constexpr int kLocalThreads = 512;           // most threads of a block (a multiple of 256)
-constexpr int kLocalItems = 24;              // most elements of a thread
-constexpr int kLocalMost = kLocalThreads * kLocalItems;
+constexpr int kLocalMost = 12288;            // elements: 24 for each of 512 threads, 12 for each of 1024
 constexpr int kPlaceBits = 14;
 static_assert(kLocalMost <= 1 << kPlaceBits, "a place fits its bits, a count its half of a word");
 constexpr int kLocalDigitBits = 9;
@@ -133,13 +131,39 @@ template <typename K> __device__ __forceinline__ void local_range(const LocalSha
     high = (K)~least((K)~(lane < warps ? (K)s.high[lane] : (K)0));
 }
 
+// Values of a thread's elements of a block (element own + i * 32) to shared memory, eight under way at a time.
+template <typename V>
+__device__ __forceinline__ void load_values(V *values, const V *from, int value_seq, int64_t base, int own, int count, int items) {
+    constexpr int AHEAD = sizeof(V) <= 8 ? 8 : 4;
+#pragma unroll 1
+    for (int first = 0; first < items; first += AHEAD) {
+        V v[AHEAD];
+#pragma unroll
+        for (int i = 0; i < AHEAD; ++i) {
+            const int at = own + (first + i) * 32;
+            if (first + i < items && at < count) {
+                if constexpr (sizeof(V) <= 8) v[i] = value_seq != kSeqNone ? sequence_value<V>(value_seq, base + at) : from[base + at];
+                else v[i] = from[base + at];
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < AHEAD; ++i) {
+            const int at = own + (first + i) * 32;
+            if (first + i < items && at < count) values[at] = v[i];
+        }
+    }
+}
+
+// Bytes of shared memory of an element.
+constexpr int local_bytes(int key_bytes, int value_bytes) { return 4 + value_bytes + (value_bytes || key_bytes == 8 ? key_bytes : 0); }
+
 // Whether elements of a key / value size travel as places.
 template <typename K> __host__ __device__ constexpr bool by_place(bool values) { return values || sizeof(K) == 8; }
 
 // Sorts `count` elements.  By place: keys (in shared memory, transformed) stay, words receive the places
 // in order.  Else: key[] holds this thread's transformed keys (element warp * 32 * items + i * 32 + lane), words
 // receive the keys less `low`.  store(p, key, word) is called for the p-th in order, possibly again.
-template <typename K, bool PLACE> struct LocalSort {
+template <typename K, bool PLACE, int ITEMS> struct LocalSort {
     LocalShared s;
     unsigned int *words;
     const K *keys;
@@ -157,19 +181,22 @@ template <typename K, bool PLACE> struct LocalSort {
         else return a > b;
     }
 
-    template <typename Digit, typename Next> __device__ __forceinline__ void pass(unsigned int (&w)[kLocalItems], Digit digit, Next next) const {
+    // counted(c): c.x and c.y are the block's count and first place of digits threadIdx.x % 256 (lower half) and
+    // 256 + threadIdx.x % 256 (upper half).
+    template <typename Digit, typename Next, typename Counted>
+    __device__ __forceinline__ void pass(unsigned int (&w)[ITEMS], Digit digit, Next next, Counted counted) const {
         unsigned int *mine = s.table + (threadIdx.x >> 5) * kLocalWords;
-        unsigned int rank[(kLocalItems + 1) / 2];  // two to a word
+        unsigned int rank[(ITEMS + 1) / 2];  // two to a word
 #pragma unroll
-        for (int i = 0; i < kLocalItems; ++i) {
+        for (int i = 0; i < ITEMS; ++i) {
             if (i >= items) break;
             const unsigned int r = local_rank(mine, digit(w[i]));
             if (i & 1) rank[i / 2] |= r << 16; else rank[i / 2] = r;
         }
         __syncthreads();
-        local_places(s);
+        counted(local_places(s));
 #pragma unroll
-        for (int i = 0; i < kLocalItems; ++i) {
+        for (int i = 0; i < ITEMS; ++i) {
             if (i >= items) break;
             words[(i & 1 ? rank[i / 2] >> 16 : rank[i / 2] & 0xFFFFu) + local_place(mine, digit(w[i]))] = next(w[i], i);
         }
@@ -281,85 +308,85 @@ template <typename K, bool PLACE> struct LocalSort {
         return bad;
     }
 
+    // Whether two of a few keys of every warp agree in all bits but the lowest `below` and differ in those: then
+    // many of the block's do.
+    __device__ __forceinline__ bool ties_likely(const K *key, int own, int below) const {
+        const int lane = threadIdx.x & 31;
+        K mine = 0;
+        if (own < count) mine = PLACE ? (K)(keys[own] - low) : (K)(key[0] - low);
+        bool tie = false;
+#pragma unroll
+        for (int k = 1; k <= 8; k *= 2) {
+            K other;
+            if constexpr (sizeof(K) == 8) other = __shfl_down_sync(0xffffffffu, mine, k);
+            else other = (K)__shfl_down_sync(0xffffffffu, (unsigned int)mine, k);
+            tie |= lane + k < 32 && own + k < count && other != mine && other >> below == mine >> below;
+        }
+        return __syncthreads_or(tie) != 0;
+    }
+
     // The tables are clear, keys (by place) are in shared memory behind a barrier, low and high are known.
     template <typename Store> __device__ __forceinline__ void run(const K *key, Store store) const {
         const int own = (int)(threadIdx.x >> 5) * 32 * items + (int)(threadIdx.x & 31);
         const K range = (K)(high - low);
         const int bits = sizeof(K) == 8 ? 64 - __clzll((long long)range) : 32 - __clz((int)(unsigned int)range);
-        unsigned int w[kLocalItems];
         if (threadIdx.x == 0) *s.found = 0u;
-        {
-            const int upper = bits < kLocalPrefixBits ? bits : kLocalPrefixBits, below = bits - upper;
-            const int passes = (upper + kLocalDigitBits - 1) / kLocalDigitBits, width = passes ? (upper + passes - 1) / passes : 0;
-            const unsigned int mask = (1u << width) - 1u;
-            // elements past the last one sort behind all others: largest digits, and last in every tie
+        int from = bits > kLocalPrefixBits ? bits - kLocalPrefixBits : 0;  // the lowest bit that is sorted by
+        if (from > 0 && ties_likely(key, own, from)) from = 0;
+        unsigned int w[ITEMS];
+        bool fresh = true;  // words hold nothing yet
+        for (;;) {
+            // By place, bits go in turns of up to 27; in the first pass of a turn the keys are looked up, later ones
+            // find their digits above the place.  Elements past the last one sort behind all others: largest digits,
+            // and last in every tie.
+            if (bits == 0) {
 #pragma unroll
-            for (int i = 0; i < kLocalItems; ++i) {
-                if (i >= items) break;
-                const int at = own + i * 32;
-                if constexpr (PLACE) w[i] = at < count ? (unsigned int)((K)(keys[at] - low) >> below) : ~0u;
-                else w[i] = at < count ? (unsigned int)(K)(key[i] - low) : ~0u;
-            }
-            if (passes == 0) {
-#pragma unroll
-                for (int i = 0; i < kLocalItems; ++i) {
+                for (int i = 0; i < ITEMS; ++i) {
                     if (i >= items) break;
-                    words[own + i * 32] = PLACE ? (unsigned int)(own + i * 32) : w[i];
+                    words[own + i * 32] = PLACE ? (unsigned int)(own + i * 32) : 0u;
                 }
                 __syncthreads();
             }
-            for (int p = 0; p < passes; ++p) {
-                if (p > 0) {
+            if (PLACE) fresh = true;
+            for (int turn = from; turn < bits;) {
+                const int left = bits - turn, length = !PLACE ? left : left % kLocalPrefixBits ? left % kLocalPrefixBits : kLocalPrefixBits;
+                const int passes = (length + kLocalDigitBits - 1) / kLocalDigitBits, width = (length + passes - 1) / passes;
+                const unsigned int mask = (1u << width) - 1u;
+                for (int p = 0; p < passes; ++p) {
+                    const bool look_up = PLACE && p == 0;
 #pragma unroll
-                    for (int i = 0; i < kLocalItems; ++i) {
+                    for (int i = 0; i < ITEMS; ++i) {
                         if (i >= items) break;
-                        w[i] = words[own + i * 32];
+                        const int at = own + i * 32;
+                        if constexpr (PLACE) w[i] = fresh ? (unsigned int)at : words[at];
+                        else w[i] = !fresh ? words[at] : at < count ? (unsigned int)(K)(key[i] - low) : ~0u;
                     }
+                    if (look_up) {
+                        unsigned int place[(ITEMS + 1) / 2];  // two to a word
+#pragma unroll
+                        for (int i = 0; i < ITEMS; ++i) {
+                            if (i >= items) break;
+                            const unsigned int at = place_of(w[i]);
+                            if (i & 1) place[i / 2] |= at << 16; else place[i / 2] = at;
+                            w[i] = (at < (unsigned int)count ? (unsigned int)((K)(keys[at] - low) >> turn) : ~0u) & (unsigned int)((1ull << length) - 1ull);
+                        }
+                        pass(w, [=](unsigned int v) { return v & mask; },
+                             [&](unsigned int v, int i) { return v >> width << kPlaceBits | (i & 1 ? place[i / 2] >> 16 : place[i / 2] & 0xFFFFu); }, [](uint2) {});
+                    } else {
+                        const int shift = PLACE ? kPlaceBits + (p - 1) * width : turn + p * width;
+                        pass(w, [=](unsigned int v) { return v >> shift & mask; }, [](unsigned int v, int) { return v; }, [](uint2) {});
+                    }
+                    fresh = false;
                 }
-                if (PLACE && p == 0) {
-                    pass(w, [=](unsigned int v) { return v & mask; },
-                         [=](unsigned int v, int i) { return v >> width << kPlaceBits | (unsigned int)(own + i * 32); });
-                } else {
-                    const int shift = PLACE ? kPlaceBits + (p - 1) * width : below + p * width;
-                    pass(w, [=](unsigned int v) { return v >> shift & mask; }, [](unsigned int v, int) { return v; });
-                }
+                turn += length;
             }
             if (!__syncthreads_or(emit(store))) return;
-            if (below > 0) {
-                if (!settle(*this, below, store)) return;
-                all_bits(*this, own, bits);
-            }
+            if (from == 0) break;
+            if (!settle(*this, from, store)) return;
+            from = 0;
         }
         repair(*this);
         emit(store);
-    }
-
-    // All digits from the lowest on.
-    static __device__ __noinline__ void all_bits(LocalSort me, int own, int bits) {
-        unsigned int w[kLocalItems];
-        const int passes = (bits + kLocalDigitBits - 1) / kLocalDigitBits, width = (bits + passes - 1) / passes;
-        const unsigned int mask = (1u << width) - 1u;
-        if (PLACE) {
-#pragma unroll
-            for (int i = 0; i < kLocalItems; ++i) {
-                if (i >= me.items) break;
-                me.words[own + i * 32] = (unsigned int)(own + i * 32);
-            }
-        }
-        for (int p = 0; p < passes; ++p) {
-            const int shift = p * width;
-#pragma unroll
-            for (int i = 0; i < kLocalItems; ++i) {
-                if (i >= me.items) break;
-                w[i] = me.words[own + i * 32];
-            }
-            me.pass(w,
-                    [&](unsigned int v) {
-                        if constexpr (PLACE) return v < (unsigned int)me.count ? (unsigned int)((K)(me.keys[v] - me.low) >> shift) & mask : mask;
-                        else return v >> shift & mask;
-                    },
-                    [](unsigned int v, int) { return v; });
-        }
     }
 };
 

@@ -1349,7 +1349,12 @@ static int sort_common(void *stream, const SortCall &call, int key_dtype, int va
     cudaStream_t s = (cudaStream_t)stream;
     if (g_timed_pass < 0) {
         bool taken = false;
-        const int rc = resident_sort(s, call, kb, value_bytes, xn, xp, temp, temp_bytes, &taken);
+        const SortScratch scratch{(char *)temp + L.off_keys, (char *)temp + L.off_values, L.control_bytes};
+        int rc = block_sort(s, call, kb, value_bytes, xn, xp, temp, &taken);
+        if (rc != B200ALG_OK || taken) return rc;
+        rc = sample_sort(s, call, kb, value_bytes, xn, xp, temp, scratch, &taken);
+        if (rc != B200ALG_OK || taken) return rc;
+        rc = resident_sort(s, call, kb, value_bytes, xn, xp, temp, temp_bytes, &taken);
         if (rc != B200ALG_OK || taken) return rc;
     }
     switch (value_bytes) {

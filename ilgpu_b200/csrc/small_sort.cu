@@ -367,32 +367,12 @@ resident_sort_kernel(SortBuffers<K, V> io, KeyXform<K> xf, TempHeader *hdr, unsi
     }
 }
 
-// Values of a thread's elements of a block (element own + i * 32) to shared memory, eight under way at a time.
-template <typename V>
-__device__ __forceinline__ void load_values(V *values, const V *from, int value_seq, int64_t base, int own, int count, int items) {
-    constexpr int AHEAD = sizeof(V) <= 8 ? 8 : 4;
-#pragma unroll 1
-    for (int first = 0; first < items; first += AHEAD) {
-        V v[AHEAD];
-#pragma unroll
-        for (int i = 0; i < AHEAD; ++i) {
-            const int at = own + (first + i) * 32;
-            if (first + i < items && at < count) {
-                if constexpr (sizeof(V) <= 8) v[i] = value_seq != kSeqNone ? sequence_value<V>(value_seq, base + at) : from[base + at];
-                else v[i] = from[base + at];
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < AHEAD; ++i) {
-            const int at = own + (first + i) * 32;
-            if (first + i < items && at < count) values[at] = v[i];
-        }
-    }
-}
-
 // ---- one block ---------------------------------------------------------------------------
+// 1024 threads of half as many elements: 5000 uint32 keys 14.3 instead of 12.3 us (turning counts into places takes 1800
+// instead of 930 cycles a pass).
+constexpr int kAloneThreads = 512, kAloneItems = kLocalMost / kAloneThreads;
 template <typename K, typename V>
-__global__ void __launch_bounds__(kLocalThreads, 1)
+__global__ void __launch_bounds__(kAloneThreads, 1)
 block_sort_kernel(SortBuffers<K, V> io, KeyXform<K> xf, TempHeader *hdr, int items, int value_seq) {
     constexpr int VB = ValueBytes<V>::value;
     constexpr bool PLACE = by_place<K>(VB != 0);
@@ -408,17 +388,17 @@ block_sort_kernel(SortBuffers<K, V> io, KeyXform<K> xf, TempHeader *hdr, int ite
     const int count = (int)effective_n(io);
     if (tid == 0) hdr->wait_limit_hit = 0u;
 
-    K key[kLocalItems];
+    K key[kAloneItems];
     K low = (K)~(K)0, high = 0;
 #pragma unroll
-    for (int i = 0; i < kLocalItems; ++i) {
+    for (int i = 0; i < kAloneItems; ++i) {
         if (i >= items) break;
         const int at = own + i * 32;
         if (at < count) key[i] = io.in[(int64_t)at * io.stride];
     }
     if constexpr (VB != 0) load_values<V>(values, io.vin, value_seq, 0, own, count, items);
 #pragma unroll
-    for (int i = 0; i < kLocalItems; ++i) {
+    for (int i = 0; i < kAloneItems; ++i) {
         if (i >= items) break;
         const int at = own + i * 32;
         if (at < count) {
@@ -430,51 +410,56 @@ block_sort_kernel(SortBuffers<K, V> io, KeyXform<K> xf, TempHeader *hdr, int ite
         }
     }
     local_range(shared, low, high);
-    const LocalSort<K, PLACE> sort{shared, words, keys, count, items, low, high};
+    const LocalSort<K, PLACE, kAloneItems> sort{shared, words, keys, count, items, low, high};
     K *const out = io.out;
     V *const vout = io.vout;
     const int64_t stride = io.stride;
     sort.run(key, [=](int p, K k, unsigned int word) {
         out[p * stride] = xf.raw(k);
-        if constexpr (VB != 0) vout[p] = values[LocalSort<K, PLACE>::place_of(word)];
+        if constexpr (VB != 0) vout[p] = values[LocalSort<K, PLACE, kAloneItems>::place_of(word)];
     });
 }
 
 // ---- host side ---------------------------------------------------------------------------
 // Which blocks (times on the GPU, us, with the launch and the copy that brings the data):
-//   one       block_sort_kernel, against a cluster, by key bytes / value bytes:
-//                          4500          6000          7500          9000         12000
+//   one       block_sort_kernel, against a cluster, by key bytes / value bytes.  What a cluster takes depends on the
+//             bytes in which keys differ; the line for integers is where identifiers below 2^20 (three bytes) cost the
+//             same either way, floating-point keys differ in all bytes.
+//                          4500          6200          7500          9000         12000
 //                1 / 0    8.4   8.3    8.2   8.4   10.2   8.6   10.3   8.2   12.3   8.8
 //                2 / 0   10.2  12.3   10.3  12.3   12.3  12.3   14.3  12.5   16.4  13.1
 //                1 / 4   12.5  13.2   12.3  13.2   14.4  13.2   16.7  13.3   21.3  24.7
 //                2 / 8   14.7  17.3   15.9  17.6   16.9  17.4   19.1  17.6   22.6  17.4
 //                4 / 0   11.3  16.6   12.3  18.4   14.3  18.5   16.4  20.8   19.1  20.8
+//                        12.1  14.3   14.3  16.4   14.4  16.2   16.4  16.4   19.2  16.4   below 2^20
 //                4 / 4   15.1  23.6   16.6  24.8   19.5  24.3   21.9  25.5   25.7  27.8
+//                        16.3  19.9   18.5  20.3   19.9  20.1   22.5  21.3   26.3  21.3   below 2^20
 //                8 / 0   12.3  29.0   14.4  35.2   16.4  34.7   18.4  37.5   22.5  39.9
+//                        13.3  15.4   16.4  16.4   18.3  16.4   20.5  19.1   24.6  18.6   below 2^20
 //                8 / 4   17.0  42.2   19.1  42.5   21.3  42.3   23.5  46.7   27.7  46.8
+//                        16.4  21.3   20.5  21.3   20.5  21.3   24.5  22.7   29.1  23.4   below 2^20
 //                8 / 8   18.7  41.9   21.2  43.3   25.3  42.4   28.3  46.9    does not fit
 //   cluster   up to 40960 elements (uint32 keys / pairs: 40000: 27 / 33 us against 29 / 32 us with a
 //             grid; 60000: 35 / 43 us against 29 / 33 us);
 //   grid      about 64 blocks until they have 4 keys per thread, then more, up to about the length from
-//             which the passes over tiles are as fast (against those: 700000 uint32 keys / pairs / 8-byte
-//             keys 51 / 61 / 104 us against 59 / 64 / 99; 2^20 uint32 keys 59 against 61 us; 800000 pairs
-//             62 against 59 us).
-constexpr int64_t alone_most(int key_bytes) { return key_bytes == 1 ? 6144 : key_bytes == 2 ? 7680 : kLocalMost; }
+//             which the passes over tiles are as fast (against those: 700000 uint32 keys 51 us against 59;
+//             2^20 uint32 keys 59 against 61 us).
+// Longer ones go by buckets (sample_sort.cu) where that is faster.
+constexpr int64_t alone_most(int key_bytes, int value_bytes, bool floating) {
+    return key_bytes == 1 ? 6144 : key_bytes == 2 ? 7680 : floating ? kLocalMost : key_bytes == 4 ? (value_bytes ? 7168 : 9216) : (value_bytes ? 8192 : 6656);
+}
 constexpr int64_t kClusterMost = 5 * kMaxCluster * kResidentThreads;
 constexpr int64_t kGridMostNarrow = 1 << 20, kGridMost = 3 << 18;
-
-// Bytes of shared memory of an element.
-static int local_bytes(int key_bytes, int value_bytes) { return 4 + value_bytes + (value_bytes || key_bytes == 8 ? key_bytes : 0); }
 
 template <typename K, typename V>
 static int run_block_sort(cudaStream_t s, const SortCall &call, uint64_t xn, uint64_t xp, void *temp, bool *taken) {
     constexpr int VB = ValueBytes<V>::value;
     const int64_t n = call.n;
-    if (n > alone_most(sizeof(K))) return B200ALG_OK;
-    const int threads = n <= kLocalThreads * 2 ? kLocalThreads / 2 : kLocalThreads;  // (1000 keys: 7.2 against 8.1 us)
+    if (n > alone_most(sizeof(K), VB, xn != xp)) return B200ALG_OK;  // (integers' transforms have one constant)
+    const int threads = n <= kAloneThreads * 2 ? kAloneThreads / 2 : kAloneThreads;  // (1000 keys: 7.2 against 8.1 us)
     const int items = (int)ceil_div(n, threads);
     const size_t smem = local_fixed_bytes(threads) + (size_t)threads * items * local_bytes(sizeof(K), VB);
-    if (items > kLocalItems || smem > kResidentSmem) return B200ALG_OK;
+    if (items > kAloneItems || smem > kResidentSmem) return B200ALG_OK;
     auto kernel = block_sort_kernel<K, V>;
     static ContextCache<int> opted_in;
     int done = 0;
@@ -497,9 +482,6 @@ struct ResidentLimits {
 template <typename K, typename V>
 static int run_resident(cudaStream_t s, const SortCall &call, uint64_t xn, uint64_t xp, void *temp, int64_t temp_bytes, bool *taken) {
     constexpr int VB = ValueBytes<V>::value, ITEMS = resident_items(sizeof(K), VB, false), CLUSTER_ITEMS = resident_items(sizeof(K), VB, true);
-    *taken = false;
-    const int rc = run_block_sort<K, V>(s, call, xn, xp, temp, taken);
-    if (rc != B200ALG_OK || *taken) return rc;
     auto kernel = resident_sort_kernel<K, V>;
     static ContextCache<ResidentLimits> cache;
     ResidentLimits lim;
@@ -580,6 +562,30 @@ static int run_resident(cudaStream_t s, const SortCall &call, uint64_t xn, uint6
 }
 
 template <typename V>
+static int block_sort_key(cudaStream_t s, int key_bytes, const SortCall &call, uint64_t xn, uint64_t xp, void *temp, bool *taken) {
+    switch (key_bytes) {
+    case 1: return run_block_sort<uint8_t, V>(s, call, xn, xp, temp, taken);
+    case 2: return run_block_sort<uint16_t, V>(s, call, xn, xp, temp, taken);
+    case 4: return run_block_sort<uint32_t, V>(s, call, xn, xp, temp, taken);
+    case 8: return run_block_sort<uint64_t, V>(s, call, xn, xp, temp, taken);
+    }
+    return B200ALG_UNSUPPORTED;
+}
+
+int block_sort(cudaStream_t s, const SortCall &call, int key_bytes, int value_bytes, uint64_t xn, uint64_t xp, void *temp, bool *taken) {
+    *taken = false;
+    switch (value_bytes) {
+    case 0: return block_sort_key<NoValue>(s, key_bytes, call, xn, xp, temp, taken);
+    case 1: return block_sort_key<uint8_t>(s, key_bytes, call, xn, xp, temp, taken);
+    case 2: return block_sort_key<uint16_t>(s, key_bytes, call, xn, xp, temp, taken);
+    case 4: return block_sort_key<uint32_t>(s, key_bytes, call, xn, xp, temp, taken);
+    case 8: return block_sort_key<uint64_t>(s, key_bytes, call, xn, xp, temp, taken);
+    case 16: return block_sort_key<uint4>(s, key_bytes, call, xn, xp, temp, taken);
+    }
+    return B200ALG_UNSUPPORTED;
+}
+
+template <typename V>
 static int resident_key(cudaStream_t s, int key_bytes, const SortCall &call, uint64_t xn, uint64_t xp, void *temp, int64_t temp_bytes, bool *taken) {
     switch (key_bytes) {
     case 1: return run_resident<uint8_t, V>(s, call, xn, xp, temp, temp_bytes, taken);
@@ -592,6 +598,7 @@ static int resident_key(cudaStream_t s, int key_bytes, const SortCall &call, uin
 
 int resident_sort(cudaStream_t s, const SortCall &call, int key_bytes, int value_bytes, uint64_t xn, uint64_t xp, void *temp,
                   int64_t temp_bytes, bool *taken) {
+    *taken = false;
     switch (value_bytes) {
     case 0: return resident_key<NoValue>(s, key_bytes, call, xn, xp, temp, temp_bytes, taken);
     case 1: return resident_key<uint8_t>(s, key_bytes, call, xn, xp, temp, temp_bytes, taken);

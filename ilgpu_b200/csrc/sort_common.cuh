@@ -91,8 +91,20 @@ struct SortCall {
     bool out_of_place;
 };
 
-// The sort of a view that fits on the GPU's SMs as a whole, in one launch (small_sort.cu).  *taken: false
-// when the view is too long for that.
+// Parts of a sort's temp: the alternate buffers (dense, n elements), and how much lies in front of them.
+struct SortScratch {
+    void *alt_keys, *alt_values;
+    int64_t control_bytes;
+};
+
+// The sort of a view by one partition into buckets that a block holds, in one launch (sample_sort.cu).  *taken:
+// false when the view is too short or too long for that.
+int sample_sort(cudaStream_t s, const SortCall &call, int key_bytes, int value_bytes, uint64_t xor_neg, uint64_t xor_pos, void *temp,
+                const SortScratch &scratch, bool *taken);
+
+// The sort of a view that fits on the GPU's SMs as a whole, in one launch (small_sort.cu): one block's, or, of keys
+// of up to 4 bytes, that of several.  *taken: false when the view is too long for that.
+int block_sort(cudaStream_t s, const SortCall &call, int key_bytes, int value_bytes, uint64_t xor_neg, uint64_t xor_pos, void *temp, bool *taken);
 int resident_sort(cudaStream_t s, const SortCall &call, int key_bytes, int value_bytes, uint64_t xor_neg, uint64_t xor_pos, void *temp,
                   int64_t temp_bytes, bool *taken);
 

@@ -1,0 +1,126 @@
+"""The sort by buckets of a sample: lengths around the places where it begins, where it gets another bucket
+or block and where it ends; distributions that put many equal keys into the sample; strided keys, sequenced
+values; a count on the device; and data that mislead the sample, which are then sorted by digits instead.
+Against a stable host sort."""
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+from ilgpu_b200 import RadixSortOperations, Sequencers
+from ilgpu_b200 import _native as N
+
+pytestmark = pytest.mark.gpu
+
+
+def _keys(rng, dtype, n, kind):
+    if dtype.kind == "f":
+        keys = rng.standard_normal(n).astype(dtype)
+        if kind == "same":
+            keys[:] = 1.5
+        elif kind == "few":
+            keys = np.rint(keys * 2) + 0.0
+        elif kind == "half":
+            keys[rng.random(n) < 0.5] = 0.25
+        elif kind == "sorted":
+            keys.sort()
+        return keys
+    keys = rng.integers(0, 1 << (dtype.itemsize * 8), size=n, dtype=dtype)
+    if kind == "same":
+        keys[:] = 12345
+    elif kind == "few":
+        keys &= dtype.type(3)
+    elif kind == "half":
+        keys[rng.random(n) < 0.5] = 7
+    elif kind == "sorted":
+        keys.sort()
+    return keys
+
+
+def _check(acc, keys, value, descending=False):
+    name = {"f4": "Float", "f8": "Double", "u4": "UInt32", "u8": "UInt64"}[keys.dtype.str[1:]]
+    floating = keys.dtype.kind == "f"
+    op = getattr(RadixSortOperations, ("Descending" if descending else "Ascending") + name)
+    order = np.argsort((-keys if floating else ~keys) if descending else keys, kind="stable")
+    dev = torch.from_numpy(keys).cuda()
+    temp = acc.Allocate1D(acc.ComputeRadixSortPairsTempStorageSize(op, torch.int64, keys.size), torch.int32)
+    if value is None:
+        acc.CreateRadixSort(op, floating)(None, dev, temp)
+    else:
+        vals = torch.from_numpy(np.arange(keys.size).astype(value)).cuda()
+        acc.CreateRadixSortPairs(op, floating)(None, dev, vals, temp)
+        np.testing.assert_array_equal(vals.cpu().numpy(), order.astype(value))
+    acc.CheckDeviceStatus(None, temp)
+    np.testing.assert_array_equal(dev.cpu().numpy(), keys[order])
+
+
+@pytest.mark.parametrize("n", [9729, 12_289, 20_000, 99_999, 100_000, 227_327, 227_329, 400_001, 700_000, 1_091_200, 1_091_201, 1_159_000, 1_546_000])
+@pytest.mark.parametrize("key,value", [(np.float64, None), (np.float64, np.int64), (np.float32, np.int32), (np.uint64, None), (np.uint64, np.uint8),
+                                       (np.uint32, np.int32), (np.uint32, np.int16)])
+@pytest.mark.parametrize("kind", ["full", "same", "few", "half", "sorted"])
+def test_lengths_and_distributions(accelerator, n, key, value, kind):
+    _check(accelerator, _keys(np.random.default_rng(n), np.dtype(key), n, kind), value, descending=kind == "half")
+
+
+def _sampled(n, sms):
+    """Positions that the blocks look at (sample_sort.cu)."""
+    blocks = min(-(-n // 1536), sms)
+    share = -(-n // blocks)
+    at = []
+    for b in range(blocks):
+        lo = min(n, b * share)
+        length = min(n - lo, share)
+        t = np.arange(128)
+        shift = (((b * 128 + t) * 2654435761 & 0xFFFFFFFF) >> 8) % max(1, length // 128)
+        at.append(lo + t * length // 128 + (shift if length >= 128 else 0))
+    return np.concatenate(at)
+
+
+@pytest.mark.parametrize("key,value", [(np.uint64, np.int32), (np.uint64, np.int16), (np.uint32, np.int64)])
+@pytest.mark.parametrize("descending", [False, True])
+def test_misled_sample(accelerator, key, value, descending):
+    n = 300_007
+    rng = np.random.default_rng(5)
+    bits = np.dtype(key).itemsize * 8
+    keys = (rng.integers(0, 1 << (bits - 1), size=n, dtype=key) >> 4) + key(1 << (bits - 1))   # all in one bucket ...
+    at = _sampled(n, torch.cuda.get_device_properties(0).multi_processor_count)
+    keys[at] = rng.integers(0, 1 << 16, size=at.size)                                          # ... but for what is looked at
+    _check(accelerator, keys, value, descending)
+
+
+@pytest.mark.parametrize("n", [100_000, 250_001])
+def test_sequenced_and_strided(accelerator, n):
+    rng = np.random.default_rng(n)
+    keys = rng.integers(0, 1 << 40, size=n, dtype=np.uint64) & 0xFFF0FF
+    op = RadixSortOperations.DescendingUInt64
+    dev, vals = torch.from_numpy(keys).cuda(), torch.zeros(n, dtype=torch.float32, device="cuda")
+    temp = accelerator.Allocate1D(accelerator.ComputeRadixSortPairsTempStorageSize(op, vals.dtype, n), torch.int32)
+    accelerator.CreateRadixSortPairs(op, sequencer=Sequencers)(None, dev, vals, Sequencers.FloatSequencer, temp)
+    np.testing.assert_array_equal(vals.cpu().numpy(), np.argsort(~keys, kind="stable"))
+    keys = rng.standard_normal(n)
+    op = RadixSortOperations.DescendingDouble
+    storage = torch.from_numpy(np.repeat(keys, 3)).cuda()
+    accelerator.CreateRadixSort(op, True)(None, storage[1::3], temp)
+    np.testing.assert_array_equal(storage.cpu().numpy()[1::3], np.sort(keys)[::-1])
+    np.testing.assert_array_equal(storage.cpu().numpy()[::3], keys)
+
+
+def test_count_on_the_device():
+    n = 300_000
+    L, rng = N.lib(), np.random.default_rng(n)
+    keys, values = rng.integers(0, 1 << 60, size=n, dtype=np.uint64), np.arange(n, dtype=np.uint32)
+    p = lambda t: ctypes.c_void_p(t.data_ptr())
+    need = ctypes.c_int64(0)
+    assert L.b200alg_radix_sort_temp_bytes(N.U64, n, 4, ctypes.byref(need)) == N.OK
+    temp = torch.empty(need.value, dtype=torch.uint8, device="cuda")
+    k, v = torch.from_numpy(keys).cuda(), torch.from_numpy(values).cuda()
+    for m in (n, n - 777, 10_001, 147, 1, 0):
+        ok, ov = torch.full((n,), 9, dtype=torch.int64, device="cuda"), torch.full((n,), 9, dtype=torch.int32, device="cuda")
+        count = torch.tensor([m], dtype=torch.int64, device="cuda")
+        assert L.b200alg_radix_sort_out_of_place(None, p(k), p(v), p(ok), p(ov), n, p(count), N.U64, 4, 0, p(temp), need.value) == N.OK
+        torch.cuda.synchronize()
+        order = np.argsort(keys[:m], kind="stable")
+        np.testing.assert_array_equal(ok.cpu().numpy()[:m].view(np.uint64), keys[:m][order])
+        np.testing.assert_array_equal(ov.cpu().numpy()[:m], order)
+        assert (ok.cpu().numpy()[m:] == 9).all() and (ov.cpu().numpy()[m:] == 9).all()
