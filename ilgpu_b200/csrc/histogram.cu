@@ -21,6 +21,8 @@ struct LocParams {
     float lo_f, scale_f, bins_f;
     long long num_bins;
     int last;  // num_bins - 1
+    unsigned int inverse32;        // floor(2^32 / num_bins), all ones for one bin
+    unsigned long long inverse64;  // floor(2^64 / num_bins), likewise
 };
 
 // ---- bin locators ---------------------------------------------------------------------
@@ -39,33 +41,43 @@ template <> struct Locate<float, B200ALG_LOCATOR_EQUAL_WIDTH_CLAMP> {
 template <typename T> struct Locate<T, B200ALG_LOCATOR_EQUAL_WIDTH_CLAMP> {
     static constexpr bool kInRange = true;
     static __device__ __forceinline__ int run(T x, const LocParams &p) {
-        const double t = fmin(fmax(((double)x - p.lo_d) * p.scale_d, 0.0), p.bins_d);
-        return min(__double2int_rz(t), p.last);
+        const double t = ((double)x - p.lo_d) * p.scale_d;
+        // Integers give no NaN, the conversion saturates, and what lies below 0 truncates to 0 or less: clamped as an
+        // integer it saves a minimum and a maximum of doubles, which are several instructions each (2 * 10^8 int32,
+        // 256 bins: 131 instead of 180 us).  Doubles are at the memory's rate either way (249 us against 256).
+        if constexpr (std::is_integral<T>::value) return min(max(__double2int_rz(t), 0), p.last);
+        else return min(__double2int_rz(fmin(fmax(t, 0.0), p.bins_d)), p.last);
     }
 };
+// x mod d by the rounded-down inverse of d: x * floor(2^k / d) / 2^k is less than one below x / d for x below 2^k, so
+// the quotient is right or one too small, and the remainder or the remainder less d is the smaller one (2 * 10^8
+// int32, 256 bins: 123 instead of 137 us with the division of the compiler).
+__device__ __forceinline__ int remainder_of(unsigned int x, const LocParams &p) {
+    const unsigned int d = (unsigned int)p.num_bins, r = x - __umulhi(x, p.inverse32) * d;
+    return (int)min(r, r - d);
+}
+__device__ __forceinline__ int remainder_of(unsigned long long x, const LocParams &p) {
+    const unsigned long long d = (unsigned long long)p.num_bins;
+    const unsigned int r = (unsigned int)(x - __umul64hi(x, p.inverse64) * d);  // below 2 d, hence below 2^32
+    return (int)min(r, r - (unsigned int)d);
+}
 template <> struct Locate<int32_t, B200ALG_LOCATOR_MODULO> {
     static constexpr bool kInRange = true;
-    static __device__ __forceinline__ int run(int32_t x, const LocParams &p) {
-        const int r = x % (int)p.num_bins;
-        return r < 0 ? -r : r;
-    }
+    static __device__ __forceinline__ int run(int32_t x, const LocParams &p) { return remainder_of(x < 0 ? 0u - (unsigned int)x : (unsigned int)x, p); }
 };
 template <> struct Locate<int64_t, B200ALG_LOCATOR_MODULO> {
     static constexpr bool kInRange = true;
     static __device__ __forceinline__ int run(int64_t x, const LocParams &p) {
-        const long long r = (long long)x % p.num_bins;
-        return (int)(r < 0 ? -r : r);
+        return remainder_of(x < 0 ? 0ull - (unsigned long long)x : (unsigned long long)x, p);
     }
 };
 template <> struct Locate<uint32_t, B200ALG_LOCATOR_MODULO> {
     static constexpr bool kInRange = true;
-    static __device__ __forceinline__ int run(uint32_t x, const LocParams &p) { return (int)(x % (unsigned int)p.num_bins); }
+    static __device__ __forceinline__ int run(uint32_t x, const LocParams &p) { return remainder_of((unsigned int)x, p); }
 };
 template <> struct Locate<uint64_t, B200ALG_LOCATOR_MODULO> {
     static constexpr bool kInRange = true;
-    static __device__ __forceinline__ int run(uint64_t x, const LocParams &p) {
-        return (int)(x % (unsigned long long)p.num_bins);
-    }
+    static __device__ __forceinline__ int run(uint64_t x, const LocParams &p) { return remainder_of((unsigned long long)x, p); }
 };
 template <> struct Locate<float, B200ALG_LOCATOR_MODULO> {
     static constexpr bool kInRange = false;
@@ -221,7 +233,7 @@ template <typename T, int LOCATOR> bool use_table(int64_t nb, int64_t n, bool de
 }
 
 template <typename T, int LOCATOR, bool HALVES>
-__global__ void __launch_bounds__(kTableThreads)
+__global__ void __launch_bounds__(kTableThreads, 1)
 histogram_table_kernel(const T *__restrict__ in, int64_t stride, int64_t n, LocParams p, void *bins, int bin_dtype, int *overflow) {
     extern __shared__ __align__(16) unsigned int table[];
     const int nb = (int)p.num_bins;
@@ -265,23 +277,40 @@ histogram_table_kernel(const T *__restrict__ in, int64_t stride, int64_t n, LocP
         static_assert(kTableChunk >= ROUND, "a chunk is whole rounds");
         const int64_t step = (int64_t)gridDim.x * kTableThreads;
         int pending = 0;
-        for (int64_t first = (int64_t)blockIdx.x * kTableThreads; first < nvec; first += NV * step) {
-            const uint4 *from = vin + first + threadIdx.x;
-            V v[NV];
-            if (first + (NV - 1) * step + kTableThreads <= nvec) {  // bounds checks cost as much as the counting
+        auto whole = [&](int64_t first) { return first + (NV - 1) * step + kTableThreads <= nvec; };
+        const int64_t begin = (int64_t)blockIdx.x * kTableThreads;
+        // The next round is on its way while one is counted, unless counting is little (floats, 32-bit counters: 20000
+        // bins 138 us with it, 134 without; 2 * 10^8 int32 into 65536 equal bins 197 with, 228 without).
+        constexpr bool AHEAD = HALVES || !(std::is_same<T, float>::value && LOCATOR == B200ALG_LOCATOR_EQUAL_WIDTH_CLAMP);
+        V v[NV];
+        if (AHEAD && whole(begin)) {
 #pragma unroll
-                for (int k = 0; k < NV; ++k) v[k].u = __ldcs(from + k * step);
+            for (int k = 0; k < NV; ++k) v[k].u = __ldcs(vin + begin + threadIdx.x + k * step);
+        }
+        for (int64_t first = begin; first < nvec; first += NV * step) {
+            if (whole(first)) {  // bounds checks cost as much as the counting
+                const bool more = AHEAD && whole(first + NV * step);
+                const uint4 *ahead = vin + first + NV * step + threadIdx.x;
+                if (!AHEAD) {
 #pragma unroll
-                for (int k = 0; k < NV; ++k)
+                    for (int k = 0; k < NV; ++k) v[k].u = __ldcs(vin + first + threadIdx.x + k * step);
+                }
 #pragma unroll
-                    for (int e = 0; e < VEC; ++e) count(v[k].t[e]);
+                for (int k = 0; k < NV; ++k) {
+                    const V now = v[k];
+                    if (more) v[k].u = __ldcs(ahead + k * step);
+#pragma unroll
+                    for (int e = 0; e < VEC; ++e) count(now.t[e]);
+                }
             } else {
+                const uint4 *from = vin + first + threadIdx.x;
 #pragma unroll 1
                 for (int k = 0; k < NV; ++k)
                     if (first + threadIdx.x + k * step < nvec) {
-                        v[0].u = __ldcs(from + k * step);
+                        V w;
+                        w.u = __ldcs(from + k * step);
 #pragma unroll
-                        for (int e = 0; e < VEC; ++e) count(v[0].t[e]);
+                        for (int e = 0; e < VEC; ++e) count(w.t[e]);
                     }
             }
             if (HALVES) {
@@ -440,6 +469,9 @@ extern "C" int b200alg_histogram(void *stream, const void *in, int64_t stride, i
     p.bins_d = (double)num_bins;
     p.bins_f = (float)num_bins;
     p.last = (int)(num_bins - 1);
+    p.inverse32 = num_bins == 1 ? ~0u : (unsigned int)((1ull << 32) / (unsigned long long)num_bins);
+    // (2^64 - 1) / d is 2^64 / d for every d that does not divide 2^64, and one less for those that do
+    p.inverse64 = ~0ull / (unsigned long long)num_bins + (num_bins > 1 && (num_bins & (num_bins - 1)) == 0 ? 1 : 0);
     // float input computes in float: a range that collapses or overflows there would put every
     // element into an edge bin without a word
     if (locator == B200ALG_LOCATOR_EQUAL_WIDTH_CLAMP && in_dtype == B200ALG_F32 &&
