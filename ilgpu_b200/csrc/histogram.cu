@@ -136,6 +136,7 @@ histogram_smem_kernel(const T *__restrict__ in, int64_t stride, int64_t n, LocPa
     extern __shared__ unsigned int sh[];
     const int nb = (int)p.num_bins;
     for (int i = threadIdx.x; i < nb * replicas; i += kHistThreads) sh[i] = 0u;
+    grid_dependency_wait();
     __syncthreads();
 
     unsigned int *mine = sh + (threadIdx.x & (replicas - 1));
@@ -240,6 +241,7 @@ histogram_table_kernel(const T *__restrict__ in, int64_t stride, int64_t n, LocP
     const int quads = ((HALVES ? (nb + 1) / 2 : nb) + 3) / 4;  // 16-byte pieces of the table
     uint4 *table4 = reinterpret_cast<uint4 *>(table);
     for (int i = threadIdx.x; i < quads; i += kTableThreads) table4[i] = make_uint4(0u, 0u, 0u, 0u);
+    grid_dependency_wait();
     __syncthreads();
     bool of = false;
     auto count = [&](T x) {
@@ -363,6 +365,7 @@ template <typename T, int LOCATOR>
 __global__ void __launch_bounds__(256)
 histogram_global_kernel(const T *__restrict__ in, int64_t stride, int64_t n, LocParams p, void *bins, int bin_dtype,
                         int *overflow) {
+    grid_dependency_wait();
     bool of = false;
     const int64_t step = (int64_t)gridDim.x * blockDim.x;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += step) {
@@ -387,9 +390,9 @@ static int launch_histogram(cudaStream_t s, const void *in, int64_t stride, int6
         const int64_t cap = (int64_t)sm_count() * (2048 / kHistThreads);
         const int blocks = (int)(want < 1 ? 1 : (want > cap ? cap : want));
         if (stride == 1)
-            histogram_smem_kernel<T, LOCATOR, true><<<blocks, kHistThreads, smem, s>>>((const T *)in, 1, n, p, bins, bin_dtype, (int *)overflow, replicas);
+            B200ALG_CUDA_TRY(launch_dependent(histogram_smem_kernel<T, LOCATOR, true>, dim3(blocks), dim3(kHistThreads), smem, s, (const T *)in, 1, n, p, bins, bin_dtype, (int *)overflow, replicas));
         else
-            histogram_smem_kernel<T, LOCATOR, false><<<blocks, kHistThreads, smem, s>>>((const T *)in, stride, n, p, bins, bin_dtype, (int *)overflow, replicas);
+            B200ALG_CUDA_TRY(launch_dependent(histogram_smem_kernel<T, LOCATOR, false>, dim3(blocks), dim3(kHistThreads), smem, s, (const T *)in, stride, n, p, bins, bin_dtype, (int *)overflow, replicas));
     } else if (table) {
         const bool halves = nb * 4 > kTableBytes;
         const size_t smem = (size_t)round_up(halves ? (nb + 1) / 2 * 4 : nb * 4, 16);
@@ -400,16 +403,15 @@ static int launch_histogram(cudaStream_t s, const void *in, int64_t stride, int6
         const unsigned int cluster = big ? 2 : kTableMaxCluster;
         static ContextCache<int> resident[4];
         int blocks = 0;
-        cudaLaunchConfig_t cfg = {};
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = cluster;
-        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-        cfg.blockDim = dim3(kTableThreads);
-        cfg.stream = s;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
         if (!resident[halves * 2 + big].find(&blocks)) {
+            cudaLaunchConfig_t cfg = {};
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = cluster;
+            attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+            cfg.blockDim = dim3(kTableThreads);
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
             B200ALG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTableBytes));
             cfg.gridDim = dim3(cluster);
             cfg.dynamicSmemBytes = kTableBytes;
@@ -419,14 +421,12 @@ static int launch_histogram(cudaStream_t s, const void *in, int64_t stride, int6
             blocks = clusters * (int)cluster;
             resident[halves * 2 + big].store(blocks);
         }
-        cfg.gridDim = dim3(blocks);
-        cfg.dynamicSmemBytes = smem;
-        B200ALG_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, (const T *)in, stride, n, p, bins, bin_dtype, (int *)overflow));
+        B200ALG_CUDA_TRY(launch_dependent_cluster(kernel, dim3(blocks), dim3(kTableThreads), smem, s, cluster, (const T *)in, stride, n, p, bins, bin_dtype, (int *)overflow));
     } else {
         int64_t want = ceil_div(n, 256 * 4);
         const int64_t cap = (int64_t)sm_count() * 8;
         const int blocks = (int)(want < 1 ? 1 : (want > cap ? cap : want));
-        histogram_global_kernel<T, LOCATOR><<<blocks, 256, 0, s>>>((const T *)in, stride, n, p, bins, bin_dtype, (int *)overflow);
+        B200ALG_CUDA_TRY(launch_dependent(histogram_global_kernel<T, LOCATOR>, dim3(blocks), dim3(256), 0, s, (const T *)in, stride, n, p, bins, bin_dtype, (int *)overflow));
     }
     B200ALG_LAUNCH_CHECK();
     return B200ALG_OK;

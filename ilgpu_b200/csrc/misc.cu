@@ -37,12 +37,16 @@ int sm_count() {
 
 template <typename T>
 __global__ void __launch_bounds__(256) fill_kernel(T *view, int64_t stride, int64_t n, T value) {
+    grid_dependency_release();
+    grid_dependency_wait();
     const int64_t step = (int64_t)gridDim.x * blockDim.x;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += step) view[i * stride] = value;
 }
 
 template <typename T>
 __global__ void __launch_bounds__(256) sequence_kernel(T *view, int64_t n, T start, T step_value) {
+    grid_dependency_release();
+    grid_dependency_wait();
     const int64_t step = (int64_t)gridDim.x * blockDim.x;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += step)
         view[i] = (T)(start + (T)i * step_value);
@@ -99,11 +103,11 @@ extern "C" int b200alg_initialize(void *stream, void *view, int64_t stride, int6
     cudaStream_t s = (cudaStream_t)stream;
     const int g = grid_for(n);
     switch (elem_bytes) {
-    case 1: fill_kernel<uint8_t><<<g, 256, 0, s>>>((uint8_t *)view, stride, n, *(const uint8_t *)value); break;
-    case 2: fill_kernel<uint16_t><<<g, 256, 0, s>>>((uint16_t *)view, stride, n, *(const uint16_t *)value); break;
-    case 4: fill_kernel<uint32_t><<<g, 256, 0, s>>>((uint32_t *)view, stride, n, *(const uint32_t *)value); break;
-    case 8: fill_kernel<uint64_t><<<g, 256, 0, s>>>((uint64_t *)view, stride, n, *(const uint64_t *)value); break;
-    case 16: fill_kernel<uint4><<<g, 256, 0, s>>>((uint4 *)view, stride, n, *(const uint4 *)value); break;
+    case 1: B200ALG_CUDA_TRY(launch_dependent(fill_kernel<uint8_t>, dim3(g), dim3(256), 0, s, (uint8_t *)view, stride, n, *(const uint8_t *)value)); break;
+    case 2: B200ALG_CUDA_TRY(launch_dependent(fill_kernel<uint16_t>, dim3(g), dim3(256), 0, s, (uint16_t *)view, stride, n, *(const uint16_t *)value)); break;
+    case 4: B200ALG_CUDA_TRY(launch_dependent(fill_kernel<uint32_t>, dim3(g), dim3(256), 0, s, (uint32_t *)view, stride, n, *(const uint32_t *)value)); break;
+    case 8: B200ALG_CUDA_TRY(launch_dependent(fill_kernel<uint64_t>, dim3(g), dim3(256), 0, s, (uint64_t *)view, stride, n, *(const uint64_t *)value)); break;
+    case 16: B200ALG_CUDA_TRY(launch_dependent(fill_kernel<uint4>, dim3(g), dim3(256), 0, s, (uint4 *)view, stride, n, *(const uint4 *)value)); break;
     default: return B200ALG_UNSUPPORTED;
     }
     B200ALG_LAUNCH_CHECK();
@@ -118,10 +122,10 @@ extern "C" int b200alg_sequence(void *stream, void *view, int64_t n, int dtype, 
     switch (dtype) {
     case B200ALG_I32: case B200ALG_U32:
         if ((uintptr_t)view % 4) return B200ALG_MISALIGNED;
-        sequence_kernel<uint32_t><<<g, 256, 0, s>>>((uint32_t *)view, n, (uint32_t)start, (uint32_t)step); break;
+        B200ALG_CUDA_TRY(launch_dependent(sequence_kernel<uint32_t>, dim3(g), dim3(256), 0, s, (uint32_t *)view, n, (uint32_t)start, (uint32_t)step)); break;
     case B200ALG_I64: case B200ALG_U64:
         if ((uintptr_t)view % 8) return B200ALG_MISALIGNED;
-        sequence_kernel<uint64_t><<<g, 256, 0, s>>>((uint64_t *)view, n, (uint64_t)start, (uint64_t)step); break;
+        B200ALG_CUDA_TRY(launch_dependent(sequence_kernel<uint64_t>, dim3(g), dim3(256), 0, s, (uint64_t *)view, n, (uint64_t)start, (uint64_t)step)); break;
     default: return B200ALG_UNSUPPORTED;
     }
     B200ALG_LAUNCH_CHECK();

@@ -53,6 +53,7 @@ template <int OP> struct AtomicApply<double, OP> {
 // one: its blocks fold their share of the input while this kernel runs and wait for it only
 // before they combine into out[0].
 template <typename T> __global__ void set_scalar_kernel(T *out, T v) {
+    grid_dependency_wait();  // what the input comes from has completed when the reduction may start
     grid_dependency_release();
     *out = v;
 }
@@ -139,6 +140,7 @@ __global__ void __launch_bounds__(THREADS) reduce_dense_kernel(const T *__restri
 constexpr int kOneBlockThreads = 1024;
 template <typename T, int OP>
 __global__ void __launch_bounds__(kOneBlockThreads) reduce_block_kernel(const T *__restrict__ in, int64_t stride, int64_t n, T *out) {
+    grid_dependency_wait();
     T r = Op<T, OP>::identity();
     if (stride == 1) {
         r = fold_dense<T, OP, kOneBlockThreads>(in, n);
@@ -167,12 +169,10 @@ static int launch_reduce(cudaStream_t s, const void *in, int64_t stride, int64_t
     constexpr int THREADS = 256;
     constexpr int VEC = 16 / sizeof(T);
     if (fits_block(n, stride, sizeof(T))) {
-        reduce_block_kernel<T, OP><<<1, kOneBlockThreads, 0, s>>>((const T *)in, stride, n, (T *)out);
-        B200ALG_LAUNCH_CHECK();
+        B200ALG_CUDA_TRY(launch_dependent(reduce_block_kernel<T, OP>, dim3(1), dim3(kOneBlockThreads), 0, s, (const T *)in, stride, n, (T *)out));
         return B200ALG_OK;
     }
-    set_scalar_kernel<T><<<1, 1, 0, s>>>((T *)out, Op<T, OP>::identity());
-    B200ALG_LAUNCH_CHECK();
+    B200ALG_CUDA_TRY(launch_dependent(set_scalar_kernel<T>, dim3(1), dim3(1), 0, s, (T *)out, Op<T, OP>::identity()));
     const int max_blocks = sm_count() * 8;
     if (stride == 1) {
         int64_t want = ceil_div(n, (int64_t)THREADS * VEC * 4);

@@ -508,6 +508,7 @@ scan_short_kernel(const T *in, int64_t in_stride, T *out, int64_t out_stride, in
     __shared__ T block_total;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int first = (int)blockIdx.x * kShortTile + tid * kShortItems;
+    grid_dependency_wait();
     if (blockIdx.x == 0 && tid == 0) hdr->wait_limit_hit = 0u;
     T v[kShortItems];
     const bool whole = vectors && first >= lead && first + kShortItems <= n;
@@ -603,18 +604,8 @@ static int launch_scan(cudaStream_t s, const void *in, int64_t in_stride, void *
     if (n_arg <= kShortCluster * kShortTile) {
         int blocks = 1;
         while (blocks * kShortTile < n_arg) blocks *= 2;
-        cudaLaunchConfig_t cfg = {};
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = blocks;
-        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-        cfg.gridDim = dim3(blocks);
-        cfg.blockDim = dim3(kShortThreads);
-        cfg.stream = s;
-        cfg.attrs = attr;
-        cfg.numAttrs = blocks > 1 ? 1 : 0;
-        B200ALG_CUDA_TRY(cudaLaunchKernelEx(&cfg, scan_short_kernel<T, OP, INCLUSIVE>, in_t, in_stride, out_t, out_stride, (int)n_arg, lead, alike,
-                                            carry_t, hdr));
+        B200ALG_CUDA_TRY(launch_dependent_cluster(scan_short_kernel<T, OP, INCLUSIVE>, dim3(blocks), dim3(kShortThreads), 0, s, (unsigned int)blocks, in_t,
+                                                  in_stride, out_t, out_stride, (int)n_arg, lead, alike, carry_t, hdr));
         return B200ALG_OK;
     }
     bool launched = false;

@@ -77,6 +77,7 @@ resident_sort_kernel(SortBuffers<K, V> io, KeyXform<K> xf, TempHeader *hdr, unsi
     static_assert(sizeof(ResidentWords) <= 1024, "room for the small words");
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    grid_dependency_wait();
     const int64_t n = effective_n(io);
     const int64_t base = (int64_t)blockIdx.x * tile;
     const int valid = (int)(n - base < 0 ? 0 : (n - base < tile ? n - base : tile));
@@ -536,14 +537,16 @@ static int run_resident(cudaStream_t s, const SortCall &call, uint64_t xn, uint6
     TempHeader *hdr = (TempHeader *)temp;
     const size_t smem = resident_smem(sizeof(K), VB, meeting == kInCluster, items);
     cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     cfg.gridDim = dim3(blocks);
     cfg.blockDim = dim3(kResidentThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = meeting == kInCluster ? 2 : 1;
     if (meeting == kInCluster) {
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
         attr[0].id = cudaLaunchAttributeClusterDimension;
         attr[0].val.clusterDim.x = blocks;
         attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
