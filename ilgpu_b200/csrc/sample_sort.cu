@@ -385,9 +385,9 @@ sample_sort_kernel(SampleSort<K, V> a) {
                 part.to[(int64_t)at * part.to_stride] = part.raw_out ? a.xf.raw(bits) : bits;
                 if constexpr (VB != 0) part.vto[at] = b.values[place];
             }
-            cg::this_grid().sync();
-            if (part.shift < 0) break;
         }
+        cg::this_grid().sync();  // the elements have been stored, and all blocks have read the counts
+        if (!too_large && part.shift < 0) break;
         // All digits of eight bits, lowest first: from the input to the alternate buffer, to the output, and so on.
         static_assert(sizeof(K) % 2 == 0, "the last pass writes the output view");
         const int pass = part.shift < 0 ? 0 : part.shift / 8 + 1;
