@@ -12,8 +12,9 @@
 //   - With values or 8-byte keys an element travels as a word: its place in the block (14 bits) below the
 //     digits that are still to come (18 bits after the first pass).  Keys and values stay where they were
 //     loaded and are fetched by place in the end.  Keys of up to four bytes alone travel as themselves.
-//   - The counts of two digits share a word (a block holds fewer than 2^14 elements), which halves what turning counts into places reads and writes.  The atomic that returns
-//     costs the same: 3.53 against 3.57 cycles on random digits.
+//   - The counts of two digits share a word (a block holds fewer than 2^14 elements), which halves what turning
+//     counts into places reads and writes.  The atomic that returns costs the same: 3.53 against 3.57 cycles on
+//     random digits.
 //
 // Order.  As in the digit pass, lanes that meet in one word are not promised any order; the comparison of
 // whole keys (and of places, where they are equal) sees to that as well.
@@ -180,6 +181,21 @@ template <typename K, bool PLACE, int ITEMS> struct LocalSort {
         if constexpr (PLACE) return key_a > key_b || (key_a == key_b && place_of(a) > place_of(b));
         else return a > b;
     }
+    // The key of a place past the last element (word ~0 where words are keys): behind all others.
+    __device__ __forceinline__ K key_or_most(unsigned int word) const {
+        if constexpr (PLACE) return place_of(word) < (unsigned int)count ? keys[place_of(word)] : (K)~(K)0;
+        else return key_at(word);
+    }
+    // Whether an element came out behind a place that holds none: in a tie of the last digits a warp's lanes past
+    // the last element, served before the others, would push it out of what emit looks at.  (Not taking part would
+    // be a test per element and pass: 9000 keys 18.5 against 16.5 us.)
+    __device__ __forceinline__ bool strays() const {
+        bool any = false;
+        for (int p = count + (int)threadIdx.x; p < items * (int)blockDim.x; p += (int)blockDim.x)
+            any |= PLACE ? place_of(words[p]) < (unsigned int)count : words[p] != ~0u;
+        if (any) atomicAdd(s.found, blockDim.x + 1u);  // more than settle takes
+        return any;
+    }
 
     // counted(c): c.x and c.y are the block's count and first place of digits threadIdx.x % 256 (lower half) and
     // 256 + threadIdx.x % 256 (upper half).
@@ -208,16 +224,16 @@ template <typename K, bool PLACE, int ITEMS> struct LocalSort {
     // What is rarely needed stays out of line and takes copies: the address of this object, or of what `store`
     // holds, in the hands of a function would keep them all in memory (pairs of 5000: 28600 cycles instead of 18000).
 
-    // Neighbours that are the wrong way round change places until none are.
+    // Neighbours that are the wrong way round change places until none are (words past the last element included).
     static __device__ __noinline__ void repair(LocalSort me) {
-        const int threads = (int)blockDim.x;
+        const int threads = (int)blockDim.x, all = me.items * threads;
         bool again = true;
-        for (int round = 0; again && round < me.count; ++round) {
+        for (int round = 0; again && round < all; ++round) {
             bool moved = false;
             for (int odd = 0; odd < 2; ++odd) {
-                for (int p = 2 * (int)threadIdx.x + odd; p + 1 < me.count; p += 2 * threads) {
+                for (int p = 2 * (int)threadIdx.x + odd; p + 1 < all; p += 2 * threads) {
                     const unsigned int a = me.words[p], b = me.words[p + 1];
-                    if (!wrong(me.key_at(a), a, me.key_at(b), b)) continue;
+                    if (!wrong(me.key_or_most(a), a, me.key_or_most(b), b)) continue;
                     me.words[p] = b;
                     me.words[p + 1] = a;
                     moved = true;
@@ -343,7 +359,7 @@ template <typename K, bool PLACE, int ITEMS> struct LocalSort {
 #pragma unroll
                 for (int i = 0; i < ITEMS; ++i) {
                     if (i >= items) break;
-                    words[own + i * 32] = PLACE ? (unsigned int)(own + i * 32) : 0u;
+                    words[own + i * 32] = PLACE ? (unsigned int)(own + i * 32) : own + i * 32 < count ? 0u : ~0u;
                 }
                 __syncthreads();
             }
@@ -380,7 +396,8 @@ template <typename K, bool PLACE, int ITEMS> struct LocalSort {
                 }
                 turn += length;
             }
-            if (!__syncthreads_or(emit(store))) return;
+            const bool stray = strays();
+            if (!__syncthreads_or(emit(store) || stray)) return;
             if (from == 0) break;
             if (!settle(*this, from, store)) return;
             from = 0;
