@@ -16,9 +16,9 @@
 //
 // The blocks meet four times, which is 5 us; 10^6 uint64 keys spend 9 us on the splitters, 13 on the partition and
 // 14 on the sort (512 threads a block; 1024 were slower below 10^6 elements, 35 against 29 us for 13000: code that
-// runs once is fetched once per launch, and more warps do not fetch it faster).  A bucket that came out larger than a block holds (the sample misled: not seen
-// with any distribution) is known to all blocks before anything has been written; then they sort by digits of
-// eight bits instead, with the same partition.
+// runs once is fetched once per launch, and more warps do not fetch it faster).  A bucket that came out larger than
+// a block holds (the sample misled: keys made for it, no distribution) is known to all blocks before anything has
+// been written; then they sort by digits of eight bits instead, with the same partition.
 #include "local_sort.cuh"
 
 #include <cooperative_groups.h>
@@ -377,13 +377,24 @@ sample_sort_kernel(SampleSort<K, V> a) {
         if (tid == 0) m->start[kPartitionDigits] = b.n;
         __syncthreads();
         if (!too_large) {
+            // (where keys alone go to buckets of the sample, any order will do: the buckets are sorted)
+            const bool in_order = VB != 0 || part.shift >= 0;
+            for (;;) {
+                bool bad = false;
 #pragma unroll 4
-            for (int p = tid; p < len; p += kSampleThreads) {
-                const unsigned int word = b.words[p], place = word & ((1u << kPlaceBits) - 1u);
-                const unsigned int at = m->first[word >> kPlaceBits] + p;
-                const K bits = b.keys[place];
-                part.to[(int64_t)at * part.to_stride] = part.raw_out ? a.xf.raw(bits) : bits;
-                if constexpr (VB != 0) part.vto[at] = b.values[place];
+                for (int p = tid; p < len; p += kSampleThreads) {
+                    const unsigned int word = b.words[p], place = word & ((1u << kPlaceBits) - 1u);
+                    const unsigned int at = m->first[word >> kPlaceBits] + p;
+                    const K bits = b.keys[place];
+                    if (in_order) bad |= p + 1 < len && b.words[p + 1] < word;
+                    part.to[(int64_t)at * part.to_stride] = part.raw_out ? a.xf.raw(bits) : bits;
+                    if constexpr (VB != 0) part.vto[at] = b.values[place];
+                }
+                // Lanes that met in one counter were served in another order than theirs: what is in which bucket is
+                // right, the order inside is put right and the elements are stored again.
+                if (!__syncthreads_or(bad)) break;
+                using Words = LocalSort<unsigned int, false, kSampleItems>;
+                Words::repair(Words{b.shared, b.words, nullptr, len, items, 0u, 0u});
             }
         }
         cg::this_grid().sync();  // the elements have been stored, and all blocks have read the counts
