@@ -474,6 +474,13 @@ def run_profile_case(case: str) -> None:
         for r in range(3):
             keys = synthetic.uniform_uint32_device(n, SEED + r, "cuda")
             sort(None, keys, temp)
+    elif case == "sort_buckets":  # 8-byte keys whose sort moves them between blocks once
+        n = 1_000_000
+        temp = acc.Allocate1D(acc.ComputeRadixSortTempStorageSize(Sorts.AscendingDouble, n), torch.int32)
+        sort = acc.CreateRadixSort(Sorts.AscendingDouble, True)
+        for r in range(3):
+            keys = synthetic.normal_float32_device(n, SEED + r, "cuda").to(torch.float64).mul_(1.0 / 3.0)
+            sort(None, keys, temp)
     elif case == "unique":       # runs of four on average
         n = 50_000_017
         starts = synthetic.uniform_float32_device(n, 6, "cuda").lt_(0.25)
@@ -892,7 +899,7 @@ def main() -> None:
     ap.add_argument("--warmup", type=int, default=5)
     ap.add_argument("--impl", default="b200", choices=["b200", "reference"])
     ap.add_argument("--no-secondary", action="store_true", help="skip the scan / reduce / histogram figures")
-    ap.add_argument("--profile-case", choices=["sort", "sort_pairs", "sort_small", "partition", "scan", "reduce", "histogram", "histogram_bins", "unique"],
+    ap.add_argument("--profile-case", choices=["sort", "sort_pairs", "sort_small", "sort_buckets", "partition", "scan", "reduce", "histogram", "histogram_bins", "unique"],
                     help="run a few launches of one primitive on a small case and exit (the target of ncu captures)")
     args = ap.parse_args()
     if args.warmup < 3:
