@@ -568,7 +568,7 @@ def run_native(args) -> None:
 
         def step_fn(i):
             sort(None, bufs[i], temp)
-        launches_per_step = 6   # digit histograms (and offsets), 4 digit passes, copy-back (exits at once)
+        launches_per_step = 7   # clear, digit histograms (and offsets), 4 digit passes, copy-back (exits at once)
         result_of = lambda i: bufs[i]
     else:
         from ilgpu_b200.multi_gpu import ShardedAlgorithms

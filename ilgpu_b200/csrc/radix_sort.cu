@@ -124,6 +124,17 @@ constexpr int kHistoThreads = 1024;
 // short inputs use 8 replicas and two blocks per SM instead.
 constexpr int kHistoMaxSmem = 128 * 1024;
 
+// What the kernels of a sort count and publish in starts at zero.  A kernel and not a memset, so that it is launched
+// while the kernel before it drains, and the histogram, which waits only before it adds to what is cleared here,
+// with it.  It waits before it lets the histogram start: the keys are there by then.  1500001 int32 keys with the copy
+// that brings them 67.9 us with a memset, 64.5 with this; 2^26 uint32 832.4 and 827.6.
+__global__ void __launch_bounds__(256) sort_clear_kernel(uint4 *words, int64_t count) {
+    grid_dependency_wait();
+    grid_dependency_release();
+    const int64_t step = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += step) words[i] = make_uint4(0u, 0u, 0u, 0u);
+}
+
 template <typename K, int RSHIFT>
 __global__ void __launch_bounds__(kHistoThreads)
 sort_histogram_kernel(const K *__restrict__ keys, int64_t stride, int64_t n, const long long *n_device, KeyXform<K> xf,
@@ -180,6 +191,7 @@ sort_histogram_kernel(const K *__restrict__ keys, int64_t stride, int64_t n, con
     } else {
         for (int64_t i = gtid; i < n; i += step) count(keys[i * stride]);
     }
+    grid_dependency_wait();  // the histogram has been cleared
     __syncthreads();
     for (int i = threadIdx.x; i < P * kRadix; i += kHistoThreads) {
         unsigned int c = 0;
@@ -1004,7 +1016,11 @@ static int run_passes(cudaStream_t s, const SortCall &call, const KeyXform<K> &x
     io.n_device = call.n_device;
 
     // the published words of the first pass; every pass clears those of the next
-    B200ALG_CUDA_TRY(cudaMemsetAsync(temp, 0, (size_t)(L.off_status + L.half_bytes), s));
+    {
+        const int64_t words = ceil_div(L.off_status + L.half_bytes, 16);
+        const int64_t want = ceil_div(words, 256 * 4), cap = (int64_t)sm_count() * 4;
+        B200ALG_CUDA_TRY(launch_dependent(sort_clear_kernel, dim3((unsigned)(want < cap ? want : cap)), dim3(256), 0, s, (uint4 *)temp, words));
+    }
     {
         const int64_t per_block = (int64_t)kHistoThreads * (16 / sizeof(K)) * 2;
         int64_t want = ceil_div(n, per_block);
@@ -1024,10 +1040,11 @@ static int run_passes(cudaStream_t s, const SortCall &call, const KeyXform<K> &x
             }
         }
         if (big)
-            sort_histogram_kernel<K, kBigShift><<<blocks, kHistoThreads, histo_smem, s>>>(io.in, io.stride, n, io.n_device, xf, ghist, gbase, hdr, call.out_of_place ? 1 : 0);
+            B200ALG_CUDA_TRY(launch_dependent(sort_histogram_kernel<K, kBigShift>, dim3(blocks), dim3(kHistoThreads), histo_smem, s, io.in, io.stride, n,
+                                              io.n_device, xf, ghist, gbase, hdr, call.out_of_place ? 1 : 0));
         else
-            sort_histogram_kernel<K, 3><<<blocks, kHistoThreads, histo_smem, s>>>(io.in, io.stride, n, io.n_device, xf, ghist, gbase, hdr, call.out_of_place ? 1 : 0);
-        B200ALG_LAUNCH_CHECK();
+            B200ALG_CUDA_TRY(launch_dependent(sort_histogram_kernel<K, 3>, dim3(blocks), dim3(kHistoThreads), histo_smem, s, io.in, io.stride, n,
+                                              io.n_device, xf, ghist, gbase, hdr, call.out_of_place ? 1 : 0));
     }
     for (int p = 0; p < L.passes; ++p) {
         XF pass_xf;

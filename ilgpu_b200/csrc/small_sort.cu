@@ -443,8 +443,8 @@ block_sort_kernel(SortBuffers<K, V> io, KeyXform<K> xf, TempHeader *hdr, int ite
 //   cluster   up to 40960 elements (uint32 keys / pairs: 40000: 27 / 33 us against 29 / 32 us with a
 //             grid; 60000: 35 / 43 us against 29 / 33 us);
 //   grid      about 64 blocks until they have 4 keys per thread, then more, up to about the length from
-//             which the passes over tiles are as fast (against those: 700000 uint32 keys 51 us against 59;
-//             2^20 uint32 keys 59 against 61 us).
+//             which the passes over tiles are as fast (against those: 2^20 uint32 keys 61.5 us against 59.6, keys
+//             below 2^20 47.2 against 54.1; 786432 uint32 keys + 8 bytes 51.3 against 55.5).
 // Longer ones go by buckets (sample_sort.cu) where that is faster.
 constexpr int64_t alone_most(int key_bytes, int value_bytes, bool floating) {
     return key_bytes == 1 ? 6144 : key_bytes == 2 ? 7680 : floating ? kLocalMost : key_bytes == 4 ? (value_bytes ? 7168 : 9216) : (value_bytes ? 8192 : 6656);

@@ -534,11 +534,11 @@ class ShardedAlgorithms:
 
     def sort_launches_per_step(self, operation: RadixSortOperation) -> int:
         """Kernels of the library launched by one SortKeys call: the sample sort and the final
-        sort (histogram, one pass per key byte, copy-back each) and the partition
+        sort (clear, histogram, one pass per key byte, copy-back each) and the partition
         (bucket histogram, offsets, count export, one pass)."""
         passes = operation.dtype.itemsize
         if self._native():
             # samples, collect, rank + pick of the splitters, row of the size matrix, plan, 3 barriers;
-            # the final sort (histogram, passes, copy-back); bucket sizes (3) and the partition (2)
-            return 9 + (2 + passes) + 5
-        return 2 * (2 + passes) + 4
+            # the final sort (clear, histogram, passes, copy-back); bucket sizes (3) and the partition (2)
+            return 9 + (3 + passes) + 5
+        return 2 * (3 + passes) + 4
