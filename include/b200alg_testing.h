@@ -36,6 +36,11 @@ int b200alg_testing_time_sort_mg(void *comm, void *stream, const void *keys, con
                                  int key_dtype, int value_bytes, int order, void *out_keys, void *out_values,
                                  int64_t out_capacity, int64_t *out_count, float *phase_ms);
 
+/* The 32-bit word of a sort's temp that tells, when the sort went by buckets of a sample (8-byte keys, and 4-byte
+ * keys with values, of some 10^4 to 1.5 * 10^6 elements), how often its elements were moved by a digit: 0 when they
+ * did go by buckets, the number of bytes in which keys differ where these are few. */
+#define B200ALG_TESTING_SORT_MOVES_WORD 58
+
 #ifdef __cplusplus
 }
 #endif

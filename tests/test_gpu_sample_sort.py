@@ -1,6 +1,7 @@
 """The sort by buckets of a sample: lengths around the places where it begins, where it gets another bucket
 or block and where it ends; distributions that put many equal keys into the sample; strided keys, sequenced
 values; a count on the device; and data that mislead the sample, which are then sorted by digits instead.
+Keys that differ in a few bytes only, which go by these from the start, and keys that only look as if they did.
 Against a stable host sort."""
 import ctypes
 
@@ -38,13 +39,18 @@ def _keys(rng, dtype, n, kind):
     return keys
 
 
+MOVES = 58  # B200ALG_TESTING_SORT_MOVES_WORD
+
+
 def _check(acc, keys, value, descending=False):
+    """The number of times that the elements were moved by a digit."""
     name = {"f4": "Float", "f8": "Double", "u4": "UInt32", "u8": "UInt64"}[keys.dtype.str[1:]]
     floating = keys.dtype.kind == "f"
     op = getattr(RadixSortOperations, ("Descending" if descending else "Ascending") + name)
     order = np.argsort((-keys if floating else ~keys) if descending else keys, kind="stable")
     dev = torch.from_numpy(keys).cuda()
     temp = acc.Allocate1D(acc.ComputeRadixSortPairsTempStorageSize(op, torch.int64, keys.size), torch.int32)
+    temp[MOVES] = -1
     if value is None:
         acc.CreateRadixSort(op, floating)(None, dev, temp)
     else:
@@ -53,6 +59,7 @@ def _check(acc, keys, value, descending=False):
         np.testing.assert_array_equal(vals.cpu().numpy(), order.astype(value))
     acc.CheckDeviceStatus(None, temp)
     np.testing.assert_array_equal(dev.cpu().numpy(), keys[order])
+    return int(temp[MOVES])
 
 
 @pytest.mark.parametrize("n", [9729, 12_289, 20_000, 99_999, 100_000, 227_327, 227_329, 400_001, 700_000, 1_091_200, 1_091_201, 1_159_000, 1_546_000])
@@ -86,7 +93,59 @@ def test_misled_sample(accelerator, key, value, descending):
     keys = (rng.integers(0, 1 << (bits - 1), size=n, dtype=key) >> 4) + key(1 << (bits - 1))   # all in one bucket ...
     at = _sampled(n, torch.cuda.get_device_properties(0).multi_processor_count)
     keys[at] = rng.integers(0, 1 << 16, size=at.size)                                          # ... but for what is looked at
-    _check(accelerator, keys, value, descending)
+    assert _check(accelerator, keys, value, descending) == np.dtype(key).itemsize   # by every digit
+
+
+def _looked(n):
+    """Positions that every block looks at (sample_sort.cu)."""
+    j = np.arange(64, dtype=np.uint64)
+    return j * np.uint64(n) // np.uint64(64) + (np.uint64(n // 64) * (j * np.uint64(2654435761) & np.uint64(0xFFFFFFFF)) >> np.uint64(32))
+
+
+def _with_bytes(rng, dtype, n, at):
+    """Keys that differ in these bytes, also the first two; the other bytes are the same in all."""
+    keys = np.full(n, 0x1122334455667788 & ((1 << 8 * np.dtype(dtype).itemsize) - 1), dtype=dtype)
+    for p in at:
+        digit = rng.integers(0, 256, size=n).astype(dtype)
+        digit[:2] = 0, 255
+        keys ^= digit << dtype(8 * p)
+    return keys
+
+
+@pytest.mark.parametrize("n", [100_000, 227_329, 800_000, 1_091_201])
+@pytest.mark.parametrize("key,value,at", [(np.uint64, np.int32, a) for a in [(), (0,), (7,), (2, 5), (0, 1, 6), (0, 1, 2, 3), (1, 3, 4, 6, 7)]] +
+                                         [(np.uint32, np.int64, a) for a in [(), (0,), (3,), (1, 2), (0, 1, 2), (0, 1, 2, 3)]])
+def test_few_bytes(accelerator, n, key, value, at):
+    for descending in (False, True):
+        moves = _check(accelerator, _with_bytes(np.random.default_rng(n), key, n, at), value, descending)
+        assert moves == (max(1, len(at)) if len(at) <= 3 else 0)
+
+
+@pytest.mark.parametrize("n", [12_289, 16_384, 40_960, 40_961, 150_001])
+@pytest.mark.parametrize("value", [None, np.int32, np.int64])
+@pytest.mark.parametrize("most,moves", [(2, 2), (256, 3), (1 << 19, 0)])
+def test_whole_numbers(accelerator, n, value, most, moves):
+    keys = np.random.default_rng(n).integers(0, most, size=n).astype(np.float64)
+    keys[0] = 0
+    assert _check(accelerator, keys, value, descending=True) == moves
+
+
+@pytest.mark.parametrize("n", [40_001, 150_001, 800_000])
+@pytest.mark.parametrize("seen,odd,moves", [
+    ((1, 2), (5,), 3), ((1, 2), (3, 5), 4), ((1, 2), (3, 5, 6), 5), ((1, 2), (3, 4, 5, 6), 0),   # higher bytes than the guess has
+    ((1,), (0,), 2), ((1, 2), (0,), 3), ((1, 2), (0, 5), 0), ((), (3,), 1), ((), (2, 3, 4, 5), 0)])  # a lower one
+def test_wrong_guess(accelerator, n, seen, odd, moves):
+    rng = np.random.default_rng(n)
+    raw = _with_bytes(rng, np.uint64, n, seen)
+    one = next(p for p in range(n // 2, n) if p not in set(_looked(n).tolist()))
+    for p in odd:
+        raw[one] ^= np.uint64(0x81) << np.uint64(8 * p)
+    if n < 100_000:
+        keys = raw.view(np.float64)   # short views go this way with floating-point keys
+        assert np.isfinite(keys).all()
+        assert _check(accelerator, keys, None) == moves
+    else:
+        assert _check(accelerator, raw, np.int32) == moves
 
 
 @pytest.mark.parametrize("n", [100_000, 250_001])
@@ -106,10 +165,13 @@ def test_sequenced_and_strided(accelerator, n):
     np.testing.assert_array_equal(storage.cpu().numpy()[::3], keys)
 
 
-def test_count_on_the_device():
+@pytest.mark.parametrize("few", [False, True])
+def test_count_on_the_device(few):
     n = 300_000
     L, rng = N.lib(), np.random.default_rng(n)
     keys, values = rng.integers(0, 1 << 60, size=n, dtype=np.uint64), np.arange(n, dtype=np.uint32)
+    if few:
+        keys &= np.uint64(0xFF00FF00)
     p = lambda t: ctypes.c_void_p(t.data_ptr())
     need = ctypes.c_int64(0)
     assert L.b200alg_radix_sort_temp_bytes(N.U64, n, 4, ctypes.byref(need)) == N.OK
