@@ -25,7 +25,6 @@
 namespace b200alg {
 
 constexpr int kLocalMost = 12288;            // elements: 24 for each of 512 threads, 12 for each of 1024
-constexpr int kPlaceBits = 14;
 static_assert(kLocalMost <= 1 << kPlaceBits, "a place fits its bits, a count its half of a word");
 constexpr int kLocalDigitBits = 9;
 constexpr int kLocalWords = 1 << (kLocalDigitBits - 1);  // counter words of a warp
@@ -171,20 +170,10 @@ template <typename K, bool PLACE, int ITEMS> struct LocalSort {
     int count, items;
     K low, high;
 
-    __device__ __forceinline__ K key_at(unsigned int word) const {
-        if constexpr (PLACE) return keys[word & ((1u << kPlaceBits) - 1u)];
-        else return (K)(low + (K)word);
-    }
-    static __device__ __forceinline__ unsigned int place_of(unsigned int word) { return word & ((1u << kPlaceBits) - 1u); }
-    // (two neighbours of the sorted order)
+    __device__ __forceinline__ K key_at(unsigned int word) const { return word_key<K, PLACE>(word, keys, low); }
+    static __device__ __forceinline__ unsigned int place_of(unsigned int word) { return b200alg::place_of(word); }
     static __device__ __forceinline__ bool wrong(K key_a, unsigned int a, K key_b, unsigned int b) {
-        if constexpr (PLACE) return key_a > key_b || (key_a == key_b && place_of(a) > place_of(b));
-        else return a > b;
-    }
-    // The key of a place past the last element (word ~0 where words are keys): behind all others.
-    __device__ __forceinline__ K key_or_most(unsigned int word) const {
-        if constexpr (PLACE) return place_of(word) < (unsigned int)count ? keys[place_of(word)] : (K)~(K)0;
-        else return key_at(word);
+        return words_out_of_order<K, PLACE>(key_a, a, key_b, b);
     }
     // Whether an element came out behind a place that holds none: in a tie of the last digits a warp's lanes past
     // the last element, served before the others, would push it out of what emit looks at.  (Not taking part would
@@ -192,7 +181,7 @@ template <typename K, bool PLACE, int ITEMS> struct LocalSort {
     __device__ __forceinline__ bool strays() const {
         bool any = false;
         for (int p = count + (int)threadIdx.x; p < items * (int)blockDim.x; p += (int)blockDim.x)
-            any |= PLACE ? place_of(words[p]) < (unsigned int)count : words[p] != ~0u;
+            any |= is_stray<PLACE>(words[p], count);
         if (any) atomicAdd(s.found, blockDim.x + 1u);  // more than settle takes
         return any;
     }
@@ -224,23 +213,10 @@ template <typename K, bool PLACE, int ITEMS> struct LocalSort {
     // What is rarely needed stays out of line and takes copies: the address of this object, or of what `store`
     // holds, in the hands of a function would keep them all in memory (pairs of 5000: 28600 cycles instead of 18000).
 
-    // Neighbours that are the wrong way round change places until none are (words past the last element included).
+    // Puts the words in order that the passes did not (those past the last element included).
     static __device__ __noinline__ void repair(LocalSort me) {
-        const int threads = (int)blockDim.x, all = me.items * threads;
-        bool again = true;
-        for (int round = 0; again && round < all; ++round) {
-            bool moved = false;
-            for (int odd = 0; odd < 2; ++odd) {
-                for (int p = 2 * (int)threadIdx.x + odd; p + 1 < all; p += 2 * threads) {
-                    const unsigned int a = me.words[p], b = me.words[p + 1];
-                    if (!wrong(me.key_or_most(a), a, me.key_or_most(b), b)) continue;
-                    me.words[p] = b;
-                    me.words[p + 1] = a;
-                    moved = true;
-                }
-                again = __syncthreads_or(moved) != 0;
-            }
-        }
+        put_words_in_order<K, PLACE>(me.words, me.keys, me.low, me.count, me.items * (int)blockDim.x, (int)threadIdx.x, (int)blockDim.x,
+                                     [](bool moved) { return __syncthreads_or(moved) != 0; });
     }
 
     // The pairs that emit found (s.part, *s.found of them) lie in groups that agree in all bits but the lowest `below`:

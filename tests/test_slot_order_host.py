@@ -1,6 +1,7 @@
-"""What puts a tile of the radix sort in order when a warp's atomics were not served in lane order, and
-the check that finds such a tile (tests/cpp/slot_order_test.cpp runs the kernels' own code on threads of
-the host, on slots that are out of order).  No GPU."""
+"""What puts a tile of the radix sort, or the words of the sort in one block and of the partition into buckets, in
+order when a warp's atomics were not served in lane order, and the check that finds such a tile
+(tests/cpp/slot_order_test.cpp runs the kernels' own code on threads of the host, on slots that are out of order).
+No GPU."""
 import os
 import subprocess
 
