@@ -25,12 +25,11 @@ def _keys(rng, dtype, n, kind):
 
 
 @pytest.mark.parametrize("n", [1, 2, 33, 256, 257, 1024, 1025, 6144, 6145, 7680, 7681, 9728, 11_777, 12_288, 12_289])
-@pytest.mark.parametrize("name", ["UInt8", "Int16", "UInt32", "Int32", "UInt64", "Int64"])
-@pytest.mark.parametrize("kind", ["full", "ties", "outlier", "0", "1", "9", "10", "18", "19", "27", "28"])
+@pytest.mark.parametrize("name,kind", [(name, kind) for name in ["UInt8", "Int16", "UInt32", "Int32", "UInt64", "Int64"]
+                                       for kind in ["full", "ties", "outlier", "0", "1", "9", "10", "18", "19", "27", "28"]
+                                       if not kind.isdigit() or int(kind) < np.dtype(NP[name]).itemsize * 8])
 def test_against_a_stable_sort(accelerator, name, n, kind):
     dtype = NP[name]
-    if kind.isdigit() and int(kind) >= np.dtype(dtype).itemsize * 8:
-        return  # more bits than the key has
     keys = _keys(np.random.default_rng(n), dtype, n, kind)
     order = np.argsort(keys, kind="stable")
     op = getattr(RadixSortOperations, "Ascending" + name)
