@@ -16,6 +16,7 @@
 // reference's: a stable sort by the transformed key.
 #include "common.cuh"
 #include "sort_common.cuh"
+#include "../../include/b200alg_testing.h"
 
 #include <type_traits>
 
@@ -33,6 +34,7 @@ enum : int {
     kCtlRole = 48,         // [48..55] blocks of this pass that have started
     kCtlHistogram = 56     // histogram blocks that have finished
 };
+static_assert(kCtlHistogram == B200ALG_TESTING_SORT_PASSES_WORD - 1, "(behind wait_limit_hit)");
 // The three buffers a sort moves its data between.
 enum : unsigned int { kBufIn = 0, kBufOut = 1, kBufAlt = 2 };
 

@@ -41,6 +41,10 @@ int b200alg_testing_time_sort_mg(void *comm, void *stream, const void *keys, con
  * did go by buckets, the number of bytes in which keys differ where these are few. */
 #define B200ALG_TESTING_SORT_MOVES_WORD 58
 
+/* The 32-bit word of a sort's temp that is not zero when the sort was made by passes over tiles.  The sorts in one
+ * launch leave it as it was. */
+#define B200ALG_TESTING_SORT_PASSES_WORD 57
+
 #ifdef __cplusplus
 }
 #endif

@@ -32,3 +32,6 @@ def to_device(a: np.ndarray) -> torch.Tensor:
 
 def to_host(t: torch.Tensor) -> np.ndarray:
     return t.cpu().numpy()
+
+
+PASSES_WORD = 57   # B200ALG_TESTING_SORT_PASSES_WORD

@@ -11,12 +11,16 @@ import torch
 from ilgpu_b200 import RadixSortOperations
 from ilgpu_b200 import _native as N
 from ilgpu_b200.algorithms import dtype_code
-from tests.helpers import NP, to_device, to_host
+from tests.helpers import NP, PASSES_WORD, to_device, to_host
 from tests.test_gpu_digit_pass import TILES
 
 pytestmark = pytest.mark.gpu
 
-LONG = 1_100_003   # keys; one launch sorts up to 2^20
+LONG = 1_600_003   # keys; one launch sorts up to 1.55 * 10^6 on 148 SMs
+
+
+def _went_by_passes(temp):
+    return int(temp.view(torch.int32)[PASSES_WORD]) != 0
 
 
 @pytest.mark.parametrize("name,value", list(TILES))
@@ -32,11 +36,11 @@ def test_few_tiles(name, value, tiles, extra):
     vb = 0 if value is None else values.itemsize
     need = ctypes.c_int64(0)
     assert N.lib().b200alg_radix_sort_temp_bytes(dtype_code(dk.dtype), LONG, vb, ctypes.byref(need)) == N.OK
-    temp = torch.empty(need.value, dtype=torch.uint8, device="cuda")
+    temp = torch.zeros(need.value, dtype=torch.uint8, device="cuda")
     p = lambda t: ctypes.c_void_p(0 if t is None else t.data_ptr())
     assert N.lib().b200alg_radix_sort_out_of_place(None, p(dk), p(dv), p(ok), p(ov), LONG, p(dn), dtype_code(dk.dtype), vb, 0, p(temp),
                                                    need.value) == N.OK
-    assert N.lib().b200alg_device_status(None, p(temp)) == N.OK
+    assert N.lib().b200alg_device_status(None, p(temp)) == N.OK and _went_by_passes(temp)
     order = np.argsort(keys[:count], kind="stable")
     got = to_host(ok)
     np.testing.assert_array_equal(got[:count], keys[:count][order])
@@ -74,13 +78,15 @@ def test_arriving(accelerator, name, kind, descending):
     # a stable descending sort: the reverse of the stable ascending sort of the reverse
     order = LONG - 1 - np.argsort(keys[::-1], kind="stable")[::-1] if descending else np.argsort(keys, kind="stable")
     view = to_device(keys)
-    temp = accelerator.Allocate1D(accelerator.ComputeRadixSortTempStorageSize(op, LONG), torch.int32)
+    temp = accelerator.Allocate1D(accelerator.ComputeRadixSortTempStorageSize(op, LONG), torch.int32).zero_()
     accelerator.CreateRadixSort(op)(None, view, temp)
+    assert _went_by_passes(temp)
     np.testing.assert_array_equal(to_host(view), keys[order])
     view, values = to_device(keys), torch.arange(LONG, dtype=torch.int32, device="cuda")
-    temp = accelerator.Allocate1D(accelerator.ComputeRadixSortPairsTempStorageSize(op, torch.int32, LONG), torch.int32)
+    temp = accelerator.Allocate1D(accelerator.ComputeRadixSortPairsTempStorageSize(op, torch.int32, LONG), torch.int32).zero_()
     accelerator.CreateRadixSortPairs(op)(None, view, values, temp)
     accelerator.CheckDeviceStatus(None, temp)
+    assert _went_by_passes(temp)
     np.testing.assert_array_equal(to_host(view), keys[order])
     np.testing.assert_array_equal(to_host(values), order)
 
@@ -92,15 +98,17 @@ def test_views(accelerator, name, offset, stride):
     storage = np.random.default_rng(offset + stride).integers(info.min, info.max, size=offset + LONG * stride, dtype=NP[name], endpoint=True)
     op = getattr(RadixSortOperations, "Ascending" + name)
     dev = to_device(storage)
-    temp = accelerator.Allocate1D(accelerator.ComputeRadixSortTempStorageSize(op, LONG), torch.int32)
+    temp = accelerator.Allocate1D(accelerator.ComputeRadixSortTempStorageSize(op, LONG), torch.int32).zero_()
     accelerator.CreateRadixSort(op)(None, dev[offset::stride][:LONG], temp)
     accelerator.CheckDeviceStatus(None, temp)
+    assert _went_by_passes(temp)
     expected = storage.copy()
     expected[offset::stride][:LONG] = np.sort(storage[offset::stride][:LONG])
     np.testing.assert_array_equal(to_host(dev), expected)   # what lies around and between stays
     if stride == 1:
         keys, values = to_device(storage), torch.arange(LONG + offset, dtype=torch.int32, device="cuda")
-        temp = accelerator.Allocate1D(accelerator.ComputeRadixSortPairsTempStorageSize(op, torch.int32, LONG), torch.int32)
+        temp = accelerator.Allocate1D(accelerator.ComputeRadixSortPairsTempStorageSize(op, torch.int32, LONG), torch.int32).zero_()
         accelerator.CreateRadixSortPairs(op)(None, keys[offset:], values[offset:], temp)
+        assert _went_by_passes(temp)
         np.testing.assert_array_equal(to_host(keys), expected)
         np.testing.assert_array_equal(to_host(values)[offset:], np.argsort(storage[offset:], kind="stable") + offset)
