@@ -70,9 +70,10 @@ def test_lengths_and_distributions(accelerator, n, key, value, kind):
     _check(accelerator, _keys(np.random.default_rng(n), np.dtype(key), n, kind), value, descending=kind == "half")
 
 
-def _sampled(n, sms):
-    """Positions that the blocks look at (sample_sort.cu)."""
-    blocks = min(-(-n // 1536), sms)
+def _sampled(n, most=None):
+    """Positions that the blocks look at in a view of n elements, launched for up to `most` (sample_sort.cu)."""
+    most = most or n
+    blocks = 16 if most <= 40_960 else min(-(-most // 1536), torch.cuda.get_device_properties(0).multi_processor_count)
     share = -(-n // blocks)
     at = []
     for b in range(blocks):
@@ -84,16 +85,75 @@ def _sampled(n, sms):
     return np.concatenate(at)
 
 
-@pytest.mark.parametrize("key,value", [(np.uint64, np.int32), (np.uint64, np.int16), (np.uint32, np.int64)])
+def _misleading(key, n, most=None):
+    """Keys that are all in one bucket but for what is looked at."""
+    rng, at, key = np.random.default_rng(5), _sampled(n, most), np.dtype(key)
+    if key.kind == "f":
+        keys = (2 + 30 * rng.random(n)).astype(key)   # (all bytes of a float differ)
+        keys[at] = rng.random(at.size)
+        return keys
+    bits = key.itemsize * 8
+    keys = (rng.integers(0, 1 << (bits - 1), size=n, dtype=key) >> key.type(4)) + key.type(1 << (bits - 1))
+    keys[at] = rng.integers(0, 1 << 16, size=at.size)
+    return keys
+
+
+@pytest.mark.parametrize("key,value,n", [(np.uint64, np.int32, 300_007), (np.uint64, np.int16, 300_007), (np.uint32, np.int64, 300_007),
+                                         (np.uint64, None, 800_003), (np.float64, None, 300_007), (np.float64, None, 30_001),
+                                         (np.float64, np.int32, 40_960), (np.float32, np.int32, 40_001)])
 @pytest.mark.parametrize("descending", [False, True])
-def test_misled_sample(accelerator, key, value, descending):
+def test_misled_sample(accelerator, key, value, n, descending):
+    assert _check(accelerator, _misleading(key, n), value, descending) == np.dtype(key).itemsize   # by every digit
+
+
+@pytest.mark.parametrize("n", [30_001, 300_007])
+def test_misled_strided(accelerator, n):
+    keys, op = _misleading(np.float64, n), RadixSortOperations.DescendingDouble
+    storage = torch.from_numpy(np.repeat(keys, 3)).cuda()
+    temp = accelerator.Allocate1D(accelerator.ComputeRadixSortTempStorageSize(op, n), torch.int32)
+    temp[MOVES] = -1
+    accelerator.CreateRadixSort(op, True)(None, storage[1::3], temp)
+    assert int(temp[MOVES]) == 8
+    got = storage.cpu().numpy()
+    np.testing.assert_array_equal(got[1::3], np.sort(keys)[::-1])
+    np.testing.assert_array_equal(got[::3], keys)     # what lies between stays
+    np.testing.assert_array_equal(got[2::3], keys)
+
+
+def test_misled_sequenced(accelerator):
     n = 300_007
-    rng = np.random.default_rng(5)
-    bits = np.dtype(key).itemsize * 8
-    keys = (rng.integers(0, 1 << (bits - 1), size=n, dtype=key) >> 4) + key(1 << (bits - 1))   # all in one bucket ...
-    at = _sampled(n, torch.cuda.get_device_properties(0).multi_processor_count)
-    keys[at] = rng.integers(0, 1 << 16, size=at.size)                                          # ... but for what is looked at
-    assert _check(accelerator, keys, value, descending) == np.dtype(key).itemsize   # by every digit
+    keys, op = _misleading(np.uint64, n), RadixSortOperations.AscendingUInt64
+    dev, vals = torch.from_numpy(keys).cuda(), torch.zeros(n, dtype=torch.float32, device="cuda")
+    temp = accelerator.Allocate1D(accelerator.ComputeRadixSortPairsTempStorageSize(op, vals.dtype, n), torch.int32)
+    temp[MOVES] = -1
+    accelerator.CreateRadixSortPairs(op, sequencer=Sequencers)(None, dev, vals, Sequencers.FloatSequencer, temp)
+    assert int(temp[MOVES]) == 8
+    order = np.argsort(keys, kind="stable")
+    np.testing.assert_array_equal(dev.cpu().numpy(), keys[order])
+    np.testing.assert_array_equal(vals.cpu().numpy(), order)
+
+
+@pytest.mark.parametrize("value_bytes", [0, 4])
+def test_misled_count_on_the_device(value_bytes):
+    most, n = 800_000, 760_001
+    L, keys = N.lib(), _misleading(np.uint64, 760_001, 800_000)
+    p = lambda t: ctypes.c_void_p(t.data_ptr() if t is not None else 0)
+    need = ctypes.c_int64(0)
+    assert L.b200alg_radix_sort_temp_bytes(N.U64, most, value_bytes, ctypes.byref(need)) == N.OK
+    temp = torch.full((need.value // 4,), -1, dtype=torch.int32, device="cuda")
+    k = torch.from_numpy(np.concatenate([keys, np.zeros(most - n, np.uint64)])).cuda()
+    ok, count = torch.full((most,), 9, dtype=torch.int64, device="cuda"), torch.tensor([n], dtype=torch.int64, device="cuda")
+    v, ov = (torch.arange(most, dtype=torch.int32, device="cuda"), torch.full((most,), 9, dtype=torch.int32, device="cuda")) if value_bytes else (None, None)
+    assert L.b200alg_radix_sort_out_of_place(None, p(k), p(v), p(ok), p(ov), most, p(count), N.U64, value_bytes, 0, p(temp), need.value) == N.OK
+    assert int(temp[MOVES]) == 8
+    order = np.argsort(keys, kind="stable")
+    got = ok.cpu().numpy()
+    np.testing.assert_array_equal(got[:n].view(np.uint64), keys[order])
+    assert (got[n:] == 9).all()
+    if value_bytes:
+        got = ov.cpu().numpy()
+        np.testing.assert_array_equal(got[:n], order)
+        assert (got[n:] == 9).all()
 
 
 def _looked(n):
