@@ -161,7 +161,7 @@ constexpr int local_bytes(int key_bytes, int value_bytes) { return 4 + value_byt
 template <typename K> __host__ __device__ constexpr bool by_place(bool values) { return values || sizeof(K) == 8; }
 
 // Sorts `count` elements.  By place: keys (in shared memory, transformed) stay, words receive the places
-// in order.  Else: key[] holds this thread's transformed keys (element warp * 32 * items + i * 32 + lane), words
+// in order; key is not read.  Else: key[] holds this thread's transformed keys (element warp * 32 * items + i * 32 + lane), words
 // receive the keys less `low`.  store(p, key, word) is called for the p-th in order, possibly again.
 template <typename K, bool PLACE, int ITEMS> struct LocalSort {
     LocalShared s;

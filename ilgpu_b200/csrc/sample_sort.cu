@@ -93,7 +93,6 @@ template <typename K, typename V> struct SampleBlock {
     static constexpr int VB = ValueBytes<V>::value;
     static constexpr int ITEMS = sample_items<K>(VB), MOST = ITEMS * kSampleThreads;
     LocalShared shared;
-    SampleShared<K> *m;
     unsigned int *words;
     V *values;
     K *keys;
@@ -153,7 +152,7 @@ __global__ void __launch_bounds__(kSampleThreads, 1)
 sample_sort_kernel(SampleSort<K, V> a) {
     using B = SampleBlock<K, V>;
     constexpr int VB = B::VB;
-    constexpr bool PLACE = by_place<K>(VB != 0);
+    static_assert(by_place<K>(VB != 0), "keys stay in shared memory and are looked up there");
     extern __shared__ __align__(128) unsigned char smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, blocks = (int)gridDim.x;
     SampleShared<K> *const m = reinterpret_cast<SampleShared<K> *>(smem + local_fixed_bytes(kSampleThreads));
@@ -165,7 +164,6 @@ sample_sort_kernel(SampleSort<K, V> a) {
     b.shared = local_shared(smem);
     local_clear(b.shared);
     grid_dependency_wait();
-    b.m = m;
     b.n = (unsigned int)effective_n(a.io);
     const unsigned int share = (b.n + blocks - 1) / blocks;
     b.lo = blockIdx.x * share < b.n ? blockIdx.x * share : b.n;
@@ -559,41 +557,23 @@ sample_sort_kernel(SampleSort<K, V> a) {
         const unsigned int start = m->start[bucket];
         const int count = (int)(m->start[bucket + 1] - start), items = (count + kSampleThreads - 1) / kSampleThreads;
         const int own = warp * 32 * items + lane;
-        K key[kSampleItems];
         K low = (K)~(K)0, high = 0;
-        if constexpr (PLACE) {
-            b.fetch(a.io.alt, 1, a.io.valt, kSeqNone, start, count, items);
-            copies_wait();
-        }
+        b.fetch(a.io.alt, 1, a.io.valt, kSeqNone, start, count, items);
+        copies_wait();
 #pragma unroll
         for (int i = 0; i < kSampleItems; ++i) {
             if (i >= items) break;
-            const int at = own + i * 32;
-            if (at < count) {
-                if constexpr (PLACE) {
-                    const K k = b.keys[at];
-                    low = k < low ? k : low;
-                    high = k > high ? k : high;
-                } else {
-                    key[i] = __ldcg(a.io.alt + start + at);
-                }
-            }
-        }
-        if constexpr (!PLACE) {
-#pragma unroll
-            for (int i = 0; i < kSampleItems; ++i) {
-                if (i >= items) break;
-                if (own + i * 32 < count) {
-                    low = key[i] < low ? key[i] : low;
-                    high = key[i] > high ? key[i] : high;
-                }
+            if (own + i * 32 < count) {
+                const K k = b.keys[own + i * 32];
+                low = k < low ? k : low;
+                high = k > high ? k : high;
             }
         }
         local_range(b.shared, low, high);
-        const LocalSort<K, PLACE, kSampleItems> sort{b.shared, b.words, b.keys, count, items, low, high};
-        sort.run(key, [=](int p, K k, unsigned int word) {
+        const LocalSort<K, true, kSampleItems> sort{b.shared, b.words, b.keys, count, items, low, high};
+        sort.run(nullptr, [=](int p, K k, unsigned int word) {
             out[(int64_t)(start + p) * stride] = xf.raw(k);
-            if constexpr (VB != 0) vout[start + p] = values[LocalSort<K, PLACE, kSampleItems>::place_of(word)];
+            if constexpr (VB != 0) vout[start + p] = values[place_of(word)];
         });
         __syncthreads();
     }
