@@ -9,6 +9,8 @@
 //     27 bits of the range in three passes.  Few keys agree in all of these unless the range has outliers;
 //     the writer compares neighbours by their whole keys, and where some are out of order it puts the groups
 //     that agree in the upper bits in order.  Where there are too many, the passes run again over all bits.
+//   - Where the range has more bits, those below the lowest one that a key of each thread has (in its distance) are left
+//     out as well: whole numbers kept as floating-point end in zeros, and are few bits without these.
 //   - With values or 8-byte keys an element travels as a word: its place in the block (14 bits) below the
 //     digits that are still to come (18 bits after the first pass).  Keys and values stay where they were
 //     loaded and are fetched by place in the end.  Keys of up to four bytes alone travel as themselves.
@@ -24,7 +26,7 @@
 
 namespace b200alg {
 
-constexpr int kLocalMost = 12288;            // elements: 24 for each of 512 threads, 12 for each of 1024
+constexpr int kLocalMost = 12288;            // elements: 24 for each of 512 threads
 static_assert(kLocalMost <= 1 << kPlaceBits, "a place fits its bits, a count its half of a word");
 constexpr int kLocalDigitBits = 9;
 constexpr int kLocalWords = 1 << (kLocalDigitBits - 1);  // counter words of a warp
@@ -38,6 +40,7 @@ struct LocalShared {
     unsigned int *part;   // [threads / 256][kLocalWords]
     unsigned int *warp_sum;          // [8]
     unsigned int *found;             // neighbours out of order
+    unsigned int *seen;              // [2]: bits of some keys' distances
     unsigned long long *low, *high;  // [32]
 };
 __host__ __device__ constexpr int local_fixed_bytes(int threads) { return threads / 32 * kLocalWords * 4 + threads / 256 * kLocalWords * 4 + 2 * 32 * 8 + 64; }
@@ -50,6 +53,7 @@ __device__ __forceinline__ LocalShared local_shared(unsigned char *smem) {
     s.high = s.low + 32;
     s.warp_sum = reinterpret_cast<unsigned int *>(s.high + 32);
     s.found = s.warp_sum + 8;
+    s.seen = s.found + 1;
     return s;
 }
 
@@ -110,6 +114,7 @@ __device__ __forceinline__ uint2 local_places(const LocalShared &s) {
 }
 
 // The smallest and the largest of the block's keys (one barrier; low / high may be written again behind the next).
+// Clears seen.
 template <typename K> __device__ __forceinline__ void local_range(const LocalShared &s, K &low, K &high) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = (int)blockDim.x >> 5;
     auto least = [](K v) {
@@ -122,6 +127,7 @@ template <typename K> __device__ __forceinline__ void local_range(const LocalSha
         }
     };
     const K warp_low = least(low), warp_high = (K)~least((K)~high);
+    if (threadIdx.x < 2) s.seen[threadIdx.x] = 0u;
     if (lane == 0) {
         s.low[warp] = (unsigned long long)warp_low;
         s.high[warp] = (unsigned long long)warp_high;
@@ -300,9 +306,10 @@ template <typename K, bool PLACE, int ITEMS> struct LocalSort {
         return bad;
     }
 
-    // Whether two of a few keys of every warp agree in all bits but the lowest `below` and differ in those: then
-    // many of the block's do.
-    __device__ __forceinline__ bool ties_likely(const K *key, int own, int below) const {
+    // The lowest bit to sort by, of more bits than the digits cover; `below` are left over.  One key of every thread is
+    // looked at.  Where two neighbours of a few agree in all bits but the lowest `below` and differ in those, many of the
+    // block's do; and what none has below its lowest bit hardly any has (else the writer finds it).
+    __device__ __forceinline__ int lowest_bit(const K *key, int own, int below) const {
         const int lane = threadIdx.x & 31;
         K mine = 0;
         if (own < count) mine = PLACE ? (K)(keys[own] - low) : (K)(key[0] - low);
@@ -314,7 +321,19 @@ template <typename K, bool PLACE, int ITEMS> struct LocalSort {
             else other = (K)__shfl_down_sync(0xffffffffu, (unsigned int)mine, k);
             tie |= lane + k < 32 && own + k < count && other != mine && other >> below == mine >> below;
         }
-        return __syncthreads_or(tie) != 0;
+        const unsigned int lower = __reduce_or_sync(0xffffffffu, (unsigned int)mine);
+        if (lane == 0) atomicOr(s.seen, lower);
+        if constexpr (sizeof(K) == 8) {
+            const unsigned int upper = __reduce_or_sync(0xffffffffu, (unsigned int)(mine >> 32));
+            if (lane == 0) atomicOr(s.seen + 1, upper);
+        }
+        tie = __syncthreads_or(tie) != 0;
+        const unsigned int first = s.seen[0];
+        int lowest = __ffs((int)first) - 1;
+        if constexpr (sizeof(K) == 8) {
+            if (first == 0u) lowest = __ffs((int)s.seen[1]) - 1 + (s.seen[1] ? 32 : 0);
+        }
+        return lowest > below || (tie && lowest >= 0) ? lowest : below;
     }
 
     // The tables are clear, keys (by place) are in shared memory behind a barrier, low and high are known.
@@ -323,8 +342,8 @@ template <typename K, bool PLACE, int ITEMS> struct LocalSort {
         const K range = (K)(high - low);
         const int bits = sizeof(K) == 8 ? 64 - __clzll((long long)range) : 32 - __clz((int)(unsigned int)range);
         if (threadIdx.x == 0) *s.found = 0u;
-        int from = bits > kLocalPrefixBits ? bits - kLocalPrefixBits : 0;  // the lowest bit that is sorted by
-        if (from > 0 && ties_likely(key, own, from)) from = 0;
+        int from = 0;  // the lowest bit that is sorted by
+        if (bits > kLocalPrefixBits) from = lowest_bit(key, own, bits - kLocalPrefixBits);
         unsigned int w[ITEMS];
         bool fresh = true;  // words hold nothing yet
         for (;;) {

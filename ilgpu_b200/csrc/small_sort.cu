@@ -425,7 +425,7 @@ block_sort_kernel(SortBuffers<K, V> io, KeyXform<K> xf, TempHeader *hdr, int ite
 // Which blocks (times on the GPU, us, with the launch and the copy that brings the data):
 //   one       block_sort_kernel, against a cluster, by key bytes / value bytes.  What a cluster takes depends on the
 //             bytes in which keys differ; the line for integers is where identifiers below 2^20 (three bytes) cost the
-//             same either way, floating-point keys differ in all bytes.
+//             same either way.
 //                          4500          6200          7500          9000         12000
 //                1 / 0    8.4   8.3    8.2   8.4   10.2   8.6   10.3   8.2   12.3   8.8
 //                2 / 0   10.2  12.3   10.3  12.3   12.3  12.3   14.3  12.5   16.4  13.1
@@ -440,14 +440,30 @@ block_sort_kernel(SortBuffers<K, V> io, KeyXform<K> xf, TempHeader *hdr, int ite
 //                8 / 4   17.0  42.2   19.1  42.5   21.3  42.3   23.5  46.7   27.7  46.8
 //                        16.4  21.3   20.5  21.3   20.5  21.3   24.5  22.7   29.1  23.4   below 2^20
 //                8 / 8   18.7  41.9   21.2  43.3   25.3  42.4   28.3  46.9    does not fit
+//             Longer floating-point keys go by buckets in a cluster (4 / 0: by bytes).  One block against these:
+//                          5000          6600          8100          9000         12288
+//                4 / 0   13.8  18.4   14.4  18.4   16.4  18.2   18.4  18.5   20.5  18.5
+//                        12.3  14.4   14.4  14.4   16.4  14.4   16.4  15.3   20.5  15.4   whole numbers below 2^8
+//                4 / 4   18.5  24.6   21.2  23.3   23.4  25.1   24.6  25.4   28.6  25.4
+//                        16.9  16.4   18.6  16.7   21.2  16.4   22.7  18.7   27.2  17.7   whole numbers below 2^8
+//                8 / 0   18.4  22.6   20.5  22.5   22.6  24.6   26.6  24.2   30.8  24.6
+//                        14.4  20.5   17.4  20.5   19.5  20.5   21.6  21.6   26.6  21.5   whole numbers below 2^8
+//                8 / 4   20.6  27.5   25.6  25.3   27.5  27.5   29.3  27.5   35.9  27.6
+//                        19.4  23.5   21.5  23.3   23.5  23.2   25.6  25.5   30.5  24.6   whole numbers below 2^8
+//             What one block does not do well is keys that need one pass: 8100 int64 below 2^8 with 4 bytes 17.3, by a
+//             block of 1024 threads with a pass per byte 13.7 (but of the full range 23.5 and 42.7).
 //   cluster   up to 40960 elements (uint32 keys / pairs: 40000: 27 / 33 us against 29 / 32 us with a
 //             grid; 60000: 35 / 43 us against 29 / 33 us);
 //   grid      about 64 blocks until they have 4 keys per thread, then more, up to about the length from
-//             which the passes over tiles are as fast (against those: 2^20 uint32 keys 61.5 us against 59.6, keys
-//             below 2^20 47.2 against 54.1; 786432 uint32 keys + 8 bytes 51.3 against 55.5).
-// Longer ones go by buckets (sample_sort.cu) where that is faster.
+//             which the passes over tiles are as fast (against those: 2^20 uint32 keys 61.4 us against 62.1, keys
+//             below 2^20 47.2 against 54.1; 786432 uint16 keys with 1, 4 and 8 bytes 37.8, 38.5 and 39.8 against 51.9,
+//             50.9 and 43.0).
+// Keys of 8 bytes, and of 4 with values, go by buckets from where that is faster (sample_least in sample_sort.cu, asked
+// before these two are).
 constexpr int64_t alone_most(int key_bytes, int value_bytes, bool floating) {
-    return key_bytes == 1 ? 6144 : key_bytes == 2 ? 7680 : floating ? kLocalMost : key_bytes == 4 ? (value_bytes ? 7168 : 9216) : (value_bytes ? 8192 : 6656);
+    if (key_bytes < 4) return key_bytes == 1 ? 6144 : 7680;
+    if (key_bytes == 4) return floating || value_bytes == 0 ? 9216 : 7168;
+    return floating ? (value_bytes ? 7168 : 8704) : (value_bytes ? 8192 : 6656);
 }
 constexpr int64_t kClusterMost = 5 * kMaxCluster * kResidentThreads;
 constexpr int64_t kGridMostNarrow = 1 << 20, kGridMost = 3 << 18;

@@ -181,7 +181,7 @@ def test_few_bytes(accelerator, n, key, value, at):
         assert moves == (max(1, len(at)) if len(at) <= 3 else 0)
 
 
-@pytest.mark.parametrize("n", [12_289, 16_384, 40_960, 40_961, 150_001])
+@pytest.mark.parametrize("n", [8705, 12_289, 16_384, 40_960, 40_961, 150_001])
 @pytest.mark.parametrize("value", [None, np.int32, np.int64])
 @pytest.mark.parametrize("most,moves", [(2, 2), (256, 3), (1 << 19, 0)])
 def test_whole_numbers(accelerator, n, value, most, moves):
