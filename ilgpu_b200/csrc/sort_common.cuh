@@ -97,14 +97,15 @@ struct SortScratch {
     int64_t control_bytes;
 };
 
-// The sort of a view by one partition into buckets that a block holds, in one launch (sample_sort.cu).  *taken:
-// false when the view is too short or too long for that.
+// A sort is made by the first of these that takes it (*taken), each in one launch, and else by passes over tiles:
+// one block's (small_sort.cu);
+int block_sort(cudaStream_t s, const SortCall &call, int key_bytes, int value_bytes, uint64_t xor_neg, uint64_t xor_pos, void *temp, bool *taken);
+
+// by one partition into buckets that a block holds, 8-byte keys and 4-byte keys with values (sample_sort.cu);
 int sample_sort(cudaStream_t s, const SortCall &call, int key_bytes, int value_bytes, uint64_t xor_neg, uint64_t xor_pos, void *temp,
                 const SortScratch &scratch, bool *taken);
 
-// The sort of a view that fits on the GPU's SMs as a whole, in one launch (small_sort.cu): one block's, or, of keys
-// of up to 4 bytes, that of several.  *taken: false when the view is too long for that.
-int block_sort(cudaStream_t s, const SortCall &call, int key_bytes, int value_bytes, uint64_t xor_neg, uint64_t xor_pos, void *temp, bool *taken);
+// by passes of a cluster or a grid that holds the view as a whole, keys of any size (small_sort.cu).
 int resident_sort(cudaStream_t s, const SortCall &call, int key_bytes, int value_bytes, uint64_t xor_neg, uint64_t xor_pos, void *temp,
                   int64_t temp_bytes, bool *taken);
 
