@@ -597,7 +597,8 @@ sample_sort_kernel(SampleSort<K, V> a) {
 // (The passes' clearing has since come to start early, 3 us less for them.)  Integers go this way from where those
 // below 2^20 lost nothing when they went by buckets too (now shorter ones of 8 bytes would gain); floating-point keys
 // wherever one block is not faster (alone_most in small_sort.cu; float keys with 4-byte values 12288: 25.3 against 26.2
-// by a cluster with a pass per byte, of whole numbers below 2^8 18.6 against 21.5).  Whole numbers
+// by a cluster with a pass per byte, of whole numbers below 2^8 18.6 against 21.5; but with 2-byte values 14000: 26.6
+// against 24.5, 19000: 26.6 and 27.1).  Whole numbers
 // kept as double below 2^8 differ in three bytes: 20000 of them 22.8 against 23.8 us by passes, 400000 39.2 and 49.0.
 // A wrong guess costs 4 to 7 us: 400000 uint64 + 4 bytes below 2^16 but for one key that differs in five bytes 55.6 us
 // (by passes 63.9), in six, which then go by buckets, 65.9 (75.4).
@@ -605,8 +606,8 @@ sample_sort_kernel(SampleSort<K, V> a) {
 constexpr int kSampleShare = 1536;
 constexpr int kSampleCluster = 16;
 constexpr int64_t kClusterSort = 40960;
-constexpr int64_t sample_least(int value_bytes, bool floating) {
-    return floating ? 1 : value_bytes ? 100000 : 700000;
+constexpr int64_t sample_least(int key_bytes, int value_bytes, bool floating) {
+    return floating ? (key_bytes == 4 && value_bytes < 4 ? 20000 : 1) : value_bytes ? 100000 : 700000;
 }
 
 struct SampleLimits {
@@ -658,7 +659,7 @@ static int run_sample_sort(cudaStream_t s, const SortCall &call, uint64_t xn, ui
         cache.store(lim);
     }
     const int64_t n = call.n;
-    if (n < sample_least(VB, xn != xp)) return B200ALG_OK;  // (integers' transforms have one constant)
+    if (n < sample_least(sizeof(K), VB, xn != xp)) return B200ALG_OK;  // (integers' transforms have one constant)
     const bool in_cluster = lim.cluster && n <= kClusterSort;
     int64_t blocks = in_cluster ? kSampleCluster : ceil_div(n, kSampleShare);
     blocks = blocks < lim.grid ? blocks : lim.grid;
